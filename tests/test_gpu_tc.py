@@ -192,3 +192,17 @@ def test_tc_copy_out_alongside_computation_covers_the_matrix(ssu, gemm_mode, mon
     plan.close()
     np.testing.assert_array_equal(full, ref)
     assert np.all(np.diag(full) == 0.0)
+
+
+def test_tc_plans_of_different_trees_run_in_turn(ssu, oracle_mod, gemm_mode):
+    """Two plans with different node counts alive at once (either created
+    last): executing one, then the other, then the first again."""
+    cases = [_case(51, 2500, 40), _case(52, 300, 40)]
+    for order in (cases, cases[::-1]):
+        plans = [ssu.Plan(tree, table, "unweighted_fp64") for tree, table in order]
+        for i in (0, 1, 0):
+            plans[i].execute()
+            ref = oracle_mod.oracle_one_off(*order[i], "unweighted_fp64")["matrix"]
+            assert rel_err(plans[i].result(), ref)[0] <= TC_REL
+        for p in plans:
+            p.close()

@@ -1786,12 +1786,14 @@ int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     SSU_CK(cudaFuncSetAttribute(tc::unweighted_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(tc::SMEM_BYTES)));
     const size_t bits_smem = sizeof(uint32_t) * (k_pad / 32);
-    if (bits_smem > 200 * 1024) {
+    if (bits_smem > tc::MAX_BITMAP_BYTES) {
         last_error = "tree too large for the tensor-core presence kernel";
         return kOutputError;
     }
+    // the same limit for every plan: the attribute is the kernel's, not the
+    // plan's, so a plan's own size would refuse the launches of other plans
     SSU_CK(cudaFuncSetAttribute(tc::presence_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(bits_smem)));
+                                static_cast<int>(tc::MAX_BITMAP_BYTES)));
     SSU_CK(alloc(&d_full, (spec.fp64 ? sizeof(double) : sizeof(float)) * std::max<uint64_t>(full_elems, 1)));
     SSU_CK(cudaStreamSynchronize(stream));
     timer.step("gemm_buffers");

@@ -73,6 +73,7 @@ constexpr int QBITS = digits::kBits;   // fixed-point bits of the largest length
 constexpr int MAX_PART = static_cast<int>(digits::kMaxPart);  // largest u v and s t
 constexpr int ACC_STRIDE = 256;        // TMEM columns between the two accumulators
 constexpr int TMEM_COLS = 512;
+constexpr size_t MAX_BITMAP_BYTES = 200 * 1024;  // presence bitmap of one sample in shared memory
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr uint32_t A_BYTES = ROWS * BLOCK_K;    // one product's A tile
