@@ -206,3 +206,77 @@ def test_tc_plans_of_different_trees_run_in_turn(ssu, oracle_mod, gemm_mode):
             assert rel_err(plans[i].result(), ref)[0] <= TC_REL
         for p in plans:
             p.close()
+
+
+def _sparse_case(seed, n_tips, n_samples, density):
+    """A table whose CSR also holds explicit zeros (not present) and samples without counts."""
+    tree, table = _case(seed, n_tips, n_samples, density)
+    rng = np.random.default_rng(seed)
+    table.data[rng.random(table.data.shape[0]) < 0.1] = 0.0
+    table.data[np.isin(table.indices, [0, n_samples // 2])] = 0.0
+    return tree, table
+
+
+@pytest.mark.parametrize("lists", ["1", "2"])
+@pytest.mark.parametrize("n_samples,n_tips,density", [(2, 40, 0.2), (127, 300, 0.03), (129, 900, 0.01), (600, 2500, 0.02),
+                                                      (2561, 700, 0.01)])
+@pytest.mark.parametrize("method", ["unweighted_fp64", "unweighted_unnormalized_fp64", "unweighted"])
+def test_tc_sparse_nodes_by_lists(ssu, oracle_mod, gemm_mode, monkeypatch, lists, n_samples, n_tips, density, method):
+    """Nodes of few samples summed through sample lists (16- and 32-bit
+    entries; the largest table is walked in two parts), the others contracted:
+    full matrix, stripe window and condensed form against the oracle."""
+    monkeypatch.setenv("UNIFRAC_B200_TC_LISTS", lists)
+    tree, table = _sparse_case(n_samples + n_tips, n_tips, n_samples, density)
+    ref = oracle_mod.oracle_one_off(tree, table, method.replace("_fp64", "") + "_fp64")["matrix"]
+    gpu, _ = ssu.one_off_matrix(tree, table, method)
+    np.testing.assert_array_equal(np.isnan(gpu), np.isnan(ref))
+    r, z = rel_err(np.nan_to_num(gpu), np.nan_to_num(ref))
+    assert r <= TC_REL and z <= 1e-9, (r, z)
+    if n_samples <= 600:
+        cf, _, _ = ssu.one_off(tree, table, method)
+        assert rel_err(np.nan_to_num(cf), np.nan_to_num(ref[np.triu_indices(n_samples, 1)]))[0] <= TC_REL
+        stop = (n_samples + 1) // 2
+        stripes, _ = ssu.partial(tree, table, method, stop // 3, stop)
+        k = np.arange(n_samples)
+        exp = np.array([ref[k, (k + s + 1) % n_samples] for s in range(stop // 3, stop)])
+        assert rel_err(np.nan_to_num(stripes), np.nan_to_num(exp))[0] <= TC_REL
+
+
+def test_tc_sparse_lists_over_column_chunks(ssu, gemm_mode, monkeypatch):
+    """15,000 samples: a row of shared sums spans two chunks of columns.  With
+    lists and with every node contracted the matrices agree to the
+    contraction's bound (each side is within it of the exact value)."""
+    tree = ssu_synth.random_binary_tree(400, 0.05, 61)
+    table = ssu_synth.presence_table(tree.tip_names(), 15000, 3, 12, 62)
+    got = []
+    for lists in ("1", "0"):
+        monkeypatch.setenv("UNIFRAC_B200_TC_LISTS", lists)
+        plan = ssu.Plan(tree, table, "unweighted")
+        for _ in range(2):  # a second pass reuses the lists' buffers
+            plan.execute()
+        got.append(plan.result())
+        plan.close()
+    far = np.abs(got[0] - got[1])
+    assert np.all(far <= 2 * TC_REL * np.abs(got[1]) + 1e-9)
+
+
+def test_tc_sparse_lists_in_a_batch(ssu, oracle_mod, monkeypatch):
+    """Tables of uneven size in one group, each with lists of its own; the
+    plan as a CUDA graph gives the same matrices."""
+    monkeypatch.setenv("UNIFRAC_B200_TC_LISTS", "1")
+    tree = ssu_synth.random_binary_tree(900, 0.05, 71)
+    tips = tree.tip_names()
+    tables = [ssu_synth.geometric_table(tips[5 * i:800 + 10 * i], n, 0.03, 6.0, 72 + i)
+              for i, n in enumerate((3, 130, 257, 64))]
+    plan = ssu.BatchPlan(tree, tables, "unweighted", autotune=0)
+    plan.execute()
+    got = plan.results()
+    plan.set_graph(True)
+    plan.execute()
+    for a, b in zip(plan.results(), got):
+        np.testing.assert_array_equal(a, b)
+    plan.close()
+    for t, m in zip(tables, got):
+        ref = oracle_mod.oracle_one_off(tree, t, "unweighted_fp64")["matrix"]
+        r, z = rel_err(np.nan_to_num(m), np.nan_to_num(ref))
+        assert r <= TC_REL and z <= 1e-9, (r, z)

@@ -19,6 +19,7 @@
 #include "ssu_gemm.cuh"
 #include "ssu_host.hpp"
 #include "ssu_kernels.cuh"
+#include "ssu_lists.cuh"
 #include "ssu_pairs.cuh"
 #include "ssu_sparse.cuh"
 #include "ssu_union.cuh"
@@ -61,6 +62,7 @@ bool parse_method(const char *name, Method &method, bool &fp64) {
 namespace {
 
 constexpr int kOutputError = 6;  // ComputeStatus output_error
+constexpr uint32_t kSharedCols = 14080;  // columns of a shared-sums row held at once (8 bytes each: two blocks an SM)
 
 // One stream-ordered memory pool per device, owned by the library, that
 // keeps freed blocks cached (no release threshold): repeated calls reuse the
@@ -366,7 +368,7 @@ struct Group {
     int32_t *d_tip_obs = nullptr;        // [tip][t1 - t0]: the tip's row in each table, or -1
     double *d_totals = nullptr;          // per column, fp64
     void *d_tot = nullptr;               // per column in T (variance adjusted)
-    uint32_t *d_block_table = nullptr;   // per 128 columns: the table (per-table lengths)
+    uint32_t *d_block_table = nullptr;   // per 128 columns: the table
     std::vector<double> totals;
     uint4 *d_tiles = nullptr;
     uint32_t n_tiles = 0, splits = 1, rows_per_split = 0;
@@ -376,18 +378,51 @@ struct Group {
     // tensor-core path, one table: first work unit and first row of each
     // band of row blocks (one extra entry closes the list)
     std::vector<uint32_t> band_unit, band_row;
+    // sample lists of the sparse nodes (n_nodes == 0: none)
+    dev::ListArgs lists;
+    // columns in order of their part of their table's samples, and the first
+    // of each part (one extra entry closes the list)
+    uint32_t *d_columns = nullptr;
+    std::vector<uint32_t> part_col;
+    uint64_t *d_shared_off = nullptr;    // condensed shared sums: first element of each table
 };
+
+// When a node goes by sample lists: by its estimated time there (per pair of
+// samples that have it, and per sample) against its time in the dense form.
+struct ListRule {
+    bool on = false;
+    double dense_s = 0.0;     // dense form: seconds per node
+    double pair_s = 0.0;      // lists: per pair of a node's samples
+    double entry_s = 0.0;     // and per sample of a node
+    double fixed_s = 0.0;     // and once; less than this is not worth the lists
+    uint32_t min_div = 8;     // at most 1 / min_div of the samples
+    int min_bits = 0;         // bits that a length keeps in the fixed point
+    bool wide = false;        // 32-bit list entries whatever the tables' sizes
+};
+
+// Sparse nodes of a plan: which embedded rows are summed through sample
+// lists, and their lengths' fixed-point scale.
+struct SparseNodes {
+    std::vector<int32_t> id_of_row;  // per embedded row: sparse node, or -1
+    std::vector<uint32_t> row;       // per sparse node: its row
+    double scale = 1.0;              // 2^s, exact sums below 2^62
+};
+SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule);
 
 // Host-built layout of the tensor-core operands (see build_gemm_layout).
 struct GemmLayout {
-    std::vector<double> lsorted, scale;  // lengths in column order; 2^-s_c per chunk
+    SparseNodes sparse;
+    // lengths in column order (contracted columns, then the sparse nodes);
+    // 2^-s_c per chunk
+    std::vector<double> lsorted, scale;
+    uint32_t k_pad = 0;                  // contracted columns, whole K blocks
     std::vector<uint32_t> chunk_end;     // first K block after chunk c
     std::vector<uint8_t> digits;         // u, s, v, t rows of k_pad bytes
     std::vector<int32_t> parent_col;     // embedded parent's column, or -1
     std::vector<int32_t> start_of_obs;   // column where a tree observation's path starts, or -1
     std::string error;
 };
-GemmLayout build_gemm_layout(const FlatTree &tree);
+GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule);
 
 struct PlanImpl {
     MethodSpec spec;
@@ -412,9 +447,11 @@ struct PlanImpl {
     // tensor-core layout built on a worker thread while setup() uploads
     // (built in setup_gemm instead when no thread can be started)
     std::future<GemmLayout> gemm_layout;
-    void start_gemm_layout(const FlatTree &tree) {
+    ListRule list_rule;
+    void start_gemm_layout(const TableSet &set, const FlatTree &tree) {
+        list_rule = tc_list_rule(set, tree.n_embedded);
         try {
-            gemm_layout = std::async(std::launch::async, build_gemm_layout, std::cref(tree));
+            gemm_layout = std::async(std::launch::async, build_gemm_layout, std::cref(set), std::cref(tree), list_rule);
         } catch (const std::exception &) {
             gemm_layout = std::future<GemmLayout>();
         }
@@ -507,6 +544,17 @@ struct PlanImpl {
     int *d_error = nullptr;
     CUtensorMap map_A{}, map_B{};
     int setup_gemm(const TableSet &set, const FlatTree &tree);
+    ListRule tc_list_rule(const TableSet &set, uint32_t n_rows) const;
+    // lists of the sparse nodes of every group (lengths per node on the device)
+    uint32_t n_sparse = 0;
+    unsigned long long *d_sparse_q = nullptr;
+    unsigned long long *d_shared = nullptr;  // shared sums of the widest group
+    double sparse_unit = 1.0;                // 2^-s
+    int setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp, const double *d_len_of_node);
+    int reset_lists(cudaStream_t s, const Group &g);
+    int shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &out, uint32_t col0, uint32_t col1);
+    void gemm_args(tc::GemmArgs &a, const Group &g, const dev::OutSpec &out) const;
+    int gemm_rows(cudaStream_t s, const Group &g);
     int build_units(uint32_t band);
     int tune_band();
     bool device_error_pending();
@@ -654,7 +702,8 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
         // 8-bit operand rows (A0, A1, B0, B1) over the padded nodes (chunk
         // padding included, allowing for 128 chunks) and r
         const uint64_t kp = (static_cast<uint64_t>(E) + tc::BLOCK_K - 1) / tc::BLOCK_K * tc::BLOCK_K + 128 * tc::BLOCK_K;
-        per_col = 2 * tc::PRODUCTS * kp + sizeof(double);
+        per_col = 2 * tc::PRODUCTS * kp + sizeof(double) +
+                  (list_rule.on ? sizeof(unsigned long long) * max_table_n / 2 : 0);  // shared sums, condensed
     }
     size_t budget = opts.group_bytes;
     if (!budget) {
@@ -737,14 +786,12 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
         for (uint32_t t = g.t0; t < g.t1; t++)
             std::copy(set.tables[t]->totals.begin(), set.tables[t]->totals.end(), g.totals.begin() + tdesc[t].base);
         SSU_CK(upload(&g.d_totals, g.totals.data(), sizeof(double) * g.ld));
-        if (per_table_len) {
-            std::vector<uint32_t> bt(g.ld / 128, 0);
-            for (uint32_t t = g.t0; t < g.t1; t++) {
-                const uint64_t w = std::max<uint64_t>(128, (static_cast<uint64_t>(tdesc[t].n) + 127) / 128 * 128);
-                for (uint64_t c = tdesc[t].base / 128; c < (tdesc[t].base + w) / 128; c++) bt[c] = t;
-            }
-            SSU_CK(upload(&g.d_block_table, bt.data(), sizeof(uint32_t) * bt.size()));
+        std::vector<uint32_t> bt(g.ld / 128, 0);
+        for (uint32_t t = g.t0; t < g.t1; t++) {
+            const uint64_t w = std::max<uint64_t>(128, (static_cast<uint64_t>(tdesc[t].n) + 127) / 128 * 128);
+            for (uint64_t c = tdesc[t].base / 128; c < (tdesc[t].base + w) / 128; c++) bt[c] = t;
         }
+        SSU_CK(upload(&g.d_block_table, bt.data(), sizeof(uint32_t) * bt.size()));
     }
     SSU_CK(upload(&d_tdesc, tdesc.data(), sizeof(dev::TableDesc) * std::max<uint32_t>(n_tables, 1)));
     timer.step("groups");
@@ -1588,18 +1635,85 @@ int PlanImpl::tune_band() {
     return build_units(best_band);
 }
 
-// Tree-only host part of the tensor-core setup (no CUDA call, so it runs on
-// a worker thread while the plan's CSR and tree are uploaded).
-// Embedded nodes grouped by the binary exponent of |length|, largest first,
+// counts[row] += the entries of table t at each tip row.
+void add_entry_counts(const TableSet &set, const FlatTree &tree, size_t t, std::vector<uint64_t> &counts) {
+    const Table &tb = *set.tables[t];
+    for (uint32_t r : tree.leaf_rows) {
+        int32_t o = tree.leaf_obs[r];
+        if (o >= 0 && !set.obs_row.empty()) {
+            const std::vector<int32_t> &m = set.obs_row[t];
+            o = static_cast<size_t>(o) < m.size() ? m[o] : -1;
+        }
+        if (o >= 0 && static_cast<uint32_t>(o) < tb.n_obs) counts[r] += tb.indptr[o + 1] - tb.indptr[o];
+    }
+}
+
+// Every internal row's count becomes the sum over its tips (tip rows hold theirs).
+void sum_over_clades(const FlatTree &tree, std::vector<uint64_t> &counts) {
+    for (uint32_t r : tree.level_rows)  // by height: children first
+        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++) counts[r] += counts[tree.child_rows[c]];
+}
+
+// Embedded rows that are cheaper by sample lists than in the dense form.  The
+// table entries under a node bound its samples (a sample with two of its tips
+// counts twice), so the choice needs the tables' offsets alone.  A row whose
+// length is below 2^(min_bits - 1) units of the fixed point stays out (its
+// rounding would be coarser than the dense form's).
+SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule) {
+    SparseNodes sp;
+    const uint32_t E = tree.n_embedded;
+    sp.id_of_row.assign(E, -1);
+    if (!rule.on || !E) return sp;
+    std::vector<uint64_t> bound(tree.n_nodes, 0);
+    std::vector<double> square(E, 0.0);  // sum over tables of the bound's square
+    uint64_t samples = 0;
+    for (size_t t = 0; t < set.tables.size(); t++) {
+        samples += set.tables[t]->n_samples;
+        std::vector<uint64_t> c(tree.n_nodes, 0);
+        add_entry_counts(set, tree, t, c);
+        sum_over_clades(tree, c);
+        for (uint32_t r = 0; r < tree.n_nodes; r++) bound[r] += c[r];
+        for (uint32_t e = 0; e < E; e++) square[e] += static_cast<double>(c[e]) * static_cast<double>(c[e]);
+    }
+    std::vector<uint8_t> in(E, 0);
+    double total = 0.0, gain = -rule.fixed_s;
+    for (uint32_t e = 0; e < E; e++) {
+        const double by_lists = 0.5 * square[e] * rule.pair_s + static_cast<double>(bound[e]) * rule.entry_s;
+        if (bound[e] * rule.min_div > samples || by_lists >= rule.dense_s) continue;
+        in[e] = 1;
+        gain += rule.dense_s - by_lists;
+        total += tree.length[e];
+    }
+    if (!(gain > 0.0) || !(total > 0.0) || !std::isfinite(total)) return sp;
+    const int s2 = 62 - static_cast<int>(std::ceil(std::log2(total * (1.0 + 1e-12))));
+    if (s2 > 1000 || s2 < -1000) return sp;
+    sp.scale = std::ldexp(1.0, s2);
+    const double lmin = std::ldexp(1.0, rule.min_bits - 1 - s2);
+    for (uint32_t e = 0; e < E; e++)
+        if (in[e] && tree.length[e] >= lmin) sp.row.push_back(e);
+    // numbered by decreasing length of their lists: a sample's nodes then come
+    // in that order, and the lists that lanes read side by side end together
+    std::stable_sort(sp.row.begin(), sp.row.end(), [&](uint32_t x, uint32_t y) { return bound[x] > bound[y]; });
+    for (size_t i = 0; i < sp.row.size(); i++) sp.id_of_row[sp.row[i]] = static_cast<int32_t>(i);
+    return sp;
+}
+
+// Host part of the tensor-core setup (no CUDA call, so it runs on a worker
+// thread while the plan's CSR and tree are uploaded).  Nodes that few samples
+// have go by sample lists (ssu_lists.cuh); the others are contracted:
+// grouped by the binary exponent of |length|, largest first,
 // packed into chunks of whole 128-node K blocks: a chunk closes (its last
 // block padded with zero-length columns) where the exponent changes or at
 // MAX_CHUNK_KB blocks.  Chunk c is scaled by 2^s_c so that its exponent's
 // largest length lies in [2^22, 2^23), which puts all its lengths there;
 // q = round(L 2^s_c) is then written as 256 u v + s t with 8-bit digits
 // (`digits::split_length`).
-GemmLayout build_gemm_layout(const FlatTree &tree) {
+GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule) {
     GemmLayout lay;
     const uint32_t E = tree.n_embedded;
+    lay.sparse = find_sparse_nodes(set, tree, rule);
+    const std::vector<int32_t> &sparse_of = lay.sparse.id_of_row;
+    uint32_t n_dense = 0;  // contracted rows
     // order by binary exponent of |length|, largest first, by row within an
     // exponent (one counting pass): every length of an exponent lies within a
     // factor of two of the others, which is all the chunks need
@@ -1609,9 +1723,11 @@ GemmLayout build_gemm_layout(const FlatTree &tree) {
         std::memcpy(&b, &a, sizeof b);
         return static_cast<int>((b >> 52) & 0x7FF);
     };
-    std::vector<uint32_t> count(kExp, 0), order(E);
+    std::vector<uint32_t> count(kExp, 0), order;
     std::vector<double> emax(kExp, 0.0);
     for (uint32_t e = 0; e < E; e++) {
+        if (sparse_of[e] >= 0) continue;
+        n_dense++;
         const double a = std::fabs(tree.length[e]);
         const int x = exponent(a);
         count[x]++;
@@ -1624,7 +1740,9 @@ GemmLayout build_gemm_layout(const FlatTree &tree) {
             count[x] = at;
             at += c;
         }
-        for (uint32_t e = 0; e < E; e++) order[count[exponent(std::fabs(tree.length[e]))]++] = e;
+        order.resize(n_dense);
+        for (uint32_t e = 0; e < E; e++)
+            if (sparse_of[e] < 0) order[count[exponent(std::fabs(tree.length[e]))]++] = e;
     }
     std::vector<int32_t> col_of_row(tree.n_nodes, -1);
     std::vector<uint32_t> lq;  // 23-bit fixed-point lengths
@@ -1647,7 +1765,7 @@ GemmLayout build_gemm_layout(const FlatTree &tree) {
     bool by_mul = true;
     size_t chunk_first = 0;
     double first = -1.0;
-    for (uint32_t i = 0; i < E; i++) {
+    for (uint32_t i = 0; i < n_dense; i++) {
         const double L = tree.length[order[i]];
         const int xe = exponent(std::fabs(L));
         if (xe != cur || lay.lsorted.size() - chunk_first >= max_cols) {
@@ -1667,9 +1785,19 @@ GemmLayout build_gemm_layout(const FlatTree &tree) {
         lay.lsorted.push_back(L);
         lq.push_back(static_cast<uint32_t>(std::min(std::floor(std::max(x, 0.0) + 0.5), qmax)));
     }
-    if (first < 0) lay.scale.push_back(1.0);  // no embedded node: one chunk of padding
+    if (first < 0) {  // no contracted node: one chunk of padding
+        lay.scale.push_back(1.0);
+        lay.lsorted.push_back(0.0);
+        lq.push_back(0u);
+    }
     pad_to_block();
     const uint32_t k_pad = static_cast<uint32_t>(lay.lsorted.size());
+    lay.k_pad = k_pad;
+    // the sparse nodes' columns follow
+    for (size_t i = 0; i < lay.sparse.row.size(); i++) {
+        col_of_row[lay.sparse.row[i]] = static_cast<int32_t>(lay.lsorted.size());
+        lay.lsorted.push_back(tree.length[lay.sparse.row[i]]);
+    }
     // digits u, s, v, t of every column, one k_pad row each
     lay.digits.assign(static_cast<size_t>(2 * tc::PRODUCTS) * k_pad, 0);
     for (uint32_t c = 0; c < k_pad; c++) {
@@ -1684,7 +1812,7 @@ GemmLayout build_gemm_layout(const FlatTree &tree) {
     std::vector<int32_t> parent_row(tree.n_nodes, -1);
     for (uint32_t r = 0; r < tree.n_nodes; r++)
         for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++) parent_row[tree.child_rows[c]] = r;
-    lay.parent_col.assign(k_pad, -1);
+    lay.parent_col.assign(lay.lsorted.size(), -1);
     for (uint32_t r = 0; r < E; r++) {
         const int32_t p = parent_row[r];
         lay.parent_col[col_of_row[r]] = (p >= 0 && static_cast<uint32_t>(p) < E) ? col_of_row[p] : -1;
@@ -1704,15 +1832,69 @@ GemmLayout build_gemm_layout(const FlatTree &tree) {
     return lay;
 }
 
+// Nodes that the contraction leaves to the sample lists.  A 128-node block
+// takes a work unit 0.40 us (and its share of the unit's ends) and the units
+// run two SMs each, so a node costs 3.6 ns a wave of units however few samples
+// have it; by lists it costs 1 ps a pair of its samples and 60 ps a sample
+// (measured, 25,000 samples x 100,000 tips: all nodes contracted 102.3 ms;
+// nodes in at most 1/20, 1/24, 1/28, 1/36 of the samples by lists 30.6, 29.9,
+// 30.2, 31.0 ms).  Tables of a few hundred samples are one wave:
+// 500 samples x 50,000 tips 432 us contracted, 210 us by this rule; 2,048
+// samples with 5% of 20,000 tips each 323 us contracted, 359 us with lists.
+// UNIFRAC_B200_TC_LISTS: 0 no lists, 1 lists wherever a node allows them, 2
+// the same with the 32-bit entries of larger tables.
+ListRule PlanImpl::tc_list_rule(const TableSet &set, uint32_t n_rows) const {
+    ListRule r;
+    const int mode = env_int("UNIFRAC_B200_TC_LISTS", -1);
+    r.on = mode != 0;
+    uint64_t units = 0;
+    for (const Table *t : set.tables) {
+        const uint64_t nkb = (static_cast<uint64_t>(t->n_samples) + tc::UMMA_M - 1) / tc::UMMA_M;
+        units += nkb * (nkb + 1);  // 256 rows x 128 columns over the upper triangle
+    }
+    const double waves = std::ceil(static_cast<double>(units) / std::max(1, n_sms / 2));
+    r.dense_s = waves * 3.6e-9;
+    r.pair_s = 1e-12;
+    r.entry_s = 6e-11;
+    r.fixed_s = 20e-6;
+    r.min_bits = tc::QBITS;  // as many as the contraction's digits hold
+    if (mode >= 1) {
+        r.dense_s = 1.0;
+        r.fixed_s = 0.0;
+        r.wide = mode == 2;
+    }
+    // the shared sums (8 bytes a pair) must fit beside the result and operands
+    if (r.on && set.tables.size() == 1) {
+        const uint64_t n = set.tables[0]->n_samples, pairs = n * n / 2;
+        if (pairs * 8 > (uint64_t(4) << 30)) {
+            size_t free_b = 0, total_b = 0;
+            int dev_id = 0;
+            uint64_t reserved = 0, used = 0;
+            if (cudaGetDevice(&dev_id) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+                if (cudaMemPool_t p = device_pool(dev_id)) {
+                    cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &reserved);
+                    cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemCurrent, &used);
+                }
+                const double have = 0.9 * (static_cast<double>(free_b) + static_cast<double>(reserved - used));
+                const double need = static_cast<double>(pairs) * (8 + 2 * (spec.fp64 ? 8 : 4)) +
+                                    2.0 * tc::PRODUCTS * static_cast<double>(n) * n_rows;
+                if (need > have) r.on = false;
+            }
+        }
+    }
+    return r;
+}
+
 int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     SetupTimer timer;
-    GemmLayout lay = gemm_layout.valid() ? gemm_layout.get() : build_gemm_layout(tree);
+    GemmLayout lay = gemm_layout.valid() ? gemm_layout.get() : build_gemm_layout(set, tree, list_rule);
     timer.step("gemm_layout");
     if (!lay.error.empty()) {
         last_error = lay.error;
         return kOutputError;
     }
-    k_pad = static_cast<uint32_t>(lay.lsorted.size());
+    k_pad = lay.k_pad;
+    const uint32_t n_cols = static_cast<uint32_t>(lay.lsorted.size());  // contracted and sparse
     n_chunks = static_cast<uint32_t>(lay.chunk_end.size());
     const std::vector<int32_t> &start_of_obs = lay.start_of_obs;
     const uint32_t n_obs_tree = static_cast<uint32_t>(start_of_obs.size());
@@ -1770,10 +1952,25 @@ int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     SSU_CK(alloc(&d_B, tc::PRODUCTS * op_bytes));
     SSU_CK(alloc(&d_r, sizeof(double) * n_pad));
     SSU_CK(upload(&d_lq, lay.digits.data(), lay.digits.size()));
-    SSU_CK(upload(&d_lsorted, lay.lsorted.data(), sizeof(double) * k_pad));
+    SSU_CK(upload(&d_lsorted, lay.lsorted.data(), sizeof(double) * n_cols));
     SSU_CK(upload(&d_chunk_scale, lay.scale.data(), sizeof(double) * n_chunks));
     SSU_CK(upload(&d_chunk_end, lay.chunk_end.data(), sizeof(uint32_t) * n_chunks));
-    SSU_CK(upload(&d_parent_col, lay.parent_col.data(), sizeof(int32_t) * k_pad));
+    SSU_CK(upload(&d_parent_col, lay.parent_col.data(), sizeof(int32_t) * n_cols));
+    if (const int rc = setup_lists(set, tree, lay.sparse, d_lsorted + k_pad)) return rc;
+    if (n_sparse) {
+        uint64_t most = 0;
+        for (Group &g : groups) {
+            std::vector<uint64_t> off(g.t1 - g.t0, 0);
+            uint64_t at = 0;
+            for (uint32_t t = g.t0; t < g.t1; t++) {
+                off[t - g.t0] = at;
+                at += static_cast<uint64_t>(tdesc[t].n) * (tdesc[t].n - 1) / 2;
+            }
+            SSU_CK(upload(&g.d_shared_off, off.data(), sizeof(uint64_t) * off.size()));
+            most = std::max(most, at);
+        }
+        SSU_CK(alloc(&d_shared, sizeof(unsigned long long) * std::max<uint64_t>(most, 1)));
+    }
     SSU_CK(alloc(&d_error, sizeof(int)));
     SSU_CK(cudaMemsetAsync(d_error, 0, sizeof(int), stream));
     if (const char *w = std::getenv("UNIFRAC_B200_WAIT_CYCLES")) gemm_wait_cycles = std::max(0LL, std::atoll(w));
@@ -1785,7 +1982,7 @@ int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     }
     SSU_CK(cudaFuncSetAttribute(tc::unweighted_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 static_cast<int>(tc::SMEM_BYTES)));
-    const size_t bits_smem = sizeof(uint32_t) * (k_pad / 32);
+    const size_t bits_smem = sizeof(uint32_t) * (k_pad / 32 + (n_sparse + 31) / 32);
     if (bits_smem > tc::MAX_BITMAP_BYTES) {
         last_error = "tree too large for the tensor-core presence kernel";
         return kOutputError;
@@ -1811,34 +2008,171 @@ bool PlanImpl::device_error_pending() {
     return h != 0;
 }
 
+// Counters of a group's lists, zeroed before its walk.
+int PlanImpl::reset_lists(cudaStream_t s, const Group &g) {
+    if (!n_sparse) return 0;
+    SSU_CK(cudaMemsetAsync(g.lists.count, 0, sizeof(uint32_t) * g.lists.slots, s));
+    SSU_CK(cudaMemsetAsync(g.lists.cursor, 0, sizeof(unsigned long long), s));
+    return 0;
+}
+
+// Shared sums of the samples in the group's columns [col0, col1).
+int PlanImpl::shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &out, uint32_t col0, uint32_t col1) {
+    if (!n_sparse || col1 <= col0) return 0;
+    uint32_t n_max = 1;
+    for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);
+    // a row's columns in chunks of whole parts that leave two blocks to an SM
+    const uint32_t part_rows = dev::list_part_rows(n_max, g.lists.parts);
+    const uint32_t chunk = std::max(1u, kSharedCols / part_rows);  // parts per chunk
+    const uint32_t chunks = (g.lists.parts + chunk - 1) / chunk;
+    const uint32_t cols = std::min<uint32_t>(n_max, std::min(kSharedCols, chunk * part_rows));
+    const uint32_t threads = cols > 4096 ? 768 : cols > 2048 ? 512 : 256;
+    const size_t smem = 2 * sizeof(uint32_t) * cols;
+    const dim3 grid(col1 - col0, chunks);
+    if (g.lists.wide)
+        dev::shared_sums_kernel<uint32_t><<<grid, threads, smem, s>>>(g.lists, out, col0, cols, chunk);
+    else
+        dev::shared_sums_kernel<uint16_t><<<grid, threads, smem, s>>>(g.lists, out, col0, cols, chunk);
+    launches++;
+    SSU_CK(cudaGetLastError());
+    return 0;
+}
+
+// Lists of the sparse nodes: offsets per (table, node) from the tables' entry
+// counts, buffers, fixed-point lengths.
+int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp,
+                          const double *d_len_of_node) {
+    n_sparse = static_cast<uint32_t>(sp.row.size());
+    sparse_unit = 1.0 / sp.scale;
+    if (!n_sparse) return 0;
+    SSU_CK(alloc(&d_sparse_q, sizeof(unsigned long long) * n_sparse));
+    dev::fixed_lengths_kernel<<<(n_sparse + 255) / 256, 256, 0, stream>>>(d_len_of_node, n_sparse, sp.scale,
+                                                                         d_sparse_q);
+    SSU_CK(cudaGetLastError());
+    for (Group &g : groups) {
+        const uint32_t tg = g.t1 - g.t0;
+        dev::ListArgs &la = g.lists;
+        la.n_nodes = n_sparse;
+        la.q = d_sparse_q;
+        la.block_table = g.d_block_table;
+        la.tables = d_tdesc;
+        la.t0 = g.t0;
+        std::vector<uint32_t> off(static_cast<size_t>(tg) * n_sparse);
+        uint64_t at = 0, ids = 0;  // at: in units of LIST_ALIGN entries
+        for (uint32_t t = g.t0; t < g.t1; t++) {
+            if (tdesc[t].n > 65536 || list_rule.wide) la.wide = 1;
+            std::vector<uint64_t> c(tree.n_nodes, 0);
+            add_entry_counts(set, tree, t, c);
+            sum_over_clades(tree, c);
+            uint32_t *o = off.data() + static_cast<size_t>(t - g.t0) * n_sparse;
+            for (uint32_t e = 0; e < n_sparse; e++) {
+                const uint64_t m = std::min<uint64_t>(c[sp.row[e]], tdesc[t].n);
+                o[e] = static_cast<uint32_t>(at);
+                at += (m + dev::LIST_ALIGN - 1) / dev::LIST_ALIGN;
+                ids += m;
+            }
+        }
+        if (at > UINT32_MAX) {
+            last_error = "too many table entries for the sparse nodes' lists";
+            return kOutputError;
+        }
+        // parts of at least a wave of blocks of the walk
+        la.slots = static_cast<uint64_t>(tg) * n_sparse;
+        la.parts = static_cast<uint32_t>(
+            std::max<uint64_t>(1, std::min<uint64_t>(dev::LIST_PARTS, g.ld / (8 * static_cast<uint64_t>(n_sms)))));
+        uint32_t n_max = 1;
+        for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);
+        while (dev::list_part_rows(n_max, la.parts) > kSharedCols) la.parts *= 2;  // (a part's columns fit a block)
+        std::vector<std::vector<uint32_t>> by_part(la.parts);
+        for (uint32_t t = g.t0; t < g.t1; t++) {
+            const uint32_t n_t = tdesc[t].n, rows = dev::list_part_rows(std::max(n_t, 1u), la.parts);
+            const uint32_t w = std::max<uint32_t>(128, (n_t + 127) / 128 * 128);
+            for (uint32_t c = 0; c < w; c++) by_part[std::min(c / rows, la.parts - 1)].push_back(tdesc[t].base + c);
+        }
+        std::vector<uint32_t> columns;
+        g.part_col.assign(1, 0);
+        for (const std::vector<uint32_t> &v : by_part) {
+            columns.insert(columns.end(), v.begin(), v.end());
+            g.part_col.push_back(static_cast<uint32_t>(columns.size()));
+        }
+        SSU_CK(upload(&g.d_columns, columns.data(), sizeof(uint32_t) * columns.size()));
+        if (la.parts > 1) SSU_CK(alloc(&la.part_count, sizeof(uint32_t) * la.slots * (la.parts - 1)));
+        const size_t bytes = (la.wide ? sizeof(uint32_t) : sizeof(uint16_t)) * at * dev::LIST_ALIGN;
+        uint32_t *d_off = nullptr;
+        SSU_CK(upload(&d_off, off.data(), sizeof(uint32_t) * off.size()));
+        la.off = d_off;
+        SSU_CK(alloc(&la.count, sizeof(uint32_t) * off.size()));
+        SSU_CK(alloc(&la.idx, bytes));
+        // the padding after each list reads as sample 0, which no row adds
+        SSU_CK(cudaMemsetAsync(la.idx, 0, std::max<size_t>(bytes, 1), stream));
+        SSU_CK(alloc(&la.node, sizeof(uint32_t) * std::max<uint64_t>(ids, 1)));
+        SSU_CK(alloc(&la.node_ptr, sizeof(unsigned long long) * g.ld));
+        SSU_CK(alloc(&la.node_cnt, sizeof(uint32_t) * g.ld));
+        SSU_CK(alloc(&la.cursor, sizeof(unsigned long long)));
+        SSU_CK(alloc(&la.rs, sizeof(unsigned long long) * g.ld));
+        SSU_CK(cudaStreamSynchronize(stream));  // the host offsets are released on return
+    }
+    constexpr int smem = static_cast<int>(2 * sizeof(uint32_t) * kSharedCols);
+    SSU_CK(cudaFuncSetAttribute(dev::shared_sums_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SSU_CK(cudaFuncSetAttribute(dev::shared_sums_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return 0;
+}
+
+// Operand rows, one-sided sums and the sparse nodes' lists of a group.
+int PlanImpl::gemm_rows(cudaStream_t s, const Group &g) {
+    if (const int rc = reset_lists(s, g)) return rc;
+    const size_t bits_smem = sizeof(uint32_t) * (k_pad / 32 + (n_sparse + 31) / 32);
+    const dev::ListArgs &la = g.lists;
+    for (uint32_t p = 0; p < la.parts; p++) {
+        const uint32_t c0 = n_sparse ? g.part_col[p] : 0;
+        const uint32_t c1 = n_sparse ? g.part_col[p + 1] : static_cast<uint32_t>(g.ld);
+        if (p)
+            SSU_CK(cudaMemcpyAsync(la.part_count + (p - 1) * la.slots, la.count, sizeof(uint32_t) * la.slots,
+                                   cudaMemcpyDeviceToDevice, s));
+        if (c1 <= c0) continue;
+        tc::presence_rows_kernel<<<c1 - c0, 256, bits_smem, s>>>(
+            g.d_sample_ptr, g.d_start_col, d_parent_col, d_lq, d_lsorted, static_cast<uint32_t>(g.ld), k_pad,
+            static_cast<uint64_t>(n_pad) * k_pad, d_A, d_B, d_r, n_sparse ? g.d_columns + c0 : nullptr, la);
+        launches++;
+    }
+    SSU_CK(cudaGetLastError());
+    return 0;
+}
+
+void PlanImpl::gemm_args(tc::GemmArgs &a, const Group &g, const dev::OutSpec &out) const {
+    a.tiles = g.d_tiles;
+    a.n_tiles = g.n_tiles;
+    a.tables = d_tdesc;
+    a.n_kblocks = k_pad / tc::BLOCK_K;
+    a.plane_rows = n_pad;
+    a.n_chunks = n_chunks;
+    a.chunk_end = d_chunk_end;
+    a.chunk_scale = d_chunk_scale;
+    a.r = d_r;
+    a.shared.S = n_sparse ? d_shared : nullptr;
+    a.shared.off = g.d_shared_off;
+    a.rs = g.lists.rs;
+    a.t0 = g.t0;
+    a.unit = sparse_unit;
+    a.normalized = spec.method == Method::unweighted ? 1 : 0;
+    a.out_fp64 = spec.fp64 ? 1 : 0;
+    a.out = out;
+    a.error = d_error;
+    a.wait_cycles = gemm_wait_cycles;
+    a.stall = union_stall;
+}
+
 int PlanImpl::execute_gemm(cudaStream_t s, const dev::OutSpec &out) {
     launches = 0;
     if (timed()) SSU_CK(cudaEventRecord(ev[0], s));
-    const size_t bits_smem = sizeof(uint32_t) * (k_pad / 32);
     for (size_t gi = 0; gi < groups.size(); gi++) {
         const Group &g = groups[gi];
-        tc::presence_rows_kernel<<<static_cast<uint32_t>(g.ld), 256, bits_smem, s>>>(
-            g.d_sample_ptr, g.d_start_col, d_parent_col, d_lq, d_lsorted, static_cast<uint32_t>(g.ld), k_pad,
-            static_cast<uint64_t>(n_pad) * k_pad, d_A, d_B, d_r);
-        launches++;
+        if (const int rc = gemm_rows(s, g)) return rc;
         if (gi == 0 && timed()) SSU_CK(cudaEventRecord(ev[1], s));
         if (g.n_tiles) {
             tc::GemmArgs a{};
-            a.tiles = g.d_tiles;
-            a.n_tiles = g.n_tiles;
-            a.tables = d_tdesc;
-            a.n_kblocks = k_pad / tc::BLOCK_K;
-            a.plane_rows = n_pad;
-            a.n_chunks = n_chunks;
-            a.chunk_end = d_chunk_end;
-            a.chunk_scale = d_chunk_scale;
-            a.r = d_r;
-            a.normalized = spec.method == Method::unweighted ? 1 : 0;
-            a.out_fp64 = spec.fp64 ? 1 : 0;
-            a.out = out;
-            a.error = d_error;
-            a.wait_cycles = gemm_wait_cycles;
-            a.stall = union_stall;
+            gemm_args(a, g, out);
+            if (const int rc = shared_sums(s, g, a.shared, 0, static_cast<uint32_t>(g.ld))) return rc;
             // two CTAs (one cluster) per work unit, started in unit order
             tc::unweighted_tc_kernel<<<2 * g.n_tiles, tc::THREADS, tc::SMEM_BYTES, s>>>(map_A, map_B, a);
             launches++;
@@ -1881,11 +2215,7 @@ int PlanImpl::execute_gemm_overlap(void *host) {
     out.mode = 0;
     out.ptr = d_full;
     zero_diagonal(s, d_full);  // the units never write the diagonal
-    const size_t bits_smem = sizeof(uint32_t) * (k_pad / 32);
-    tc::presence_rows_kernel<<<static_cast<uint32_t>(g.ld), 256, bits_smem, s>>>(
-        g.d_sample_ptr, g.d_start_col, d_parent_col, d_lq, d_lsorted, static_cast<uint32_t>(g.ld), k_pad,
-        static_cast<uint64_t>(n_pad) * k_pad, d_A, d_B, d_r);
-    launches++;
+    if (const int rc = gemm_rows(s, g)) return rc;
     SSU_CK(cudaEventRecord(band_ev[nb], s));
     SSU_CK(cudaStreamWaitEvent(s1, band_ev[nb], 0));
     for (uint32_t p = 0; p < nb; p++) {
@@ -1893,21 +2223,11 @@ int PlanImpl::execute_gemm_overlap(void *host) {
         const uint32_t u0 = g.band_unit[p], u1 = g.band_unit[p + 1];
         if (u1 > u0) {
             tc::GemmArgs a{};
+            gemm_args(a, g, out);
             a.tiles = g.d_tiles + u0;
             a.n_tiles = u1 - u0;
-            a.tables = d_tdesc;
-            a.n_kblocks = k_pad / tc::BLOCK_K;
-            a.plane_rows = n_pad;
-            a.n_chunks = n_chunks;
-            a.chunk_end = d_chunk_end;
-            a.chunk_scale = d_chunk_scale;
-            a.r = d_r;
-            a.normalized = spec.method == Method::unweighted ? 1 : 0;
-            a.out_fp64 = spec.fp64 ? 1 : 0;
-            a.out = out;
-            a.error = d_error;
-            a.wait_cycles = gemm_wait_cycles;
-            a.stall = union_stall;
+            // the band's units read the shared sums of the band's rows alone
+            if (const int rc = shared_sums(st, g, a.shared, g.band_row[p], std::min(g.band_row[p + 1], n_t))) return rc;
             tc::unweighted_tc_kernel<<<2 * (u1 - u0), tc::THREADS, tc::SMEM_BYTES, st>>>(map_A, map_B, a);
             launches++;
         }
@@ -1973,7 +2293,7 @@ int Plan::create(const Table &table, const FlatTree &tree, const MethodSpec &spe
     set.tables.push_back(&table);
     set.embedded.push_back(tree.n_embedded);
     m.gemm = use_tensor_cores(spec, set, tree, false);
-    if (m.gemm) m.start_gemm_layout(tree);
+    if (m.gemm) m.start_gemm_layout(set, tree);
     int rc = m.setup(set, tree, BatchOptions{});
     if (!rc) rc = m.gemm ? m.setup_gemm(set, tree) : spec.fp64 ? m.setup_method<double>() : m.setup_method<float>();
     if (rc) {
@@ -2001,7 +2321,7 @@ int Plan::create_batch(const TableSet &set, const FlatTree &tree, const MethodSp
     m.stream = static_cast<cudaStream_t>(stream);
     m.autotune = resolve_autotune(opts.autotune, true);
     m.gemm = use_tensor_cores(spec, set, tree, true);
-    if (m.gemm) m.start_gemm_layout(tree);
+    if (m.gemm) m.start_gemm_layout(set, tree);
     int rc = m.setup(set, tree, opts);
     if (!rc) rc = m.gemm ? m.setup_gemm(set, tree) : spec.fp64 ? m.setup_method<double>() : m.setup_method<float>();
     if (rc) {

@@ -34,6 +34,11 @@
 // 2^-s_c.  The only rounding before fp64 is the quantisation of each length
 // (relative at most 2^-23).
 //
+// Only nodes that enough samples have are contracted: a node costs the
+// contraction the same however few samples have it, so nodes that few have
+// are summed exactly through sample lists first (ssu_lists.cuh) and their
+// part of G is added when the distances are formed.
+//
 // Work unit: a cluster of two CTAs (cta_group::2) owns 256 rows k x 128
 // columns l of one table.  Per 32 nodes, two MMAs of M = 256 (128 rows per
 // CTA) x N = 128 (64 columns of B held by each CTA), one per product, into
@@ -55,6 +60,7 @@
 
 #include "ssu_digits.hpp"
 #include "ssu_kernels.cuh"
+#include "ssu_lists.cuh"
 
 namespace ssu {
 namespace tc {
@@ -76,15 +82,21 @@ constexpr int TMEM_COLS = 512;
 constexpr size_t MAX_BITMAP_BYTES = 200 * 1024;  // presence bitmap of one sample in shared memory
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
+constexpr int EPI_ROWS = 4;       // rows of a warp finished together in the epilogue
+static_assert(ROWS % (EPI_WARPS * EPI_ROWS) == 0, "whole groups of rows per epilogue warp");
+constexpr int EPI_LD = COLS + 1;  // row stride of the epilogue's shared tile (conflict-free both ways)
 constexpr uint32_t A_BYTES = ROWS * BLOCK_K;    // one product's A tile
 constexpr uint32_t B_BYTES = B_ROWS * BLOCK_K;  // one product's B tile
 constexpr uint32_t STAGE_BYTES = PRODUCTS * (A_BYTES + B_BYTES);  // per CTA
-constexpr size_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+// ring, barriers, one-sided sums of the unit (and the ring's alignment)
+constexpr size_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + sizeof(double) * (2 * ROWS + COLS);
+static_assert(ROWS == COLS, "one loop loads the one-sided sums of rows and columns");
 static_assert(UMMA_N % 16 == 0 && UMMA_N <= 256, "kind::i8 with M = 256 takes N in multiples of 16 up to 256");
 static_assert(PRODUCTS * UMMA_N <= ACC_STRIDE && 2 * ACC_STRIDE <= TMEM_COLS,
               "two accumulators must fit the TMEM allocation");
 static_assert(A_BYTES % 1024 == 0 && B_BYTES % 1024 == 0, "operand tiles must keep 1024-byte swizzle alignment");
 static_assert(SMEM_BYTES <= 227 * 1024, "stage ring exceeds shared memory");
+static_assert(sizeof(double) * ROWS * EPI_LD <= STAGES * STAGE_BYTES, "the epilogue's tile lies over the ring");
 static_assert(static_cast<long long>(MAX_CHUNK_KB) * BLOCK_K * MAX_PART < (1LL << 31), "product sums must stay exact");
 static_assert((static_cast<long long>(MAX_PART) << 8) + MAX_PART >= (1LL << QBITS) - 1,
               "256 u v + s t must reach the largest length");
@@ -102,6 +114,11 @@ struct GemmArgs {
     const uint32_t *chunk_end;  // first K block after chunk c
     const double *chunk_scale;  // 2^-s_c per chunk
     const double *r;            // per operand row: fp64 sum of the present lengths
+    // sparse nodes, not contracted: G gains (rs[k] - shared[k][l]) * unit
+    dev::SharedOut shared;      // S == nullptr: none
+    const unsigned long long *rs;
+    uint32_t t0;                // the group's first table
+    double unit;
     int normalized;
     int out_fp64;
     dev::OutSpec out;
@@ -213,6 +230,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// barrier of the epilogue warps
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory"); }
+
 __device__ __forceinline__ void fail(int *shared_abort, int *global_err, int code) {
     atomicExch(shared_abort, 1);
     atomicCAS(global_err, ERR_NONE, code);
@@ -230,6 +250,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     uint64_t *done = acce + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
+    int *emit_flag = abort_flag + 1;
+    double *rk_s = reinterpret_cast<double *>(smem + STAGES * STAGE_BYTES + 256);  // [ROWS] r of the rows
+    double *rl_s = rk_s + ROWS;                                                    // [COLS] r of the columns
+    unsigned long long *rs_s = reinterpret_cast<unsigned long long *>(rl_s + COLS);  // [ROWS] sparse sums
 
     const uint32_t rank = cluster_rank();
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -305,7 +329,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             // MMA issuer for the pair
             constexpr uint32_t idesc = i8_idesc(UMMA_M, UMMA_N);
             uint32_t kb = 0;
+            // (a chunk's end is loaded while the chunk before it is issued: the
+            // load's latency at each chunk's start left the tensor cores idle
+            // for over 1 us a chunk)
+            uint32_t next_end = args.chunk_end[0];
             for (uint32_t c = 0; c < nchunks && !*vabort; c++) {
+                const uint32_t kend = next_end;
+                if (c + 1 < nchunks) next_end = args.chunk_end[c + 1];
                 const uint32_t buf = c & 1, reuse = c >> 1;
                 if (reuse > 0 && !mbar_wait_cl(acce + buf, (reuse - 1) & 1, budget)) {
                     fail(abort_flag, args.error, ERR_ACC_EMPTY_WAIT);
@@ -313,7 +343,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 }
                 tc_fence_after();
                 const uint32_t d = tmem + buf * ACC_STRIDE;
-                const uint32_t kstart = kb, kend = args.chunk_end[c];
+                const uint32_t kstart = kb;
                 bool good = true;
                 for (; kb < kend; kb++) {
                     const uint32_t s = kb % STAGES, use = kb / STAGES;
@@ -344,24 +374,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             umma_commit_pair(done);
         }
     } else {
-        // epilogue: warp w reads TMEM lanes 32*(w%4).. and half (w-2)/4 of the
+        // epilogue: warp w reads TMEM lanes 32*(w%4).. and part (w-2)/4 of the
         // 128 columns, each column's two product sums
         const int q = warp & 3;
-        const int half = (warp - 2) >> 2;
-        constexpr int HC = COLS / 2;  // columns per epilogue warp
+        const int part = (warp - 2) >> 2;
+        constexpr int HC = COLS * 4 / EPI_WARPS;  // columns per epilogue warp
         double acc[HC];
 #pragma unroll
         for (int i = 0; i < HC; i++) acc[i] = 0.0;
+        // one-sided sums of the unit's rows and columns, for the distances
+        for (int i = threadIdx.x - 64; i < ROWS; i += 32 * EPI_WARPS) {
+            const bool in = k0 + i < td.n;
+            rk_s[i] = in ? args.r[td.base + k0 + i] : 0.0;
+            rs_s[i] = in && args.shared.S ? args.rs[td.base + k0 + i] : 0ull;
+            rl_s[i] = l0 + i < td.n ? args.r[td.base + l0 + i] : 0.0;
+        }
+        double next_scale = args.chunk_scale[0];
         for (uint32_t c = 0; c < nchunks; c++) {
             const uint32_t buf = c & 1, use = c >> 1;
+            const double sc = next_scale;
+            if (c + 1 < nchunks) next_scale = args.chunk_scale[c + 1];
             if (*vabort || !mbar_wait_cl(accf + buf, use & 1, budget)) {
                 fail(abort_flag, args.error, ERR_ACC_FULL_WAIT);
                 ok = false;
                 break;
             }
             tc_fence_after();
-            const double sc = args.chunk_scale[c];
-            const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * ACC_STRIDE + half * HC;
+            const uint32_t base = tmem + (static_cast<uint32_t>(q * 32) << 16) + buf * ACC_STRIDE + part * HC;
 #pragma unroll
             for (int g = 0; g < HC / 16; g++) {
                 // 16 columns of each product
@@ -379,28 +418,93 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acce0 + buf * 8);
         }
+        // The unit's G goes through shared memory (the ring: every stage has
+        // been read once the last chunk is complete), so that the sparse
+        // nodes' sums are read, and the rows and their mirror images written,
+        // along rows.  Straight from the accumulator's layout (a row per
+        // lane) every load and store touched 32 rows: about 70 us a unit.
         const uint32_t n = td.n;
-        const uint32_t k = k0 + q * 32 + lane;
-        if (ok && !*vabort && k < n) {
+        double *tile_s = reinterpret_cast<double *>(smem);  // [ROWS][EPI_LD]
+        if (ok) {  // (a warp that gave up has set the abort flag)
+#pragma unroll
+            for (int j = 0; j < HC; j++) tile_s[(q * 32 + lane) * EPI_LD + part * HC + j] = acc[j];
+        }
+        epilogue_sync();
+        // one decision for all epilogue warps: they meet at the barriers below
+        if (warp == 2 && lane == 0) *emit_flag = *vabort ? 0 : 1;
+        epilogue_sync();
+        if (*reinterpret_cast<volatile int *>(emit_flag)) {
             dev::OutSpec o = args.out;
             if (o.mode == 0)
                 o.ptr = static_cast<char *>(o.ptr) + td.out_off * (args.out_fp64 ? sizeof(double) : sizeof(float));
-            const double *rt = args.r + td.base;
-            const double rk = rt[k];
-            const uint32_t lb = l0 + half * HC;
-            // fully unrolled: acc stays in registers
+            double rl[COLS / 32];
 #pragma unroll
-            for (int j = 0; j < HC; j++) {
-                const uint32_t l = lb + j;
-                if (k < l && l < n) {
-                    const double rl = rt[l];
-                    const double g = acc[j];
-                    const double x = 2.0 * g + (rl - rk);
-                    const double v = args.normalized ? x / (rl + g) : x;
-                    if (o.mode == 0 && !args.out_fp64)
-                        dev::emit_pair<float>(o, n, k, l, static_cast<float>(v));
-                    else
-                        dev::emit_pair<double>(o, n, k, l, v);
+            for (int i = 0; i < COLS / 32; i++) rl[i] = rl_s[lane + 32 * i];
+            // EPI_ROWS rows of a warp at a time: their sparse sums are all in
+            // flight together (a row at a time waited out the memory's latency
+            // 16 times: 35 us a unit)
+            const unsigned long long *S = args.shared.S ? dev::shared_row(args.shared, td, tile.z - args.t0, 0) : nullptr;
+            const bool packed = args.shared.off != nullptr;
+            for (uint32_t r0 = warp - 2; r0 < ROWS; r0 += EPI_WARPS * EPI_ROWS) {
+                if (k0 + r0 >= n) break;
+                unsigned long long sh[EPI_ROWS][COLS / 32], rsk[EPI_ROWS];
+                double rk[EPI_ROWS];
+#pragma unroll
+                for (int u = 0; u < EPI_ROWS; u++) {
+                    const uint32_t k = k0 + r0 + u * EPI_WARPS;
+                    const uint64_t kk = k;
+                    // (row k relative to row 0, see shared_row)
+                    const uint64_t ro = packed ? kk * (2ull * n - kk - 1) / 2 - kk : kk * n;
+                    rk[u] = rk_s[k - k0];
+                    rsk[u] = rs_s[k - k0];
+#pragma unroll
+                    for (int i = 0; i < COLS / 32; i++) {
+                        const uint32_t l = l0 + lane + 32 * i;
+                        sh[u][i] = S && k < l && l < n ? S[ro + l] : 0ull;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < EPI_ROWS; u++) {
+                    const uint32_t k = k0 + r0 + u * EPI_WARPS;
+                    double *ts = tile_s + (r0 + u * EPI_WARPS) * EPI_LD;
+#pragma unroll
+                    for (int i = 0; i < COLS / 32; i++) {
+                        const uint32_t l = l0 + lane + 32 * i;
+                        if (k < l && l < n) {
+                            const double g = fma(static_cast<double>(rsk[u] - sh[u][i]), args.unit, ts[lane + 32 * i]);
+                            const double x = 2.0 * g + (rl[i] - rk[u]);
+                            const double v = args.normalized ? x / (rl[i] + g) : x;
+                            if (o.mode != 0) {
+                                dev::emit_pair<double>(o, n, k, l, v);
+                            } else {
+                                ts[lane + 32 * i] = v;
+                                const uint64_t at = static_cast<uint64_t>(k) * n + l;
+                                if (args.out_fp64)
+                                    static_cast<double *>(o.ptr)[at] = v;
+                                else
+                                    static_cast<float *>(o.ptr)[at] = static_cast<float>(v);
+                            }
+                        }
+                    }
+                }
+            }
+            epilogue_sync();
+            if (o.mode == 0) {
+                for (uint32_t col = warp - 2; col < COLS; col += EPI_WARPS) {
+                    const uint32_t l = l0 + col;
+                    if (l >= n) break;
+#pragma unroll
+                    for (int i = 0; i < ROWS / 32; i++) {
+                        const uint32_t k = k0 + lane + 32 * i;
+                        if (k < l) {
+                            const double v = tile_s[(lane + 32 * i) * EPI_LD + col];
+                            const uint64_t at = static_cast<uint64_t>(l) * n + k;
+                            if (args.out_fp64)
+                                static_cast<double *>(o.ptr)[at] = v;
+                            else
+                                static_cast<float *>(o.ptr)[at] = static_cast<float>(v);
+                        }
+                    }
                 }
             }
         }
@@ -489,34 +593,30 @@ __global__ void __launch_bounds__(1024) exclusive_scan_kernel(const uint32_t *__
     }
 }
 
-// Presence rows for the contraction, one CTA per sample (padding rows too):
+// Presence rows for the contraction, one CTA per sample (padding rows too;
+// `column`: the launch's columns, nullptr: all):
 // walk up from every present tip, marking embedded ancestors in a shared
-// bitmap (stopping at nodes already marked), then write the sample's rows of
+// bitmap over the contracted columns [0, k_pad) and then the sparse nodes
+// (stopping at nodes already marked), then write the sample's rows of
 // A0 = X u, A1 = X s, B0 = (1 - X) v and B1 = (1 - X) t (8-bit, 16 nodes and
 // 16 bytes per store; A1 and B1 `plane` bytes after A0 and B0), and
-// r = sum L of the present nodes (fp64, fixed reduction order).  lq holds
-// the node digits u, s, v, t: digit i at lq + i * k_pad.
-__global__ void presence_rows_kernel(const uint32_t *__restrict__ sample_ptr, const int32_t *__restrict__ start_col,
-                                     const int32_t *__restrict__ parent_col, const uint8_t *__restrict__ lq,
-                                     const double *__restrict__ l_sorted, uint32_t n, uint32_t k_pad, uint64_t plane,
-                                     uint8_t *__restrict__ A, uint8_t *__restrict__ B, double *__restrict__ r) {
-    extern __shared__ uint32_t bits[];  // k_pad / 32 words
+// r = sum L of the present nodes (fp64, fixed reduction order), and the
+// sample's entries of the sparse nodes' lists.  lq holds the node digits u,
+// s, v, t: digit i at lq + i * k_pad.
+__global__ void __launch_bounds__(256)
+    presence_rows_kernel(const uint32_t *__restrict__ sample_ptr, const int32_t *__restrict__ start_col,
+                         const int32_t *__restrict__ parent_col, const uint8_t *__restrict__ lq,
+                         const double *__restrict__ l_sorted, uint32_t n, uint32_t k_pad, uint64_t plane,
+                         uint8_t *__restrict__ A, uint8_t *__restrict__ B, double *__restrict__ r,
+                         const uint32_t *__restrict__ column, const dev::ListArgs la) {
+    extern __shared__ uint32_t bits[];  // k_pad / 32 words, then the sparse nodes'
     __shared__ double red[256];
-    const uint32_t j = blockIdx.x;
-    const uint32_t words = k_pad / 32;
+    const uint32_t j = column ? column[blockIdx.x] : blockIdx.x;
+    const uint32_t sp_words = (la.n_nodes + 31) / 32;
+    const uint32_t words = k_pad / 32 + sp_words;
     for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) bits[w] = 0u;
     __syncthreads();
-    if (j < n) {
-        for (uint32_t e = sample_ptr[j] + threadIdx.x; e < sample_ptr[j + 1]; e += blockDim.x) {
-            int32_t c = start_col[e];
-            while (c >= 0) {
-                const uint32_t m = 1u << (c & 31);
-                const uint32_t old = atomicOr(&bits[c >> 5], m);
-                if (old & m) break;
-                c = parent_col[c];
-            }
-        }
-    }
+    if (j < n) dev::mark_paths(start_col + sample_ptr[j], sample_ptr[j + 1] - sample_ptr[j], parent_col, bits);
     __syncthreads();
     const uint64_t row = static_cast<uint64_t>(j) * k_pad;
     double part = 0.0;
@@ -542,6 +642,7 @@ __global__ void presence_rows_kernel(const uint32_t *__restrict__ sample_ptr, co
         for (int t = 0; t < 16; t++)
             if ((b >> t) & 1u) part += l_sorted[c16 + t];
     }
+    if (la.n_nodes) dev::write_lists(la, j, bits + k_pad / 32, sp_words, l_sorted + k_pad, part);
     red[threadIdx.x] = part;
     __syncthreads();
     if (threadIdx.x == 0) {
