@@ -502,3 +502,87 @@ def test_page_locked_results_are_recycled(ssu):
         assert st == 0
         assert res.contents.flags & 0x2000, "result not page-locked"
         L.destroy_mat_full_fp64(ctypes.byref(res))
+
+
+# ---- fp64 unweighted in whole numbers (sample lists + presence words)
+
+def _stripe_mode(monkeypatch, call):
+    """`call` with the presence-word stripe form over the embedding (the general path)."""
+    monkeypatch.setenv("UNIFRAC_B200_UNWEIGHTED_MODE", "stripe")
+    try:
+        return call()
+    finally:
+        monkeypatch.delenv("UNIFRAC_B200_UNWEIGHTED_MODE")
+
+
+@pytest.mark.parametrize("n,n_tips,density", [(1, 40, 0.2), (2, 40, 0.2), (31, 70, 0.2), (33, 1200, 0.01), (129, 300, 0.9),
+                                              (640, 2000, 0.02), (1501, 400, 0.02), (2433, 500, 0.01)])
+@pytest.mark.parametrize("method", ["unweighted_fp64", "unweighted_unnormalized_fp64"])
+def test_whole_number_unweighted_matches_the_stripe_form(ssu, monkeypatch, method, n, n_tips, density):
+    """Both tile shapes (32 x 32 and 128 x 64), nodes by lists alone, by words
+    alone and by both, explicit zeros and empty samples, a walk in two parts;
+    full matrix, window, condensed, bypassed tips."""
+    tree, table = _case(500 + n, n_tips=n_tips, n_samples=n, density=density, drop=5)
+    rng = np.random.default_rng(n)
+    table.data[rng.random(table.data.shape[0]) < 0.1] = 0.0
+    table.data[np.isin(table.indices, [n // 2])] = 0.0
+    stop = (n + 1) // 2
+    calls = [lambda: ssu.one_off_matrix(tree, table, method)[0],
+             lambda: ssu.one_off_matrix(tree, table, method, bypass_tips=True)[0],
+             lambda: ssu.one_off(tree, table, method)[0],
+             lambda: ssu.partial(tree, table, method, stop // 3, stop)[0]]
+    for call in calls if n > 1 else calls[:3]:
+        got, ref = call(), _stripe_mode(monkeypatch, call)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+        check_fp64(np.nan_to_num(got), np.nan_to_num(ref))
+
+
+def test_whole_number_unweighted_close_and_identical_samples(ssu, oracle_mod):
+    """Samples equal to another one, or differing by one of the shortest tips:
+    their tiles are recomputed in the stripe form."""
+    tree, table = _case(77, n_tips=900, n_samples=150, density=0.1, drop=0)
+    tree.lengths = np.where(tree.lengths > 0, tree.lengths * 10.0 ** np.random.default_rng(3).uniform(-6, 0, tree.lengths.shape), 0.0)
+    dense = table.dense()
+    lengths = dict(zip(tree.tip_names(), tree.tip_lengths()))
+    shortest = np.argsort([lengths[o] for o in table.obs_ids])
+    for j in range(0, 60, 2):
+        dense[:, j + 1] = dense[:, j]
+        if j % 4 == 0:
+            dense[shortest[j % 7], j + 1] = 0.0 if dense[shortest[j % 7], j] > 0 else 3.0
+    table = ssu_synth.Table.from_dense(dense, table.obs_ids, table.sample_ids)
+    for method in ("unweighted_fp64", "unweighted_unnormalized_fp64"):
+        gpu, _ = ssu.one_off_matrix(tree, table, method)
+        check_fp64(gpu, oracle_mod.oracle_one_off(tree, table, method)["matrix"])
+
+
+def test_whole_number_unweighted_in_a_batch_and_as_a_graph(ssu, monkeypatch):
+    tree = ssu_synth.random_binary_tree(800, 0.1, 5)
+    tips = tree.tip_names()
+    tables = [ssu_synth.geometric_table(tips[3 * i:700 + 20 * i], n, 0.05, 10.0, 60 + i)
+              for i, n in enumerate((5, 64, 200, 33))]
+
+    def run():
+        plan = ssu.BatchPlan(tree, tables, "unweighted_fp64")
+        plan.execute()
+        first = plan.results()
+        plan.set_graph(True)
+        for _ in range(2):
+            plan.execute()
+        for a, b in zip(plan.results(), first):
+            np.testing.assert_array_equal(a, b)
+        plan.close()
+        return first
+    for got, ref in zip(run(), _stripe_mode(monkeypatch, run)):
+        check_fp64(got, ref)
+
+
+@pytest.mark.parametrize("what", ["negative length", "infinite count", "negative count"])
+def test_whole_number_unweighted_leaves_other_inputs_to_the_stripe_form(ssu, monkeypatch, what):
+    tree, table = _case(81, n_tips=300, n_samples=70, density=0.1)
+    if what == "negative length":
+        tree.lengths = tree.lengths.copy()
+        tree.lengths[np.flatnonzero(tree.structure)[5]] = -0.01
+    else:
+        table.data[3] = np.inf if what == "infinite count" else -2.0
+    call = lambda: ssu.one_off_matrix(tree, table, "unweighted_fp64")[0]  # noqa: E731
+    np.testing.assert_array_equal(call(), _stripe_mode(monkeypatch, call))

@@ -384,6 +384,7 @@ struct Group {
     // of each part (one extra entry closes the list)
     uint32_t *d_columns = nullptr;
     std::vector<uint32_t> part_col;
+    size_t list_bytes = 0;
     uint64_t *d_shared_off = nullptr;    // condensed shared sums: first element of each table
 };
 
@@ -405,6 +406,8 @@ struct ListRule {
 struct SparseNodes {
     std::vector<int32_t> id_of_row;  // per embedded row: sparse node, or -1
     std::vector<uint32_t> row;       // per sparse node: its row
+    // [table][sparse node]: bound of its samples (entries under the node)
+    std::vector<std::vector<uint32_t>> entries;
     double scale = 1.0;              // 2^s, exact sums below 2^62
 };
 SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule);
@@ -549,8 +552,15 @@ struct PlanImpl {
     uint32_t n_sparse = 0;
     unsigned long long *d_sparse_q = nullptr;
     unsigned long long *d_shared = nullptr;  // shared sums of the widest group
-    double sparse_unit = 1.0;                // 2^-s
-    int setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp, const double *d_len_of_node);
+    double sparse_unit = 1.0;                // 2^-s (contraction)
+    double *d_list_unit = nullptr;           // the same, as the lists' kernels left it
+    int setup_sample_lists(const TableSet &set, const std::vector<int32_t> &start_of_obs);
+    // Fixed-point lengths of n columns, the sparse nodes' from column `first`
+    // on.  `path`: per column the length from it upward (the scale is then
+    // the finest that every sample's sum allows); nullptr: sp.scale
+    int setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp, const double *d_len_of_col,
+                    uint32_t n, uint32_t first, const std::vector<double> *path,
+                    const std::vector<int32_t> &start_of_obs);
     int reset_lists(cudaStream_t s, const Group &g);
     int shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &out, uint32_t col0, uint32_t col1);
     void gemm_args(tc::GemmArgs &a, const Group &g, const dev::OutSpec &out) const;
@@ -565,6 +575,19 @@ struct PlanImpl {
     // event per band of rows
     cudaStream_t aux[2] = {nullptr, nullptr};
     std::vector<cudaEvent_t> band_ev;
+
+    // fp64 unweighted: the nodes that few samples have by sample lists, the
+    // others by presence words, both from a walk over each sample's tips (no
+    // embedding); n_words counts the dense nodes' words, n_words_all all
+    bool walk_bits = false;
+    uint32_t n_words_all = 0;
+    double *d_len_cols = nullptr;
+    unsigned long long *d_nib = nullptr;  // nibble sums of the dense nodes' words
+    PairKernel<double> k_stripe;          // the stripe form, for the tiles that the whole-number form flags
+    ListRule bits_list_rule(const TableSet &set) const;
+    int setup_walk_bits(const TableSet &set, const FlatTree &tree);
+    int walk_bits_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles, uint32_t ntiles,
+                        uint32_t splits, uint32_t rows, bool first, bool last);
 
     // CUDA graph of execute()
     bool graph_on = false, capturing = false;
@@ -764,10 +787,19 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
         return kOutputError;
     }
 
-    // per group: the tips' rows in each table, the per-column totals
+    // per group: the tips' rows in each table, the per-column totals (what the
+    // embedding reads; the forms that walk up from the tips have lists of their own)
+    const bool embeds = !gemm && !walk_bits;
     n_tips = static_cast<uint32_t>(tree.leaf_rows.size());
     const bool per_table_len = !faith && !set.row_active.empty();
     for (Group &g : groups) {
+        std::vector<uint32_t> bt(g.ld / 128, 0);
+        for (uint32_t t = g.t0; t < g.t1; t++) {
+            const uint64_t w = std::max<uint64_t>(128, (static_cast<uint64_t>(tdesc[t].n) + 127) / 128 * 128);
+            for (uint64_t c = tdesc[t].base / 128; c < (tdesc[t].base + w) / 128; c++) bt[c] = t;
+        }
+        SSU_CK(upload(&g.d_block_table, bt.data(), sizeof(uint32_t) * bt.size()));
+        if (!embeds) continue;
         const uint32_t tg = g.t1 - g.t0;
         std::vector<int32_t> tip_obs(static_cast<size_t>(n_tips) * std::max<uint32_t>(tg, 1), -1);
         for (uint32_t i = 0; i < n_tips; i++) {
@@ -786,15 +818,12 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
         for (uint32_t t = g.t0; t < g.t1; t++)
             std::copy(set.tables[t]->totals.begin(), set.tables[t]->totals.end(), g.totals.begin() + tdesc[t].base);
         SSU_CK(upload(&g.d_totals, g.totals.data(), sizeof(double) * g.ld));
-        std::vector<uint32_t> bt(g.ld / 128, 0);
-        for (uint32_t t = g.t0; t < g.t1; t++) {
-            const uint64_t w = std::max<uint64_t>(128, (static_cast<uint64_t>(tdesc[t].n) + 127) / 128 * 128);
-            for (uint64_t c = tdesc[t].base / 128; c < (tdesc[t].base + w) / 128; c++) bt[c] = t;
-        }
-        SSU_CK(upload(&g.d_block_table, bt.data(), sizeof(uint32_t) * bt.size()));
     }
     SSU_CK(upload(&d_tdesc, tdesc.data(), sizeof(dev::TableDesc) * std::max<uint32_t>(n_tables, 1)));
     timer.step("groups");
+    for (auto &e : ev) SSU_CK(cudaEventCreate(&e));
+    host_len.assign(tree.length.begin(), tree.length.begin() + E);
+    if (!embeds) return 0;
 
     // tree
     SSU_CK(upload(&d_tip_rows, tree.leaf_rows.data(), sizeof(uint32_t) * n_tips));
@@ -808,7 +837,6 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
     }
     // embedded lengths in T, rows [0, E); per table (zero where a row is
     // not embedded in that table's own tree) with bypassed tips in a batch
-    host_len.assign(tree.length.begin(), tree.length.begin() + E);
     const uint32_t n_len = per_table_len ? n_tables : 1;
     len_stride = per_table_len ? E : 0;
     if (spec.fp64 || faith) {
@@ -825,7 +853,6 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
                     (!per_table_len || set.row_active[t][e]) ? static_cast<float>(host_len[e]) : 0.0f;
         SSU_CK(upload(reinterpret_cast<float **>(&d_len), len.data(), sizeof(float) * len.size()));
     }
-    for (auto &e : ev) SSU_CK(cudaEventCreate(&e));
     timer.step("tree_upload");
     return 0;
 }
@@ -1456,6 +1483,12 @@ int PlanImpl::execute_T(cudaStream_t s, const dev::OutSpec &out) {
     if (timed()) SSU_CK(cudaEventRecord(ev[0], s));
     for (size_t gi = 0; gi < groups.size(); gi++) {
         const Group &g = groups[gi];
+        if (walk_bits) {
+            if (const int rc = walk_bits_stage(s, g, out, g.d_tiles, g.n_tiles, g.splits, g.rows_per_split, gi == 0,
+                                               gi + 1 == groups.size()))
+                return rc;
+            continue;
+        }
         int rc = embed<T>(s, g);
         if (!rc) rc = prepare<T>(s, g);
         if (rc) return rc;
@@ -1532,7 +1565,9 @@ int PlanImpl::run_windowed(int mode, void *d_out, uint32_t start, uint32_t stop)
     launches = 0;
     const uint32_t nt = static_cast<uint32_t>(tiles.size());
     int rc = 0;
-    if (spec.fp64) {
+    if (walk_bits) {
+        rc = walk_bits_stage(stream, g, o, d_t, nt, s, rows, true, true);
+    } else if (spec.fp64) {
         rc = embed<double>(stream, g);
         if (!rc) rc = prepare<double>(stream, g);
         if (!rc) rc = pair_stage<double>(stream, g, o, d_t, nt, s, rows, true);
@@ -1635,8 +1670,33 @@ int PlanImpl::tune_band() {
     return build_units(best_band);
 }
 
+// Row of every row's parent, or -1 under the root.
+std::vector<int32_t> parent_rows(const FlatTree &tree) {
+    std::vector<int32_t> parent(tree.n_nodes, -1);
+    for (uint32_t r = 0; r < tree.n_nodes; r++)
+        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++)
+            parent[tree.child_rows[c]] = static_cast<int32_t>(r);
+    return parent;
+}
+
+// Starting column of each tree observation: its tip's, or the tip's parent's
+// when tips are bypassed; -1 where neither is embedded.
+std::vector<int32_t> path_starts(const FlatTree &tree, const std::vector<int32_t> &parent_row,
+                                 const std::vector<int32_t> &col_of_row) {
+    uint32_t n_obs = 0;
+    for (uint32_t r : tree.leaf_rows) n_obs = std::max<uint32_t>(n_obs, tree.leaf_obs[r] + 1);
+    std::vector<int32_t> start(n_obs, -1);
+    for (uint32_t r : tree.leaf_rows) {
+        const int32_t obs = tree.leaf_obs[r];
+        if (obs < 0) continue;
+        const int32_t node = r < tree.n_embedded ? static_cast<int32_t>(r) : parent_row[r];
+        start[obs] = (node >= 0 && static_cast<uint32_t>(node) < tree.n_embedded) ? col_of_row[node] : -1;
+    }
+    return start;
+}
+
 // counts[row] += the entries of table t at each tip row.
-void add_entry_counts(const TableSet &set, const FlatTree &tree, size_t t, std::vector<uint64_t> &counts) {
+void add_entry_counts(const TableSet &set, const FlatTree &tree, size_t t, std::vector<uint32_t> &counts) {
     const Table &tb = *set.tables[t];
     for (uint32_t r : tree.leaf_rows) {
         int32_t o = tree.leaf_obs[r];
@@ -1649,9 +1709,12 @@ void add_entry_counts(const TableSet &set, const FlatTree &tree, size_t t, std::
 }
 
 // Every internal row's count becomes the sum over its tips (tip rows hold theirs).
-void sum_over_clades(const FlatTree &tree, std::vector<uint64_t> &counts) {
+void sum_over_clades(const FlatTree &tree, std::vector<uint32_t> &counts) {
     for (uint32_t r : tree.level_rows)  // by height: children first
-        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++) counts[r] += counts[tree.child_rows[c]];
+        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++) {
+            const uint64_t sum = static_cast<uint64_t>(counts[r]) + counts[tree.child_rows[c]];
+            counts[r] = static_cast<uint32_t>(std::min<uint64_t>(sum, UINT32_MAX));  // (repeated tip names)
+        }
 }
 
 // Embedded rows that are cheaper by sample lists than in the dense form.  The
@@ -1664,16 +1727,22 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
     const uint32_t E = tree.n_embedded;
     sp.id_of_row.assign(E, -1);
     if (!rule.on || !E) return sp;
-    std::vector<uint64_t> bound(tree.n_nodes, 0);
+    // (a table holds fewer than 2^32 entries, so its counts fit 32 bits)
+    const size_t n_tables = set.tables.size();
+    std::vector<std::vector<uint32_t>> counts(n_tables);
+    std::vector<uint64_t> bound(E, 0);
     std::vector<double> square(E, 0.0);  // sum over tables of the bound's square
     uint64_t samples = 0;
-    for (size_t t = 0; t < set.tables.size(); t++) {
+    for (size_t t = 0; t < n_tables; t++) {
         samples += set.tables[t]->n_samples;
-        std::vector<uint64_t> c(tree.n_nodes, 0);
+        std::vector<uint32_t> &c = counts[t];
+        c.assign(tree.n_nodes, 0);
         add_entry_counts(set, tree, t, c);
         sum_over_clades(tree, c);
-        for (uint32_t r = 0; r < tree.n_nodes; r++) bound[r] += c[r];
-        for (uint32_t e = 0; e < E; e++) square[e] += static_cast<double>(c[e]) * static_cast<double>(c[e]);
+        for (uint32_t e = 0; e < E; e++) {
+            bound[e] += c[e];
+            square[e] += static_cast<double>(c[e]) * static_cast<double>(c[e]);
+        }
     }
     std::vector<uint8_t> in(E, 0);
     double total = 0.0, gain = -rule.fixed_s;
@@ -1689,12 +1758,27 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
     if (s2 > 1000 || s2 < -1000) return sp;
     sp.scale = std::ldexp(1.0, s2);
     const double lmin = std::ldexp(1.0, rule.min_bits - 1 - s2);
+    // numbered by decreasing length of their lists (a counting sort): a
+    // sample's nodes then come in that order, and the lists that lanes read side
+    // by side end together
+    std::vector<uint32_t> at(samples + 2, 0);
+    for (uint32_t e = 0; e < E; e++) {
+        in[e] = in[e] && tree.length[e] >= lmin;
+        if (in[e]) at[samples - bound[e] + 1]++;
+    }
+    for (uint64_t i = 1; i < at.size(); i++) at[i] += at[i - 1];
+    sp.row.resize(at.back());
     for (uint32_t e = 0; e < E; e++)
-        if (in[e] && tree.length[e] >= lmin) sp.row.push_back(e);
-    // numbered by decreasing length of their lists: a sample's nodes then come
-    // in that order, and the lists that lanes read side by side end together
-    std::stable_sort(sp.row.begin(), sp.row.end(), [&](uint32_t x, uint32_t y) { return bound[x] > bound[y]; });
-    for (size_t i = 0; i < sp.row.size(); i++) sp.id_of_row[sp.row[i]] = static_cast<int32_t>(i);
+        if (in[e]) {
+            sp.id_of_row[e] = static_cast<int32_t>(at[samples - bound[e]]);
+            sp.row[at[samples - bound[e]]++] = e;
+        }
+    sp.entries.resize(n_tables);
+    for (size_t t = 0; t < n_tables; t++) {
+        sp.entries[t].resize(sp.row.size());
+        for (size_t i = 0; i < sp.row.size(); i++)
+            sp.entries[t][i] = std::min(counts[t][sp.row[i]], set.tables[t]->n_samples);
+    }
     return sp;
 }
 
@@ -1809,27 +1893,65 @@ GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const Li
         for (int i = 0; i < 4; i++) lay.digits[static_cast<size_t>(i) * k_pad + c] = d[i];
     }
     // parents among embedded nodes
-    std::vector<int32_t> parent_row(tree.n_nodes, -1);
-    for (uint32_t r = 0; r < tree.n_nodes; r++)
-        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++) parent_row[tree.child_rows[c]] = r;
+    const std::vector<int32_t> parent_row = parent_rows(tree);
     lay.parent_col.assign(lay.lsorted.size(), -1);
     for (uint32_t r = 0; r < E; r++) {
         const int32_t p = parent_row[r];
         lay.parent_col[col_of_row[r]] = (p >= 0 && static_cast<uint32_t>(p) < E) ? col_of_row[p] : -1;
     }
-    // starting column of each tree observation: its tip, or the tip's parent
-    // when tips are bypassed
-    uint32_t n_obs_tree = 0;
-    for (uint32_t r : tree.leaf_rows) n_obs_tree = std::max<uint32_t>(n_obs_tree, tree.leaf_obs[r] + 1);
-    lay.start_of_obs.assign(n_obs_tree, -1);
-    for (uint32_t r : tree.leaf_rows) {
-        const int32_t obs = tree.leaf_obs[r];
-        if (obs < 0) continue;
-        int32_t node = static_cast<int32_t>(r);
-        if (r >= E) node = parent_row[r];
-        lay.start_of_obs[obs] = (node >= 0 && static_cast<uint32_t>(node) < E) ? col_of_row[node] : -1;
-    }
+    lay.start_of_obs = path_starts(tree, parent_row, col_of_row);
     return lay;
+}
+
+// Starting columns of every operand row or sample (start_of_obs: per tree
+// observation, the column where its path upward starts, or -1).
+int PlanImpl::setup_sample_lists(const TableSet &set, const std::vector<int32_t> &start_of_obs) {
+    const uint32_t n_obs_tree = static_cast<uint32_t>(start_of_obs.size());
+    // per group: operand rows = the group's columns; each row's list of
+    // starting columns (one per table row of an observation with a positive
+    // count), built on the device from the uploaded CSR: count, scan, place
+    for (Group &g : groups) {
+        uint64_t nnz_g = 0;
+        for (uint32_t t = g.t0; t < g.t1; t++) nnz_g += set.tables[t]->nnz();
+        uint32_t *d_count = nullptr, *d_fill = nullptr;
+        SSU_CK(alloc(&d_count, sizeof(uint32_t) * g.ld));
+        SSU_CK(alloc(&d_fill, sizeof(uint32_t) * g.ld));
+        SSU_CK(alloc(&g.d_sample_ptr, sizeof(uint32_t) * (g.ld + 1)));
+        SSU_CK(alloc(&g.d_start_col, sizeof(int32_t) * std::max<uint64_t>(nnz_g, 1)));
+        SSU_CK(cudaMemsetAsync(d_count, 0, sizeof(uint32_t) * g.ld, stream));
+        std::vector<int32_t *> d_row_start(g.t1 - g.t0, nullptr);
+        for (uint32_t t = g.t0; t < g.t1; t++) {
+            const Table &tb = *set.tables[t];
+            std::vector<int32_t> row_start(std::max<uint32_t>(tb.n_obs, 1), -1);
+            if (set.obs_row.empty()) {
+                for (uint32_t o = 0; o < n_obs_tree && o < tb.n_obs; o++) row_start[o] = start_of_obs[o];
+            } else {
+                const std::vector<int32_t> &m = set.obs_row[t];
+                for (uint32_t o = 0; o < n_obs_tree && o < m.size(); o++)
+                    if (m[o] >= 0 && static_cast<uint32_t>(m[o]) < tb.n_obs) row_start[m[o]] = start_of_obs[o];
+            }
+            SSU_CK(upload(&d_row_start[t - g.t0], row_start.data(), sizeof(int32_t) * row_start.size()));
+        }
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass == 1) {
+                tc::exclusive_scan_kernel<<<1, 1024, 0, stream>>>(d_count, static_cast<uint32_t>(g.ld),
+                                                                  g.d_sample_ptr);
+                SSU_CK(cudaMemcpyAsync(d_fill, g.d_sample_ptr, sizeof(uint32_t) * g.ld, cudaMemcpyDeviceToDevice,
+                                       stream));
+            }
+            for (uint32_t t = g.t0; t < g.t1; t++) {
+                const Table &tb = *set.tables[t];
+                const dev::TableDesc &d = tdesc[t];
+                if (tb.n_obs == 0 || tb.nnz() == 0) continue;
+                const uint64_t threads = static_cast<uint64_t>(tb.n_obs) * 32;
+                tc::sample_lists_kernel<<<static_cast<uint32_t>((threads + 255) / 256), 256, 0, stream>>>(
+                    d_indptr + d.indptr_off, d_indices + d.nnz_off, d_data + d.nnz_off, d_row_start[t - g.t0],
+                    tb.n_obs, d.base, d_count, pass ? d_fill : nullptr, g.d_start_col);
+            }
+        }
+        SSU_CK(cudaGetLastError());
+    }
+    return 0;
 }
 
 // Nodes that the contraction leaves to the sample lists.  A 128-node block
@@ -1896,53 +2018,6 @@ int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     k_pad = lay.k_pad;
     const uint32_t n_cols = static_cast<uint32_t>(lay.lsorted.size());  // contracted and sparse
     n_chunks = static_cast<uint32_t>(lay.chunk_end.size());
-    const std::vector<int32_t> &start_of_obs = lay.start_of_obs;
-    const uint32_t n_obs_tree = static_cast<uint32_t>(start_of_obs.size());
-    // per group: operand rows = the group's columns; each row's list of
-    // starting columns (one per table row of an observation with a positive
-    // count), built on the device from the uploaded CSR: count, scan, place
-    for (Group &g : groups) {
-        uint64_t nnz_g = 0;
-        for (uint32_t t = g.t0; t < g.t1; t++) nnz_g += set.tables[t]->nnz();
-        uint32_t *d_count = nullptr, *d_fill = nullptr;
-        SSU_CK(alloc(&d_count, sizeof(uint32_t) * g.ld));
-        SSU_CK(alloc(&d_fill, sizeof(uint32_t) * g.ld));
-        SSU_CK(alloc(&g.d_sample_ptr, sizeof(uint32_t) * (g.ld + 1)));
-        SSU_CK(alloc(&g.d_start_col, sizeof(int32_t) * std::max<uint64_t>(nnz_g, 1)));
-        SSU_CK(cudaMemsetAsync(d_count, 0, sizeof(uint32_t) * g.ld, stream));
-        std::vector<int32_t *> d_row_start(g.t1 - g.t0, nullptr);
-        for (uint32_t t = g.t0; t < g.t1; t++) {
-            const Table &tb = *set.tables[t];
-            std::vector<int32_t> row_start(std::max<uint32_t>(tb.n_obs, 1), -1);
-            if (set.obs_row.empty()) {
-                for (uint32_t o = 0; o < n_obs_tree && o < tb.n_obs; o++) row_start[o] = start_of_obs[o];
-            } else {
-                const std::vector<int32_t> &m = set.obs_row[t];
-                for (uint32_t o = 0; o < n_obs_tree && o < m.size(); o++)
-                    if (m[o] >= 0 && static_cast<uint32_t>(m[o]) < tb.n_obs) row_start[m[o]] = start_of_obs[o];
-            }
-            SSU_CK(upload(&d_row_start[t - g.t0], row_start.data(), sizeof(int32_t) * row_start.size()));
-        }
-        for (int pass = 0; pass < 2; pass++) {
-            if (pass == 1) {
-                tc::exclusive_scan_kernel<<<1, 1024, 0, stream>>>(d_count, static_cast<uint32_t>(g.ld),
-                                                                  g.d_sample_ptr);
-                SSU_CK(cudaMemcpyAsync(d_fill, g.d_sample_ptr, sizeof(uint32_t) * g.ld, cudaMemcpyDeviceToDevice,
-                                       stream));
-            }
-            for (uint32_t t = g.t0; t < g.t1; t++) {
-                const Table &tb = *set.tables[t];
-                const dev::TableDesc &d = tdesc[t];
-                if (tb.n_obs == 0 || tb.nnz() == 0) continue;
-                const uint64_t threads = static_cast<uint64_t>(tb.n_obs) * 32;
-                tc::sample_lists_kernel<<<static_cast<uint32_t>((threads + 255) / 256), 256, 0, stream>>>(
-                    d_indptr + d.indptr_off, d_indices + d.nnz_off, d_data + d.nnz_off, d_row_start[t - g.t0],
-                    tb.n_obs, d.base, d_count, pass ? d_fill : nullptr, g.d_start_col);
-            }
-        }
-        SSU_CK(cudaGetLastError());
-    }
-    timer.step("gemm_sample_lists");
     const uint32_t band = static_cast<uint32_t>(std::max(1, env_int("UNIFRAC_B200_TC_BAND", 4)));
     if (const int rc = build_units(band)) return rc;
     timer.step("gemm_tiles");
@@ -1956,7 +2031,7 @@ int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     SSU_CK(upload(&d_chunk_scale, lay.scale.data(), sizeof(double) * n_chunks));
     SSU_CK(upload(&d_chunk_end, lay.chunk_end.data(), sizeof(uint32_t) * n_chunks));
     SSU_CK(upload(&d_parent_col, lay.parent_col.data(), sizeof(int32_t) * n_cols));
-    if (const int rc = setup_lists(set, tree, lay.sparse, d_lsorted + k_pad)) return rc;
+    if (const int rc = setup_lists(set, tree, lay.sparse, d_lsorted + k_pad, n_cols - k_pad, 0, nullptr, lay.start_of_obs)) return rc;
     if (n_sparse) {
         uint64_t most = 0;
         for (Group &g : groups) {
@@ -2010,9 +2085,9 @@ bool PlanImpl::device_error_pending() {
 
 // Counters of a group's lists, zeroed before its walk.
 int PlanImpl::reset_lists(cudaStream_t s, const Group &g) {
-    if (!n_sparse) return 0;
-    SSU_CK(cudaMemsetAsync(g.lists.count, 0, sizeof(uint32_t) * g.lists.slots, s));
-    SSU_CK(cudaMemsetAsync(g.lists.cursor, 0, sizeof(unsigned long long), s));
+    if (!g.lists.cursor) return 0;
+    // (the cursor lies just before the counts)
+    SSU_CK(cudaMemsetAsync(g.lists.cursor, 0, sizeof(unsigned long long) + sizeof(uint32_t) * g.lists.slots, s));
     return 0;
 }
 
@@ -2041,19 +2116,20 @@ int PlanImpl::shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &
 // Lists of the sparse nodes: offsets per (table, node) from the tables' entry
 // counts, buffers, fixed-point lengths.
 int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp,
-                          const double *d_len_of_node) {
+                          const double *d_len_of_col, uint32_t n, uint32_t first, const std::vector<double> *path,
+                          const std::vector<int32_t> &start_of_obs) {
     n_sparse = static_cast<uint32_t>(sp.row.size());
     sparse_unit = 1.0 / sp.scale;
-    if (!n_sparse) return 0;
-    SSU_CK(alloc(&d_sparse_q, sizeof(unsigned long long) * n_sparse));
-    dev::fixed_lengths_kernel<<<(n_sparse + 255) / 256, 256, 0, stream>>>(d_len_of_node, n_sparse, sp.scale,
-                                                                         d_sparse_q);
-    SSU_CK(cudaGetLastError());
+    if (!n_sparse && !path) return setup_sample_lists(set, start_of_obs);
+    SSU_CK(alloc(&d_sparse_q, sizeof(unsigned long long) * n));
+    SSU_CK(alloc(&d_list_unit, sizeof(double)));
+    double *d_path = nullptr;
+    if (path) SSU_CK(upload(&d_path, path->data(), sizeof(double) * path->size()));
     for (Group &g : groups) {
         const uint32_t tg = g.t1 - g.t0;
         dev::ListArgs &la = g.lists;
         la.n_nodes = n_sparse;
-        la.q = d_sparse_q;
+        la.q = d_sparse_q + first;
         la.block_table = g.d_block_table;
         la.tables = d_tdesc;
         la.t0 = g.t0;
@@ -2061,12 +2137,9 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
         uint64_t at = 0, ids = 0;  // at: in units of LIST_ALIGN entries
         for (uint32_t t = g.t0; t < g.t1; t++) {
             if (tdesc[t].n > 65536 || list_rule.wide) la.wide = 1;
-            std::vector<uint64_t> c(tree.n_nodes, 0);
-            add_entry_counts(set, tree, t, c);
-            sum_over_clades(tree, c);
             uint32_t *o = off.data() + static_cast<size_t>(t - g.t0) * n_sparse;
             for (uint32_t e = 0; e < n_sparse; e++) {
-                const uint64_t m = std::min<uint64_t>(c[sp.row[e]], tdesc[t].n);
+                const uint64_t m = sp.entries[t][e];
                 o[e] = static_cast<uint32_t>(at);
                 at += (m + dev::LIST_ALIGN - 1) / dev::LIST_ALIGN;
                 ids += m;
@@ -2101,17 +2174,30 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
         uint32_t *d_off = nullptr;
         SSU_CK(upload(&d_off, off.data(), sizeof(uint32_t) * off.size()));
         la.off = d_off;
-        SSU_CK(alloc(&la.count, sizeof(uint32_t) * off.size()));
+        SSU_CK(alloc(&la.cursor, sizeof(unsigned long long) + sizeof(uint32_t) * off.size()));
+        la.count = reinterpret_cast<uint32_t *>(la.cursor + 1);
         SSU_CK(alloc(&la.idx, bytes));
-        // the padding after each list reads as sample 0, which no row adds
-        SSU_CK(cudaMemsetAsync(la.idx, 0, std::max<size_t>(bytes, 1), stream));
+        g.list_bytes = bytes;
         SSU_CK(alloc(&la.node, sizeof(uint32_t) * std::max<uint64_t>(ids, 1)));
         SSU_CK(alloc(&la.node_ptr, sizeof(unsigned long long) * g.ld));
         SSU_CK(alloc(&la.node_cnt, sizeof(uint32_t) * g.ld));
-        SSU_CK(alloc(&la.cursor, sizeof(unsigned long long)));
         SSU_CK(alloc(&la.rs, sizeof(unsigned long long) * g.ld));
-        SSU_CK(cudaStreamSynchronize(stream));  // the host offsets are released on return
     }
+    // (kernels last: an upload from pageable memory waits for those before it)
+    if (const int rc = setup_sample_lists(set, start_of_obs)) return rc;
+    for (Group &g : groups)  // the padding after each list reads as sample 0, which no row adds
+        if (n_sparse) SSU_CK(cudaMemsetAsync(g.lists.idx, 0, std::max<size_t>(g.list_bytes, 1), stream));
+    unsigned long long *d_top = nullptr;
+    if (path) {
+        SSU_CK(alloc(&d_top, sizeof(unsigned long long)));
+        SSU_CK(cudaMemsetAsync(d_top, 0, sizeof(unsigned long long), stream));
+        for (const Group &g : groups)
+            dev::list_bound_kernel<<<static_cast<uint32_t>((g.ld + 7) / 8), 256, 0, stream>>>(
+                g.d_sample_ptr, g.d_start_col, static_cast<uint32_t>(g.ld), d_path, d_top);
+    }
+    dev::fixed_lengths_kernel<<<(n + 255) / 256, 256, 0, stream>>>(d_len_of_col, n, d_top, sp.scale, d_sparse_q,
+                                                                  d_list_unit);
+    SSU_CK(cudaGetLastError());
     constexpr int smem = static_cast<int>(2 * sizeof(uint32_t) * kSharedCols);
     SSU_CK(cudaFuncSetAttribute(dev::shared_sums_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     SSU_CK(cudaFuncSetAttribute(dev::shared_sums_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -2182,6 +2268,170 @@ int PlanImpl::execute_gemm(cudaStream_t s, const dev::OutSpec &out) {
     if (out.mode == 0) zero_diagonal(s, out.ptr);
     if (timed()) SSU_CK(cudaEventRecord(ev[3], s));
     SSU_CK(cudaGetLastError());
+    return 0;
+}
+
+// ------------------------------------------- fp64 unweighted by presence words
+
+// Nodes left to the sample lists in the whole-number form.  A dense node costs
+// 0.08 ps a pair of all samples (10.3 us a 64-node word at 2,048 samples), at
+// least 10 ns where the tables do not fill the SMs; by lists it costs 1 ps a
+// pair of its samples and 60 ps a sample.  The node is by lists up to about a quarter
+// of the samples.  Times with half and one and a half times that dense cost:
+// 2,048 samples x 20,000 tips 654, 655, 695 us; 4,096 x 50,000 2,672,
+// 2,577, 2,587 us; with least costs of 10, 20, 40, 80 ns: 500 x 50,000 213,
+// 236, 263, 299 us.  (The stripe form over every node: 7,910 us for the
+// first.)
+ListRule PlanImpl::bits_list_rule(const TableSet &set) const {
+    ListRule r;
+    r.on = true;
+    double pairs = 0.0;
+    for (const Table *t : set.tables) pairs += 0.5 * t->n_samples * static_cast<double>(t->n_samples);
+    r.dense_s = std::max(pairs * 8e-14, 1e-8);
+    r.pair_s = 1e-12;
+    r.entry_s = 6e-11;
+    r.min_div = 1;
+    return r;
+}
+
+int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
+    SetupTimer timer;
+    const ListRule rule = bits_list_rule(set);
+    const SparseNodes sp = find_sparse_nodes(set, tree, rule);
+    // columns: the dense rows in order, padded to whole words, then the sparse nodes
+    uint32_t n_dense = 0;
+    std::vector<int32_t> col(tree.n_nodes, -1);
+    for (uint32_t e = 0; e < E; e++)
+        if (sp.id_of_row[e] < 0) col[e] = static_cast<int32_t>(n_dense++);
+    n_words = (n_dense + 63) / 64;
+    const uint32_t first = n_words * 64;
+    for (size_t i = 0; i < sp.row.size(); i++) col[sp.row[i]] = static_cast<int32_t>(first + i);
+    n_words_all = n_words + (static_cast<uint32_t>(sp.row.size()) + 63) / 64;
+    const uint32_t n_cols = std::max(1u, n_words_all * 64);
+    std::vector<double> len(n_cols, 0.0), path(n_cols, 0.0);
+    std::vector<int32_t> parent(n_cols, -1), parent_row = parent_rows(tree);
+    for (uint32_t r = E; r-- > 0;) {  // parents follow their children
+        const int32_t p = parent_row[r];
+        len[col[r]] = tree.length[r];
+        if (p >= 0 && static_cast<uint32_t>(p) < E) parent[col[r]] = col[p];
+        path[col[r]] = (parent[col[r]] >= 0 ? path[parent[col[r]]] : 0.0) + tree.length[r];
+    }
+    timer.step("bits_layout");
+    uint64_t big_tiles = 0;  // 128 x 64 tiles of the upper triangles
+    for (const dev::TableDesc &d : tdesc) big_tiles += static_cast<uint64_t>((d.n + 127) / 128) * ((d.n + 127) / 128 + 1);
+    const SharedBitsPair pair =
+        shared_bits_pair(spec.method == Method::unweighted, big_tiles < static_cast<uint64_t>(n_sms));
+    kd = pair.shared;
+    k_stripe = pair.stripe;
+    for (PairKernel<double> *k : {&kd, &k_stripe}) {
+        int bps = 0;
+        if (k->configure(k->smem) != cudaSuccess || k->occupancy(&bps, k->threads, k->smem) != cudaSuccess || bps < 1) {
+            last_error = "pair kernel does not fit on the device";
+            return kOutputError;
+        }
+        k->blocks_per_sm = bps;
+    }
+    const PairKernel<double> &k = kd;
+    uint32_t max_tiles = 1;
+    for (Group &g : groups) {
+        std::vector<uint4> tiles;
+        for (uint32_t t = g.t0; t < g.t1; t++) append_tiles(tiles, t, tdesc[t].base, tdesc[t].n, k.BM, k.BN, false, 0, 0);
+        g.n_tiles = static_cast<uint32_t>(tiles.size());
+        max_tiles = std::max(max_tiles, g.n_tiles);
+        SSU_CK(upload(&g.d_tiles, tiles.data(), sizeof(uint4) * tiles.size()));
+        choose_splits<double>(k, g.n_tiles, g.splits, g.rows_per_split);
+        if (g.splits > 1)
+            partial_bytes = std::max(partial_bytes, sizeof(double) * k.partial_per_tile * g.n_tiles * g.splits);
+    }
+    if (partial_bytes) SSU_CK(alloc(&d_partial, partial_bytes));
+    SSU_CK(alloc(&d_flags, sizeof(int) * max_tiles));
+    SSU_CK(upload(&d_parent_col, parent.data(), sizeof(int32_t) * n_cols));
+    SSU_CK(upload(&d_len_cols, len.data(), sizeof(double) * n_cols));
+    if (const int rc = setup_lists(set, tree, sp, d_len_cols, n_cols, first, &path, path_starts(tree, parent_row, col)))
+        return rc;
+    timer.step("bits_lists");
+    lut_stride = 0;
+    SSU_CK(alloc(&d_nib, sizeof(unsigned long long) * dev::NIB_TABLE * std::max(n_words, 1u)));
+    if (n_words) dev::build_nibbles_kernel<<<n_words, dev::NIB_TABLE, 0, stream>>>(d_sparse_q, n_words, d_nib);
+    SSU_CK(alloc(&d_P, sizeof(unsigned long long) * ld * std::max(n_words_all, 1u)));
+    SSU_CK(alloc(&d_lut, sizeof(double) * 2048 * std::max(n_words_all, 1u)));
+    if (n_words_all) {
+        dev::build_lut_kernel<double><<<dim3(n_words_all * 8, 1), 256, 0, stream>>>(d_len_cols, n_cols,
+                                                                                   static_cast<double *>(d_lut), 0, 0);
+        SSU_CK(cudaGetLastError());
+    }
+    SSU_CK(alloc(&d_full, sizeof(double) * std::max<uint64_t>(full_elems, 1)));
+    d_shared = static_cast<unsigned long long *>(d_full);  // a pair's sum is read before its distance is written
+    SSU_CK(cudaFuncSetAttribute(dev::presence_words_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(tc::MAX_BITMAP_BYTES)));
+    tuning = "sample lists";
+    timer.step("bits_buffers");
+    return 0;
+}
+
+// One group: the walk (presence words, lists), the sparse nodes' shared sums,
+// the presence-word kernel over the dense words, then over every word on the
+// tiles it flagged.
+int PlanImpl::walk_bits_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
+                              uint32_t ntiles, uint32_t splits, uint32_t rows, bool first, bool last) {
+    if (const int rc = reset_lists(s, g)) return rc;
+    const dev::ListArgs &la = g.lists;
+    const size_t smem = sizeof(unsigned long long) * n_words_all;
+    for (uint32_t p = 0; p < la.parts; p++) {
+        const uint32_t c0 = n_sparse ? g.part_col[p] : 0;
+        const uint32_t c1 = n_sparse ? g.part_col[p + 1] : static_cast<uint32_t>(g.ld);
+        if (p)
+            SSU_CK(cudaMemcpyAsync(la.part_count + (p - 1) * la.slots, la.count, sizeof(uint32_t) * la.slots,
+                                   cudaMemcpyDeviceToDevice, s));
+        if (c1 <= c0) continue;
+        dev::presence_words_kernel<<<c1 - c0, 256, smem, s>>>(g.d_sample_ptr, g.d_start_col, d_parent_col, d_len_cols,
+                                                             d_sparse_q, n_words, n_words_all, g.ld, d_P,
+                                                             n_sparse ? g.d_columns + c0 : nullptr, la);
+        launches++;
+    }
+    SSU_CK(cudaGetLastError());
+    if (first && timed()) SSU_CK(cudaEventRecord(ev[1], s));
+    if (ntiles) {
+        const PairKernel<double> &k = kd;
+        dev::PairArgs<double> a{};
+        a.tiles = tiles;
+        a.n_tiles = ntiles;
+        a.tables = d_tdesc;
+        a.P = d_P;
+        a.nib = d_nib;
+        a.E = n_words;
+        a.ld = g.ld;
+        a.out = out;
+        a.n_splits = std::max(1u, splits);
+        a.rows_per_split = splits > 1 ? rows : n_words;
+        a.partial = splits > 1 ? static_cast<double *>(d_partial) : nullptr;
+        a.rs = la.rs;
+        a.unit = d_list_unit;
+        a.flags_out = d_flags;
+        if (n_sparse) {
+            a.shared.S = d_shared;
+            if (const int rc = shared_sums(s, g, a.shared, 0, static_cast<uint32_t>(g.ld))) return rc;
+        }
+        SSU_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * ntiles, s));
+        const uint64_t slots = static_cast<uint64_t>(std::max(1, n_sms * k.blocks_per_sm));
+        k.launch(a, static_cast<uint32_t>(std::min<uint64_t>(static_cast<uint64_t>(ntiles) * a.n_splits, slots)), k.smem,
+                 s);
+        launches++;
+        if (a.partial) {
+            k.finalize(a, s);
+            launches++;
+        }
+        a.tile_flags = d_flags;
+        a.lut = static_cast<const double *>(d_lut);
+        a.E = n_words_all;
+        a.n_splits = 1;
+        a.rows_per_split = n_words_all;
+        a.partial = nullptr;
+        k_stripe.launch(a, static_cast<uint32_t>(std::min<uint64_t>(ntiles, slots)), k_stripe.smem, s);
+        launches++;
+        SSU_CK(cudaGetLastError());
+    }
+    if (last && timed()) SSU_CK(cudaEventRecord(ev[2], s));
     return 0;
 }
 
@@ -2279,6 +2529,26 @@ bool use_tensor_cores(const MethodSpec &spec, const TableSet &set, const FlatTre
     return want;
 }
 
+// fp64 unweighted results from presence words and sample lists: counts and
+// lengths that are not negative and finite (presence is then "some tip below
+// has a count", and lists hold whole-number lengths), one length per node for
+// all tables, a bitmap of the nodes in shared memory, and no request for the
+// plain stripe form.
+bool use_walk_bits(const MethodSpec &spec, const TableSet &set, const FlatTree &tree) {
+    if (!spec.fp64 || spec.vaw || spec.unweighted_stripe || !set.row_active.empty() ||
+        !(spec.method == Method::unweighted || spec.method == Method::unweighted_unnormalized))
+        return false;
+    if (tree.n_embedded / 8 + 64 > tc::MAX_BITMAP_BYTES) return false;
+    for (uint32_t e = 0; e < tree.n_embedded; e++)
+        if (!(tree.length[e] >= 0.0 && std::isfinite(tree.length[e]))) return false;
+    for (const Table *t : set.tables) {
+        if (!t->nonneg) return false;
+        for (double x : t->totals)
+            if (!std::isfinite(x)) return false;
+    }
+    return true;
+}
+
 }  // namespace
 
 int Plan::create(const Table &table, const FlatTree &tree, const MethodSpec &spec, void *stream, Plan **out,
@@ -2293,9 +2563,14 @@ int Plan::create(const Table &table, const FlatTree &tree, const MethodSpec &spe
     set.tables.push_back(&table);
     set.embedded.push_back(tree.n_embedded);
     m.gemm = use_tensor_cores(spec, set, tree, false);
+    m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
     if (m.gemm) m.start_gemm_layout(set, tree);
     int rc = m.setup(set, tree, BatchOptions{});
-    if (!rc) rc = m.gemm ? m.setup_gemm(set, tree) : spec.fp64 ? m.setup_method<double>() : m.setup_method<float>();
+    if (!rc)
+        rc = m.gemm        ? m.setup_gemm(set, tree)
+             : m.walk_bits ? m.setup_walk_bits(set, tree)
+             : spec.fp64   ? m.setup_method<double>()
+                           : m.setup_method<float>();
     if (rc) {
         err = m.last_error;
         delete p;
@@ -2321,9 +2596,14 @@ int Plan::create_batch(const TableSet &set, const FlatTree &tree, const MethodSp
     m.stream = static_cast<cudaStream_t>(stream);
     m.autotune = resolve_autotune(opts.autotune, true);
     m.gemm = use_tensor_cores(spec, set, tree, true);
+    m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
     if (m.gemm) m.start_gemm_layout(set, tree);
     int rc = m.setup(set, tree, opts);
-    if (!rc) rc = m.gemm ? m.setup_gemm(set, tree) : spec.fp64 ? m.setup_method<double>() : m.setup_method<float>();
+    if (!rc)
+        rc = m.gemm        ? m.setup_gemm(set, tree)
+             : m.walk_bits ? m.setup_walk_bits(set, tree)
+             : spec.fp64   ? m.setup_method<double>()
+                           : m.setup_method<float>();
     if (rc) {
         err = m.last_error;
         delete p;

@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(256)
         for (int t = 0; t < 16; t++)
             if ((b >> t) & 1u) part += l_sorted[c16 + t];
     }
-    if (la.n_nodes) dev::write_lists(la, j, bits + k_pad / 32, sp_words, l_sorted + k_pad, part);
+    if (la.n_nodes) dev::write_lists(la, j, bits + k_pad / 32, sp_words, l_sorted + k_pad, 0ull, part);
     red[threadIdx.x] = part;
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -365,6 +365,19 @@ __device__ __forceinline__ void emit_pair(const OutSpec &o, uint32_t n, uint32_t
     }
 }
 
+// Where row k of a table's shared sums (ssu_lists.cuh) is stored: S[k][l] at
+// row(k) + l for l > k, either n apart (full) or packed (condensed).
+struct SharedOut {
+    unsigned long long *S = nullptr;
+    const uint64_t *off = nullptr;  // condensed: first element of each table of the group; nullptr: full, at out_off
+};
+__device__ __forceinline__ unsigned long long *shared_row(const SharedOut &o, const TableDesc &td, uint32_t t_local,
+                                                          uint32_t k) {
+    const uint64_t kk = k, n = td.n;
+    // (one element before the row's first: indexed by l > k)
+    return o.off ? o.S + o.off[t_local] + kk * (2 * n - kk - 1) / 2 - (kk + 1) : o.S + td.out_off + kk * n;
+}
+
 // Work of one pair launch: tiles (x = k block, y = l block in the group's
 // columns, z = table) times node splits, walked by a persistent grid.
 template <typename T>
@@ -389,6 +402,12 @@ struct PairArgs {
     OutSpec out;
     T *partial;       // per-split raw accumulators; nullptr when not split
     const int *tile_flags;  // when set, only tiles with a non-zero flag are computed
+    // pair_shared_bits_kernel: nodes summed through sample lists, not in P
+    SharedOut shared;              // S == nullptr: none
+    const unsigned long long *rs;  // per column: fixed-point length of its nodes
+    const unsigned long long *nib; // [words][16][16] sums of fixed-point lengths by nibble
+    const double *unit;            // value of one fixed-point unit
+    int *flags_out;                // tiles to recompute in the stripe form
 };
 
 // ---- per-term operators (one (k, l) pair, one embedded node) -------------
@@ -793,6 +812,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 1) pair_bits_kernel(con
     const uint32_t n_work = a.n_tiles * a.n_splits;
     for (uint32_t wi = blockIdx.x; wi < n_work; wi += gridDim.x) {
         const uint32_t split = wi / a.n_tiles, ti = wi - split * a.n_tiles;
+        if (a.tile_flags && !a.tile_flags[ti]) continue;  // uniform over the CTA
         const uint4 tile = a.tiles[ti];
         const uint32_t k0 = tile.x * BM, l0 = tile.y * BN;
         const uint32_t w_begin = split * a.rows_per_split;
@@ -904,6 +924,174 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 1) pair_bits_kernel(con
 template <typename T, int BM, int BN, int KW>
 constexpr size_t pair_bits_smem() {
     return 2 * KW * (8 * 256 * sizeof(T) + (BM + BN) * sizeof(unsigned long long));
+}
+
+// ---- unweighted in whole numbers ------------------------------------------
+//
+// With the lengths as whole numbers q of a fixed-point unit, a pair only needs
+// its shared sum S = sum of q over the nodes both samples have:
+//   xor = (rs_k + rs_l - 2 S) unit,   or = (rs_k + rs_l - S) unit,
+// exact differences, whatever the order.  Per 64-node word: the AND of the two
+// samples' presence bits, and 16 sums by nibble.  A nibble's table is 128
+// bytes, one row of the shared memory's banks, so 32 lanes read 32 nibbles of
+// any values at once, where the stripe form's byte tables (2 KB) serve them in
+// several turns, twice (xor and or): at 2,048 samples 26 us a word of nodes
+// that many samples have, 10.3 us in this form.  Nodes that few
+// samples have come from the sample lists (a.shared).
+constexpr int NIB_TABLE = 16 * 16;  // sums per word
+
+static __global__ void build_nibbles_kernel(const unsigned long long *__restrict__ q, uint32_t n_words,
+                                            unsigned long long *__restrict__ nib) {
+    const uint32_t w = blockIdx.x, i = threadIdx.x / 16, v = threadIdx.x % 16;
+    unsigned long long s = 0;
+    for (uint32_t b = 0; b < 4; b++)
+        if ((v >> b) & 1u) s += q[w * 64 + i * 4 + b];
+    nib[static_cast<uint64_t>(w) * NIB_TABLE + threadIdx.x] = s;
+}
+
+// Where a pair's distance is below this share of its samples' own lengths,
+// the half unit that each length was rounded by could show: its tile is
+// flagged and recomputed in the stripe form over every node.
+constexpr double kSharedTau = 0.02;
+
+template <bool NORMALIZED, int BM, int BN, int TM, int TN>
+__device__ __forceinline__ void shared_bits_epilogue(const PairArgs<double> &a, uint32_t ti, int tx, int ty,
+                                                     const unsigned long long (&acc)[TM][TN]) {
+    const uint4 tile = a.tiles[ti];
+    const TableDesc td = a.tables[tile.z];
+    const uint32_t k0 = tile.x * BM - td.base, l0 = tile.y * BN - td.base;
+    OutSpec o = a.out;
+    if (o.mode == 0) o.ptr = static_cast<double *>(o.ptr) + td.out_off;
+    const double unit = *a.unit;
+    unsigned long long rl[TN];
+#pragma unroll
+    for (int j = 0; j < TN; j++) {
+        const uint32_t l = l0 + tile_row<BN, TN>(tx, j);
+        rl[j] = l < td.n ? a.rs[td.base + l] : 0ull;
+    }
+    bool close = false;
+#pragma unroll
+    for (int i = 0; i < TM; i++) {
+        const uint32_t k = k0 + tile_row<BM, TM>(ty, i);
+        if (k >= td.n) continue;
+        const unsigned long long *row = a.shared.S ? shared_row(a.shared, td, 0, k) : nullptr;
+        const unsigned long long rk = a.rs[td.base + k];
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+            const uint32_t l = l0 + tile_row<BN, TN>(tx, j);
+            if (!(k < l && l < td.n)) continue;
+            const unsigned long long own = rk + rl[j], sh = acc[i][j] + (row ? row[l] : 0ull);
+            const double x = static_cast<double>(own - 2 * sh);
+            close = close || x < kSharedTau * static_cast<double>(own);
+            emit_pair<double>(o, td.n, k, l, NORMALIZED ? x / static_cast<double>(own - sh) : x * unit);
+        }
+    }
+    if (close) atomicOr(a.flags_out + ti, 1);
+}
+
+template <bool NORMALIZED, int BM, int BN, int TM, int TN, int KW>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), 2) pair_shared_bits_kernel(const PairArgs<double> a) {
+    using u64 = unsigned long long;
+    constexpr int NT = (BM / TM) * (BN / TN);
+    constexpr int TX = BN / TN;
+    __shared__ __align__(128) u64 Ns[2][KW][NIB_TABLE];
+    __shared__ __align__(16) u64 As[2][KW][BM];
+    __shared__ __align__(16) u64 Bs[2][KW][BN];
+    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const uint32_t n_work = a.n_tiles * a.n_splits;
+    for (uint32_t wi = blockIdx.x; wi < n_work; wi += gridDim.x) {
+        const uint32_t split = wi / a.n_tiles, ti = wi - split * a.n_tiles;
+        const uint4 tile = a.tiles[ti];
+        const uint32_t k0 = tile.x * BM, l0 = tile.y * BN;
+        const uint32_t w_begin = split * a.rows_per_split;
+        const uint32_t w_end = min(a.E, w_begin + a.rows_per_split);
+        u64 acc[TM][TN];
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+            for (int j = 0; j < TN; j++) acc[i][j] = 0ull;
+        auto load_stage = [&](int st, uint32_t w0) {
+            auto rows = [&](u64 *dst, const u64 *src, uint64_t stride, int row_chunks) {
+                for (int c = tid; c < KW * row_chunks; c += NT) {
+                    const int r = c / row_chunks, q = c % row_chunks;
+                    const bool ok = w0 + r < w_end;
+                    cp_async16(dst + (r * row_chunks + q) * 2,
+                               src + static_cast<uint64_t>(ok ? w0 + r : 0) * stride + q * 2, ok ? 16 : 0);
+                }
+            };
+            rows(Ns[st][0], a.nib, NIB_TABLE, NIB_TABLE / 2);
+            rows(As[st][0], a.P + k0, a.ld, BM / 2);
+            rows(Bs[st][0], a.P + l0, a.ld, BN / 2);
+        };
+        const uint32_t n_chunks = w_end > w_begin ? (w_end - w_begin + KW - 1) / KW : 0;
+        if (n_chunks > 0) load_stage(0, w_begin);
+        cp_async_commit();
+        for (uint32_t ch = 0; ch < n_chunks; ch++) {
+            const int st = ch & 1;
+            if (ch + 1 < n_chunks) load_stage(st ^ 1, w_begin + (ch + 1) * KW);
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+#pragma unroll 1
+            for (int r = 0; r < KW; r++) {
+                const unsigned char *nib = reinterpret_cast<const unsigned char *>(Ns[st][r]);
+                u64 av[TM], bv[TN];
+#pragma unroll
+                for (int i = 0; i < TM; i++) av[i] = As[st][r][tile_row<BM, TM>(ty, i)];
+#pragma unroll
+                for (int j = 0; j < TN; j++) bv[j] = Bs[st][r][tile_row<BN, TN>(tx, j)];
+#pragma unroll
+                for (int i = 0; i < TM; i++) {
+#pragma unroll
+                    for (int j = 0; j < TN; j++) {
+                        const u64 both = av[i] & bv[j];
+                        const uint32_t half[2] = {static_cast<uint32_t>(both), static_cast<uint32_t>(both >> 32)};
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            if (half[h] == 0) continue;
+                            // 8 nibbles; 8 v is a nibble's byte offset in its 128-byte table
+                            u64 s = *reinterpret_cast<const u64 *>(nib + h * 1024 + ((half[h] << 3) & 0x78u));
+#pragma unroll
+                            for (int q = 1; q < 8; q++)
+                                s += *reinterpret_cast<const u64 *>(nib + h * 1024 + q * 128 +
+                                                                    ((half[h] >> (4 * q - 3)) & 0x78u));
+                            acc[i][j] += s;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        cp_async_wait<0>();
+        if (a.partial) {
+            u64 *dst = reinterpret_cast<u64 *>(a.partial) + (static_cast<uint64_t>(split) * a.n_tiles + ti) * BM * BN;
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) dst[(i * TN + j) * NT + tid] = acc[i][j];
+        } else {
+            shared_bits_epilogue<NORMALIZED, BM, BN, TM, TN>(a, ti, tx, ty, acc);
+        }
+        __syncthreads();  // shared memory is reused by the next work item
+    }
+}
+
+// The splits' sums of each tile (exact, so in any order), then the epilogue.
+template <bool NORMALIZED, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) shared_bits_finalize_kernel(const PairArgs<double> a) {
+    constexpr int NT = (BM / TM) * (BN / TN);
+    const int tid = threadIdx.x;
+    unsigned long long acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+            acc[i][j] = 0ull;
+            for (uint32_t s = 0; s < a.n_splits; s++)
+                acc[i][j] += reinterpret_cast<const unsigned long long *>(
+                    a.partial)[(static_cast<uint64_t>(s) * a.n_tiles + blockIdx.x) * BM * BN + (i * TN + j) * NT + tid];
+        }
+    shared_bits_epilogue<NORMALIZED, BM, BN, TM, TN>(a, blockIdx.x, tid % (BN / TN), tid / (BN / TN), acc);
 }
 
 }  // namespace dev

@@ -60,10 +60,38 @@ __host__ __device__ __forceinline__ uint32_t list_part_rows(uint32_t n, uint32_t
     return (n + parts - 1) / parts;
 }
 
-// q = round(L 2^s)
-static __global__ void fixed_lengths_kernel(const double *__restrict__ len, uint32_t n, double scale,
-                                            unsigned long long *__restrict__ q) {
+// top = the largest sum, over a sample's tips, of the sparse length above the
+// tip (path); it bounds every sample's sum over its sparse nodes (shared ones
+// count more than once here).  A warp per sample; positive doubles order as
+// whole numbers.
+static __global__ void __launch_bounds__(256)
+    list_bound_kernel(const uint32_t *__restrict__ sample_ptr, const int32_t *__restrict__ start, uint32_t n,
+                      const double *__restrict__ path, unsigned long long *__restrict__ top) {
+    const uint32_t j = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (j >= n) return;
+    double s = 0.0;
+    for (uint32_t e = sample_ptr[j] + lane; e < sample_ptr[j + 1]; e += 32)
+        if (start[e] >= 0) s += path[start[e]];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) atomicMax(top, static_cast<unsigned long long>(__double_as_longlong(s)));
+}
+
+// q = round(L 2^s), unit = 2^-s.  The scale is `least`, at which the sum of
+// every sparse length stays below 2^62 units, or (top != nullptr) the finest
+// at which the largest sample's does.
+static __global__ void fixed_lengths_kernel(const double *__restrict__ len, uint32_t n,
+                                            const unsigned long long *__restrict__ top, double least,
+                                            unsigned long long *__restrict__ q, double *__restrict__ unit) {
+    double scale = least;
+    if (top) {
+        const double m = __longlong_as_double(static_cast<long long>(*top));
+        int x = 0;
+        frexp(m * (1.0 + 1e-9), &x);  // m < 2^x
+        if (m > 0.0) scale = fmax(ldexp(1.0, min(62 - x, 1000)), least);
+    }
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *unit = 1.0 / scale;
     if (i < n) q[i] = static_cast<unsigned long long>(__double2ll_rn(len[i] * scale));
 }
 
@@ -97,12 +125,13 @@ static __device__ __forceinline__ void mark_paths(const int32_t *__restrict__ st
 
 // Both sides of the lists for column j, from its presence bitmap over the
 // sparse nodes (words 32-bit words in shared memory), by the whole block of
-// 256 threads; writes rs[j] and adds the threads' shares of the nodes' fp64
-// lengths to `part`.  Thread t takes consecutive words, so the sample side
+// 256 threads; writes rs[j], the threads' `sum` included, and adds their
+// shares of the nodes' fp64 lengths to `part`.  Thread t takes consecutive words, so the sample side
 // comes out in node order; the positions on the node side come from one
 // atomic per entry.
 static __device__ __forceinline__ void write_lists(const ListArgs &la, uint32_t j, const uint32_t *bits, uint32_t words,
-                                                   const double *__restrict__ len, double &part) {
+                                                   const double *__restrict__ len, unsigned long long sum,
+                                                   double &part) {
     __shared__ uint32_t warp_tot[8];
     __shared__ unsigned long long warp_q[8];
     __shared__ unsigned long long first;
@@ -144,7 +173,6 @@ static __device__ __forceinline__ void write_lists(const ListArgs &la, uint32_t 
     const uint32_t t = la.block_table[j >> 7];
     const uint32_t pos = j - la.tables[t].base;
     const uint64_t slot0 = static_cast<uint64_t>(t - la.t0) * la.n_nodes;
-    unsigned long long sum = 0;
     constexpr int U = 4;  // entries of a thread in flight
     for (uint32_t i0 = threadIdx.x; i0 < total; i0 += U * 256) {
         uint32_t e[U], rank[U], off[U];
@@ -181,19 +209,6 @@ static __device__ __forceinline__ void write_lists(const ListArgs &la, uint32_t 
         for (int w = 0; w < 8; w++) s += warp_q[w];
         la.rs[j] = s;
     }
-}
-
-// Where row k of a table's shared sums is stored: S[k][l] at row(k) + l for
-// l > k, either n apart (full) or packed (condensed).
-struct SharedOut {
-    unsigned long long *S = nullptr;
-    const uint64_t *off = nullptr;  // condensed: first element of each table of the group; nullptr: full, at out_off
-};
-__device__ __forceinline__ unsigned long long *shared_row(const SharedOut &o, const TableDesc &td, uint32_t t_local,
-                                                          uint32_t k) {
-    const uint64_t kk = k, n = td.n;
-    // (one element before the row's first: indexed by l > k)
-    return o.off ? o.S + o.off[t_local] + kk * (2 * n - kk - 1) / 2 - (kk + 1) : o.S + td.out_off + kk * n;
 }
 
 // 32-bit shared-memory additions where c < n, without a branch: the first
@@ -322,6 +337,37 @@ __global__ void __launch_bounds__(768, 2)
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x)
         row[c0 + i] = (static_cast<unsigned long long>(hi[i]) << 32) | lo[i];
+}
+
+// Presence words of the unweighted forms, one block of 256 threads per
+// sample: bit b of P[w][j] is node column 64 w + b of sample j, for the dense
+// nodes' words and then the sparse nodes'; and the sample's entries of the
+// sparse nodes' lists.  Walking up from the sample's own tips replaces the
+// embedding (proportions of every node for every sample, 95% of them zero).
+static __global__ void __launch_bounds__(256)
+    presence_words_kernel(const uint32_t *__restrict__ sample_ptr, const int32_t *__restrict__ start,
+                          const int32_t *__restrict__ parent, const double *__restrict__ len,
+                          const unsigned long long *__restrict__ q, uint32_t dense_words, uint32_t n_words, uint64_t ld,
+                          unsigned long long *__restrict__ P, const uint32_t *__restrict__ column, const ListArgs la) {
+    extern __shared__ uint32_t bits[];  // 2 n_words
+    const uint32_t j = column ? column[blockIdx.x] : blockIdx.x;
+    for (uint32_t w = threadIdx.x; w < 2 * n_words; w += 256) bits[w] = 0u;
+    __syncthreads();
+    mark_paths(start + sample_ptr[j], sample_ptr[j + 1] - sample_ptr[j], parent, bits);
+    __syncthreads();
+    for (uint32_t w = threadIdx.x; w < n_words; w += 256)
+        P[static_cast<uint64_t>(w) * ld + j] =
+            (static_cast<unsigned long long>(bits[2 * w + 1]) << 32) | bits[2 * w];
+    unsigned long long sum = 0;
+    for (uint32_t w = threadIdx.x; w < 2 * dense_words; w += 256) {
+        uint32_t m = bits[w];
+        while (m) {
+            sum += q[w * 32 + __ffs(m) - 1];
+            m &= m - 1;
+        }
+    }
+    double unused = 0.0;
+    write_lists(la, j, bits + 2 * dense_words, 2 * (n_words - dense_words), len + 64ull * dense_words, sum, unused);
 }
 
 }  // namespace dev

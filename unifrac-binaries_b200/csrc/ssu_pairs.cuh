@@ -83,6 +83,38 @@ PairKernel<T> bits_kernel(const char *name, const char *shape) {
     return k;
 }
 
+// The whole-number unweighted form (fp64 results).
+template <bool NORM, int BM, int BN, int TM, int TN, int KW>
+PairKernel<double> shared_bits_kernel(const char *name, const char *shape) {
+    PairKernel<double> k;
+    k.BM = BM;
+    k.BN = BN;
+    k.threads = (BM / TM) * (BN / TN);
+    k.row_quantum = KW;
+    k.partial_per_tile = static_cast<size_t>(BM) * BN;
+    k.name = name;
+    k.shape = shape;
+    k.launch = [](const dev::PairArgs<double> &a, uint32_t ctas, size_t, cudaStream_t s) {
+        dev::pair_shared_bits_kernel<NORM, BM, BN, TM, TN, KW><<<ctas, (BM / TM) * (BN / TN), 0, s>>>(a);
+    };
+    k.finalize = [](const dev::PairArgs<double> &a, cudaStream_t s) {
+        dev::shared_bits_finalize_kernel<NORM, BM, BN, TM, TN><<<a.n_tiles, (BM / TM) * (BN / TN), 0, s>>>(a);
+    };
+    k.configure = [](size_t) { return cudaSuccess; };
+    k.occupancy = [](int *blocks, int threads, size_t) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            blocks, dev::pair_shared_bits_kernel<NORM, BM, BN, TM, TN, KW>, threads, 0);
+    };
+    return k;
+}
+// The whole-number form and the stripe form in the same tile shape (the tiles
+// that the first flags are recomputed by the second): 128 x 64, or 32 x 32 where
+// those would not fill the SMs.
+struct SharedBitsPair {
+    PairKernel<double> shared, stripe;
+};
+SharedBitsPair shared_bits_pair(bool normalized, bool small);
+
 // alpha kind: 1 -> sqrt, 2 -> identity, 3 -> constant 1, 0 -> pow
 inline int alpha_kind(double alpha) {
     if (alpha == 0.5) return 1;

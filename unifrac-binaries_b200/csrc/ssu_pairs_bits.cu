@@ -14,6 +14,21 @@ std::vector<PairKernel<T>> bits_candidates(bool normalized) {
             bits_kernel<T, false, 64, 64, 4, 4, KW>("pair_bits<unweighted_unnormalized>", "64x64/4x4")};
 }
 
+template <bool NORM>
+static SharedBitsPair shared_bits_of(const char *name, const char *stripe, bool small) {
+    if (small)
+        return {shared_bits_kernel<NORM, 32, 32, 2, 2, 4>(name, "32x32/2x2"),
+                bits_kernel<double, NORM, 32, 32, 2, 2, 2>(stripe, "32x32/2x2")};
+    return {shared_bits_kernel<NORM, 128, 64, 8, 4, 4>(name, "128x64/8x4"),
+            bits_kernel<double, NORM, 128, 64, 8, 4, 2>(stripe, "128x64/8x4")};
+}
+
+SharedBitsPair shared_bits_pair(bool normalized, bool small) {
+    return normalized ? shared_bits_of<true>("pair_shared_bits<unweighted>", "pair_bits<unweighted>", small)
+                      : shared_bits_of<false>("pair_shared_bits<unweighted_unnormalized>",
+                                              "pair_bits<unweighted_unnormalized>", small);
+}
+
 template std::vector<PairKernel<double>> bits_candidates<double>(bool);
 template std::vector<PairKernel<float>> bits_candidates<float>(bool);
 
