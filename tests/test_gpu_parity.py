@@ -586,3 +586,108 @@ def test_whole_number_unweighted_leaves_other_inputs_to_the_stripe_form(ssu, mon
         table.data[3] = np.inf if what == "infinite count" else -2.0
     call = lambda: ssu.one_off_matrix(tree, table, "unweighted_fp64")[0]  # noqa: E731
     np.testing.assert_array_equal(call(), _stripe_mode(monkeypatch, call))
+
+
+# ---- weighted by sample lists (walk from the tips, lists, dense rows)
+
+def _dense_mode(monkeypatch, call):
+    """`call` with the dense pair kernel over the embedding (the general path)."""
+    monkeypatch.setenv("UNIFRAC_B200_WEIGHTED_MODE", "dense")
+    try:
+        return call()
+    finally:
+        monkeypatch.delenv("UNIFRAC_B200_WEIGHTED_MODE")
+
+
+def _polytomy(tree, rng):
+    """The tree with about a third of its internal nodes merged into their parents."""
+    keep = np.ones(len(tree.structure), dtype=bool)
+    stack = []
+    for i, o in enumerate(tree.structure):
+        if o:
+            stack.append(i)
+        else:
+            j = stack.pop()
+            if stack and i - j > 1 and rng.random() < 0.35:
+                keep[i] = keep[j] = False
+    return ssu_synth.BPTree(tree.structure[keep], tree.lengths[keep], [n for n, k in zip(tree.names, keep) if k])
+
+
+def _check_weighted(got, ref, fp64):
+    """fp64: the parity bars.  fp32: the dense fp32 form's own error (sums of
+    single-precision terms over every node), as in the comparisons of the sparse
+    and dense forms above; 1e-6 of the largest value where two samples are close."""
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+    if fp64:
+        check_fp64(np.nan_to_num(got), np.nan_to_num(ref))
+    else:
+        np.testing.assert_allclose(got, ref, rtol=5e-6, atol=1e-6 * max(1.0, float(np.nanmax(np.abs(ref), initial=0))))
+
+
+@pytest.mark.parametrize("n,n_tips,density", [(1, 40, 0.2), (2, 40, 0.2), (33, 1200, 0.01), (37, 3500, 0.9), (129, 300, 0.9),
+                                              (640, 2000, 0.02), (1250, 500, 0.02)])
+@pytest.mark.parametrize("method", ["weighted_normalized", "weighted_unnormalized"])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_weighted_by_lists_matches_the_dense_form(ssu, monkeypatch, method, prec, n, n_tips, density):
+    """Nodes by lists alone, by rows alone and by both; samples of more nodes
+    than shared memory holds (3,500 tips at 90%), a walk in two parts, polytomies,
+    explicit zeros and empty samples; full matrix, bypassed tips, raw counts,
+    condensed, window."""
+    rng = np.random.default_rng(n)
+    tree, table = _case(700 + n, n_tips=n_tips, n_samples=n, density=density, drop=5)
+    tree = _polytomy(tree, rng)
+    table.data[rng.random(table.data.shape[0]) < 0.1] = 0.0
+    table.data[np.isin(table.indices, [n // 2])] = 0.0
+    m = f"{method}_{prec}"
+    stop = (n + 1) // 2
+    calls = [lambda: ssu.one_off_matrix(tree, table, m)[0], lambda: ssu.one_off_matrix(tree, table, m, bypass_tips=True)[0],
+             lambda: ssu.one_off_matrix(tree, table, m, normalize=False)[0], lambda: ssu.one_off(tree, table, m)[0],
+             lambda: ssu.partial(tree, table, m, stop // 3, stop)[0]]
+    for call in calls if n > 1 else calls[:4]:
+        _check_weighted(call(), _dense_mode(monkeypatch, call), prec == "fp64")
+
+
+def test_weighted_by_lists_in_a_batch_as_a_graph_and_in_groups(ssu, monkeypatch):
+    tree = ssu_synth.random_binary_tree(800, 0.1, 5)
+    tips = tree.tip_names()
+    tables = [ssu_synth.geometric_table(tips[3 * i:700 + 20 * i], n, 0.05, 10.0, 60 + i)
+              for i, n in enumerate((5, 64, 200, 33))]
+    for method, fp64 in (("weighted_normalized_fp64", True), ("weighted_unnormalized", False)):
+        def run(group_bytes=0, graph=True):
+            plan = ssu.BatchPlan(tree, tables, method, group_bytes=group_bytes, autotune=0)
+            groups = plan.n_groups()
+            plan.execute()
+            first = plan.results()
+            plan.set_graph(graph)
+            for _ in range(2):
+                plan.execute()
+            for a, b in zip(plan.results(), first):
+                np.testing.assert_array_equal(a, b)
+            plan.close()
+            return first, groups
+        (whole, _), (split, groups) = run(), run(group_bytes=1)
+        assert groups > 1
+        ref, _ = _dense_mode(monkeypatch, run)
+        for a, b, c in zip(whole, split, ref):
+            _check_weighted(a, c, fp64)
+            _check_weighted(b, c, fp64)
+
+
+@pytest.mark.parametrize("what", ["negative length", "infinite count", "two tips of one name"])
+def test_weighted_by_lists_leaves_other_inputs_to_the_embedding(ssu, monkeypatch, what):
+    tree, table = _case(83, n_tips=300, n_samples=70, density=0.1)
+    if what == "negative length":
+        tree.lengths = tree.lengths.copy()
+        tree.lengths[np.flatnonzero(tree.structure)[5]] = -0.01
+    elif what == "infinite count":
+        table.data[3] = np.inf
+    else:
+        names = [i for i, x in enumerate(tree.names) if x]
+        tree.names = list(tree.names)
+        tree.names[names[-1]] = tree.names[names[0]]  # (the last tip is not in the table)
+    for method in ("weighted_normalized_fp64", "unweighted_fp64"):
+        call = lambda: ssu.one_off_matrix(tree, table, method)[0]  # noqa: E731
+        ref = _dense_mode(monkeypatch, call) if method.startswith("weighted") else _stripe_mode(monkeypatch, call)
+        got = call()
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+        check_fp64(np.nan_to_num(got), np.nan_to_num(ref))

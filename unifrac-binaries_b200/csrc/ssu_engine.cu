@@ -21,6 +21,7 @@
 #include "ssu_kernels.cuh"
 #include "ssu_lists.cuh"
 #include "ssu_pairs.cuh"
+#include "ssu_rows.cuh"
 #include "ssu_sparse.cuh"
 #include "ssu_union.cuh"
 
@@ -375,6 +376,7 @@ struct Group {
     // tensor-core path: per operand row, the starting columns of its tips
     uint32_t *d_sample_ptr = nullptr;
     int32_t *d_start_col = nullptr;
+    double *d_start_val = nullptr;       // weighted walk: the entries' counts
     // tensor-core path, one table: first work unit and first row of each
     // band of row blocks (one extra entry closes the list)
     std::vector<uint32_t> band_unit, band_row;
@@ -410,7 +412,22 @@ struct SparseNodes {
     std::vector<std::vector<uint32_t>> entries;
     double scale = 1.0;              // 2^s, exact sums below 2^62
 };
-SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule);
+SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const std::vector<int32_t> &parent,
+                              const ListRule &rule, const std::vector<uint32_t> *height = nullptr);
+
+// Host-built layout of the weighted walk (see build_walk_layout).
+struct WalkLayout {
+    SparseNodes sparse;
+    uint32_t n_cols = 0, sparse0 = 0, dense0 = 0, n_dense = 0;
+    std::vector<int32_t> parent;         // per node column
+    std::vector<int2> child;
+    std::vector<double> len;
+    std::vector<int32_t> kids;
+    std::vector<uint32_t> level;
+    std::vector<int32_t> start_of_obs;
+    double path_max = 0.0;               // longest path from the root to a tip
+};
+WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule, bool fp64);
 
 // Host-built layout of the tensor-core operands (see build_gemm_layout).
 struct GemmLayout {
@@ -451,6 +468,19 @@ struct PlanImpl {
     // (built in setup_gemm instead when no thread can be started)
     std::future<GemmLayout> gemm_layout;
     ListRule list_rule;
+    // the same for the weighted walk, where the tree is large enough to pay
+    // for a thread
+    std::future<WalkLayout> walk_layout;
+    void start_walk_layout(const TableSet &set, const FlatTree &tree) {
+        list_rule = weighted_list_rule(set);
+        if (tree.n_nodes < 8192) return;
+        try {
+            walk_layout = std::async(std::launch::async, build_walk_layout, std::cref(set), std::cref(tree), list_rule,
+                                     spec.fp64);
+        } catch (const std::exception &) {
+            walk_layout = std::future<WalkLayout>();
+        }
+    }
     void start_gemm_layout(const TableSet &set, const FlatTree &tree) {
         list_rule = tc_list_rule(set, tree.n_embedded);
         try {
@@ -561,6 +591,7 @@ struct PlanImpl {
     int setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp, const double *d_len_of_col,
                     uint32_t n, uint32_t first, const std::vector<double> *path,
                     const std::vector<int32_t> &start_of_obs);
+    int list_attributes();
     int reset_lists(cudaStream_t s, const Group &g);
     int shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &out, uint32_t col0, uint32_t col1);
     void gemm_args(tc::GemmArgs &a, const Group &g, const dev::OutSpec &out) const;
@@ -576,6 +607,21 @@ struct PlanImpl {
     cudaStream_t aux[2] = {nullptr, nullptr};
     std::vector<cudaEvent_t> band_ev;
 
+    // weighted methods: node values from a walk over each sample's tips, the
+    // nodes that few samples have by sample lists, the others by the dense
+    // tile kernel over their rows alone
+    bool walk_weighted = false;
+    dev::WalkArgs walk{};
+    uint32_t n_dense_rows = 0;
+    double walk_unit = 1.0;
+    uint32_t *d_close = nullptr;
+    size_t walk_smem = 0;
+    ListRule weighted_list_rule(const TableSet &set) const;
+    template <typename T>
+    int setup_walk_weighted(const TableSet &set, const FlatTree &tree);
+    template <typename T>
+    int walk_weighted_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
+                            uint32_t ntiles, uint32_t splits, bool first, bool last);
     // fp64 unweighted: the nodes that few samples have by sample lists, the
     // others by presence words, both from a walk over each sample's tips (no
     // embedding); n_words counts the dense nodes' words, n_words_all all
@@ -744,7 +790,7 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
     // the hybrid weighted kernel gathers rows at random: narrow groups keep
     // its rows close in memory (measured on 20 replicates of 5,000 samples:
     // 414 ms as one 100k-column group, 377 ms as 5k-column groups)
-    hybrid = !faith && !gemm && !spec.vaw && nonneg_data && set.row_active.empty() &&
+    hybrid = !faith && !gemm && !walk_weighted && !spec.vaw && nonneg_data && set.row_active.empty() &&
              (spec.method == Method::weighted_normalized || spec.method == Method::weighted_unnormalized);
     if (const char *m = std::getenv("UNIFRAC_B200_WEIGHTED_MODE"))
         if (std::string(m) == "dense") hybrid = false;
@@ -789,7 +835,7 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
 
     // per group: the tips' rows in each table, the per-column totals (what the
     // embedding reads; the forms that walk up from the tips have lists of their own)
-    const bool embeds = !gemm && !walk_bits;
+    const bool embeds = !gemm && !walk_bits && !walk_weighted;
     n_tips = static_cast<uint32_t>(tree.leaf_rows.size());
     const bool per_table_len = !faith && !set.row_active.empty();
     for (Group &g : groups) {
@@ -799,6 +845,12 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
             for (uint64_t c = tdesc[t].base / 128; c < (tdesc[t].base + w) / 128; c++) bt[c] = t;
         }
         SSU_CK(upload(&g.d_block_table, bt.data(), sizeof(uint32_t) * bt.size()));
+        if (walk_weighted) {
+            g.totals.assign(g.ld, 0.0);
+            for (uint32_t t = g.t0; t < g.t1; t++)
+                std::copy(set.tables[t]->totals.begin(), set.tables[t]->totals.end(), g.totals.begin() + tdesc[t].base);
+            SSU_CK(upload(&g.d_totals, g.totals.data(), sizeof(double) * g.ld));
+        }
         if (!embeds) continue;
         const uint32_t tg = g.t1 - g.t0;
         std::vector<int32_t> tip_obs(static_cast<size_t>(n_tips) * std::max<uint32_t>(tg, 1), -1);
@@ -1489,6 +1541,12 @@ int PlanImpl::execute_T(cudaStream_t s, const dev::OutSpec &out) {
                 return rc;
             continue;
         }
+        if (walk_weighted) {
+            if (const int rc = walk_weighted_stage<T>(s, g, out, g.d_tiles, g.n_tiles, g.splits, gi == 0,
+                                                      gi + 1 == groups.size()))
+                return rc;
+            continue;
+        }
         int rc = embed<T>(s, g);
         if (!rc) rc = prepare<T>(s, g);
         if (rc) return rc;
@@ -1567,6 +1625,9 @@ int PlanImpl::run_windowed(int mode, void *d_out, uint32_t start, uint32_t stop)
     int rc = 0;
     if (walk_bits) {
         rc = walk_bits_stage(stream, g, o, d_t, nt, s, rows, true, true);
+    } else if (walk_weighted) {
+        rc = spec.fp64 ? walk_weighted_stage<double>(stream, g, o, d_t, nt, s, true, true)
+                       : walk_weighted_stage<float>(stream, g, o, d_t, nt, s, true, true);
     } else if (spec.fp64) {
         rc = embed<double>(stream, g);
         if (!rc) rc = prepare<double>(stream, g);
@@ -1708,13 +1769,17 @@ void add_entry_counts(const TableSet &set, const FlatTree &tree, size_t t, std::
     }
 }
 
-// Every internal row's count becomes the sum over its tips (tip rows hold theirs).
-void sum_over_clades(const FlatTree &tree, std::vector<uint32_t> &counts) {
-    for (uint32_t r : tree.level_rows)  // by height: children first
-        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++) {
-            const uint64_t sum = static_cast<uint64_t>(counts[r]) + counts[tree.child_rows[c]];
-            counts[r] = static_cast<uint32_t>(std::min<uint64_t>(sum, UINT32_MAX));  // (repeated tip names)
-        }
+// Every internal row's count becomes the sum over its tips (tip rows hold
+// theirs): bypassed tips lie behind the embedded rows, which are in postorder.
+void sum_over_clades(const FlatTree &tree, const std::vector<int32_t> &parent, std::vector<uint32_t> &counts) {
+    auto up = [&](uint32_t r) {
+        const int32_t p = parent[r];
+        if (p < 0) return;
+        const uint64_t sum = static_cast<uint64_t>(counts[p]) + counts[r];
+        counts[p] = static_cast<uint32_t>(std::min<uint64_t>(sum, UINT32_MAX));  // (repeated tip names)
+    };
+    for (uint32_t r = tree.n_embedded; r < tree.n_nodes; r++) up(r);
+    for (uint32_t r = 0; r < tree.n_embedded; r++) up(r);
 }
 
 // Embedded rows that are cheaper by sample lists than in the dense form.  The
@@ -1722,34 +1787,44 @@ void sum_over_clades(const FlatTree &tree, std::vector<uint32_t> &counts) {
 // counts twice), so the choice needs the tables' offsets alone.  A row whose
 // length is below 2^(min_bits - 1) units of the fixed point stays out (its
 // rounding would be coarser than the dense form's).
-SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule) {
+SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const std::vector<int32_t> &parent,
+                              const ListRule &rule, const std::vector<uint32_t> *height) {
     SparseNodes sp;
     const uint32_t E = tree.n_embedded;
     sp.id_of_row.assign(E, -1);
+    sp.entries.resize(set.tables.size());
     if (!rule.on || !E) return sp;
     // (a table holds fewer than 2^32 entries, so its counts fit 32 bits)
     const size_t n_tables = set.tables.size();
     std::vector<std::vector<uint32_t>> counts(n_tables);
-    std::vector<uint64_t> bound(E, 0);
-    std::vector<double> square(E, 0.0);  // sum over tables of the bound's square
+    std::vector<uint64_t> sum;
+    std::vector<double> square;  // sum over tables of the bound's square
     uint64_t samples = 0;
     for (size_t t = 0; t < n_tables; t++) {
         samples += set.tables[t]->n_samples;
-        std::vector<uint32_t> &c = counts[t];
-        c.assign(tree.n_nodes, 0);
-        add_entry_counts(set, tree, t, c);
-        sum_over_clades(tree, c);
-        for (uint32_t e = 0; e < E; e++) {
-            bound[e] += c[e];
-            square[e] += static_cast<double>(c[e]) * static_cast<double>(c[e]);
-        }
+        counts[t].assign(tree.n_nodes, 0);
+        add_entry_counts(set, tree, t, counts[t]);
+        sum_over_clades(tree, parent, counts[t]);
     }
-    std::vector<uint8_t> in(E, 0);
+    if (n_tables > 1) {
+        sum.assign(E, 0);
+        square.assign(E, 0.0);
+        for (const std::vector<uint32_t> &c : counts)
+            for (uint32_t e = 0; e < E; e++) {
+                sum[e] += c[e];
+                square[e] += static_cast<double>(c[e]) * static_cast<double>(c[e]);
+            }
+    }
+    auto bound = [&](uint32_t e) -> uint64_t { return n_tables > 1 ? sum[e] : counts[0][e]; };
+    std::vector<uint32_t> rows;
+    rows.reserve(E);
     double total = 0.0, gain = -rule.fixed_s;
     for (uint32_t e = 0; e < E; e++) {
-        const double by_lists = 0.5 * square[e] * rule.pair_s + static_cast<double>(bound[e]) * rule.entry_s;
-        if (bound[e] * rule.min_div > samples || by_lists >= rule.dense_s) continue;
-        in[e] = 1;
+        const uint64_t m = bound(e);
+        const double x = static_cast<double>(m);
+        const double by_lists = 0.5 * (n_tables > 1 ? square[e] : x * x) * rule.pair_s + x * rule.entry_s;
+        if (m * rule.min_div > samples || by_lists >= rule.dense_s) continue;
+        rows.push_back(e);
         gain += rule.dense_s - by_lists;
         total += tree.length[e];
     }
@@ -1757,29 +1832,112 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
     const int s2 = 62 - static_cast<int>(std::ceil(std::log2(total * (1.0 + 1e-12))));
     if (s2 > 1000 || s2 < -1000) return sp;
     sp.scale = std::ldexp(1.0, s2);
-    const double lmin = std::ldexp(1.0, rule.min_bits - 1 - s2);
-    // numbered by decreasing length of their lists (a counting sort): a
-    // sample's nodes then come in that order, and the lists that lanes read side
-    // by side end together
-    std::vector<uint32_t> at(samples + 2, 0);
-    for (uint32_t e = 0; e < E; e++) {
-        in[e] = in[e] && tree.length[e] >= lmin;
-        if (in[e]) at[samples - bound[e] + 1]++;
+    if (rule.min_bits) {
+        const double lmin = std::ldexp(1.0, rule.min_bits - 1 - s2);
+        rows.erase(std::remove_if(rows.begin(), rows.end(), [&](uint32_t e) { return tree.length[e] < lmin; }),
+                   rows.end());
     }
+    // numbered by decreasing length of their lists (within a height, where the
+    // walk needs children first), by counting sorts: a sample's nodes then come
+    // in that order, and the lists that lanes read side by side end together
+    std::vector<uint32_t> at(samples + 2, 0);
+    for (uint32_t e : rows) at[samples - bound(e) + 1]++;
     for (uint64_t i = 1; i < at.size(); i++) at[i] += at[i - 1];
-    sp.row.resize(at.back());
-    for (uint32_t e = 0; e < E; e++)
-        if (in[e]) {
-            sp.id_of_row[e] = static_cast<int32_t>(at[samples - bound[e]]);
-            sp.row[at[samples - bound[e]]++] = e;
-        }
-    sp.entries.resize(n_tables);
+    sp.row.resize(rows.size());
+    for (uint32_t e : rows) sp.row[at[samples - bound(e)]++] = e;
+    if (height) {
+        uint32_t top = 0;
+        for (uint32_t e : rows) top = std::max(top, (*height)[e]);
+        at.assign(top + 2, 0);
+        for (uint32_t e : rows) at[(*height)[e] + 1]++;
+        for (uint32_t i = 1; i < at.size(); i++) at[i] += at[i - 1];
+        for (uint32_t e : sp.row) rows[at[(*height)[e]]++] = e;
+        sp.row.swap(rows);
+    }
+    for (size_t i = 0; i < sp.row.size(); i++) sp.id_of_row[sp.row[i]] = static_cast<int32_t>(i);
     for (size_t t = 0; t < n_tables; t++) {
         sp.entries[t].resize(sp.row.size());
         for (size_t i = 0; i < sp.row.size(); i++)
             sp.entries[t][i] = std::min(counts[t][sp.row[i]], set.tables[t]->n_samples);
     }
     return sp;
+}
+
+// Host part of the weighted walk's setup (no CUDA call).  Node columns:
+// value-only rows (bypassed tips), the sparse nodes and the dense nodes by
+// height, each section from a multiple of 32.
+WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule, bool fp64) {
+    WalkLayout lay;
+    const uint32_t E = tree.n_embedded, K = tree.n_nodes;
+    const std::vector<int32_t> parent_row = parent_rows(tree);
+    std::vector<uint32_t> height(K, 0);
+    uint32_t top = 0;
+    auto lift = [&](uint32_t r) {
+        const int32_t p = parent_row[r];
+        if (p >= 0) height[p] = std::max(height[p], height[r] + 1);
+        top = std::max(top, height[r]);
+    };
+    for (uint32_t r = E; r < K; r++) lift(r);
+    for (uint32_t r = 0; r < E; r++) lift(r);
+    lay.sparse = find_sparse_nodes(set, tree, parent_row, rule, &height);
+    const SparseNodes &sp = lay.sparse;
+    std::vector<uint32_t> dense(E - sp.row.size()), at(top + 2, 0);
+    for (uint32_t e = 0; e < E; e++)
+        if (sp.id_of_row[e] < 0) at[height[e] + 1]++;
+    for (uint32_t h = 1; h < at.size(); h++) at[h] += at[h - 1];
+    for (uint32_t e = 0; e < E; e++)
+        if (sp.id_of_row[e] < 0) dense[at[height[e]]++] = e;
+    lay.n_dense = static_cast<uint32_t>(dense.size());
+    lay.sparse0 = (K - E + 31) / 32 * 32;
+    lay.dense0 = lay.sparse0 + (static_cast<uint32_t>(sp.row.size()) + 31) / 32 * 32;
+    lay.n_cols = std::max(32u, lay.dense0 + (lay.n_dense + 31) / 32 * 32);
+    std::vector<int32_t> col(K);
+    for (uint32_t r = E; r < K; r++) col[r] = static_cast<int32_t>(r - E);
+    auto place = [&](const std::vector<uint32_t> &rows, uint32_t first) {
+        uint32_t h = 0;
+        for (uint32_t i = 0; i < rows.size(); i++) {
+            const uint32_t r = rows[i];
+            col[r] = static_cast<int32_t>(first + i);
+            if (height[r] != h) {  // a level of internal nodes starts (and the one before it ends)
+                if (h) lay.level.push_back(first + i);
+                lay.level.push_back(first + i);
+                h = height[r];
+            }
+        }
+        if (h) lay.level.push_back(first + static_cast<uint32_t>(rows.size()));
+    };
+    place(sp.row, lay.sparse0);
+    place(dense, lay.dense0);
+    lay.parent.assign(lay.n_cols, -1);
+    lay.child.assign(lay.n_cols, make_int2(-1, -1));
+    lay.len.assign(lay.n_cols, 0.0);
+    std::vector<double> path(K);
+    auto down = [&](uint32_t r) {  // parents before children
+        const int32_t p = parent_row[r];
+        const uint32_t c = static_cast<uint32_t>(col[r]);
+        if (p >= 0) lay.parent[c] = col[p];
+        if (r < E) lay.len[c] = fp64 ? tree.length[r] : static_cast<double>(static_cast<float>(tree.length[r]));
+        path[r] = (p >= 0 ? path[p] : 0.0) + lay.len[c];
+        lay.path_max = std::max(lay.path_max, path[r]);
+        const uint32_t k0 = tree.child_ptr[r], k1 = tree.child_ptr[r + 1];
+        if (k1 - k0 <= 2) {
+            if (k1 > k0) lay.child[c].x = col[tree.child_rows[k0]];
+            if (k1 > k0 + 1) lay.child[c].y = col[tree.child_rows[k0 + 1]];
+        } else {
+            lay.child[c] = make_int2(static_cast<int>(lay.kids.size()), -2);
+            lay.kids.push_back(static_cast<int32_t>(k1 - k0));
+            for (uint32_t k = k0; k < k1; k++) lay.kids.push_back(col[tree.child_rows[k]]);
+        }
+    };
+    for (uint32_t r = E; r-- > 0;) down(r);
+    for (uint32_t r = E; r < K; r++) down(r);
+    // every tip starts at its own column
+    uint32_t n_obs = 0;
+    for (uint32_t r : tree.leaf_rows) n_obs = std::max<uint32_t>(n_obs, tree.leaf_obs[r] + 1);
+    lay.start_of_obs.assign(n_obs, -1);
+    for (uint32_t r : tree.leaf_rows)
+        if (tree.leaf_obs[r] >= 0) lay.start_of_obs[tree.leaf_obs[r]] = col[r];
+    return lay;
 }
 
 // Host part of the tensor-core setup (no CUDA call, so it runs on a worker
@@ -1795,7 +1953,8 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
 GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule) {
     GemmLayout lay;
     const uint32_t E = tree.n_embedded;
-    lay.sparse = find_sparse_nodes(set, tree, rule);
+    const std::vector<int32_t> parent_row = parent_rows(tree);
+    lay.sparse = find_sparse_nodes(set, tree, parent_row, rule);
     const std::vector<int32_t> &sparse_of = lay.sparse.id_of_row;
     uint32_t n_dense = 0;  // contracted rows
     // order by binary exponent of |length|, largest first, by row within an
@@ -1893,7 +2052,6 @@ GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const Li
         for (int i = 0; i < 4; i++) lay.digits[static_cast<size_t>(i) * k_pad + c] = d[i];
     }
     // parents among embedded nodes
-    const std::vector<int32_t> parent_row = parent_rows(tree);
     lay.parent_col.assign(lay.lsorted.size(), -1);
     for (uint32_t r = 0; r < E; r++) {
         const int32_t p = parent_row[r];
@@ -1918,6 +2076,7 @@ int PlanImpl::setup_sample_lists(const TableSet &set, const std::vector<int32_t>
         SSU_CK(alloc(&d_fill, sizeof(uint32_t) * g.ld));
         SSU_CK(alloc(&g.d_sample_ptr, sizeof(uint32_t) * (g.ld + 1)));
         SSU_CK(alloc(&g.d_start_col, sizeof(int32_t) * std::max<uint64_t>(nnz_g, 1)));
+        if (walk_weighted) SSU_CK(alloc(&g.d_start_val, sizeof(double) * std::max<uint64_t>(nnz_g, 1)));
         SSU_CK(cudaMemsetAsync(d_count, 0, sizeof(uint32_t) * g.ld, stream));
         std::vector<int32_t *> d_row_start(g.t1 - g.t0, nullptr);
         for (uint32_t t = g.t0; t < g.t1; t++) {
@@ -1946,7 +2105,7 @@ int PlanImpl::setup_sample_lists(const TableSet &set, const std::vector<int32_t>
                 const uint64_t threads = static_cast<uint64_t>(tb.n_obs) * 32;
                 tc::sample_lists_kernel<<<static_cast<uint32_t>((threads + 255) / 256), 256, 0, stream>>>(
                     d_indptr + d.indptr_off, d_indices + d.nnz_off, d_data + d.nnz_off, d_row_start[t - g.t0],
-                    tb.n_obs, d.base, d_count, pass ? d_fill : nullptr, g.d_start_col);
+                    tb.n_obs, d.base, d_count, pass ? d_fill : nullptr, g.d_start_col, g.d_start_val);
             }
         }
         SSU_CK(cudaGetLastError());
@@ -2104,10 +2263,11 @@ int PlanImpl::shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &
     const uint32_t threads = cols > 4096 ? 768 : cols > 2048 ? 512 : 256;
     const size_t smem = 2 * sizeof(uint32_t) * cols;
     const dim3 grid(col1 - col0, chunks);
-    if (g.lists.wide)
-        dev::shared_sums_kernel<uint32_t><<<grid, threads, smem, s>>>(g.lists, out, col0, cols, chunk);
-    else
-        dev::shared_sums_kernel<uint16_t><<<grid, threads, smem, s>>>(g.lists, out, col0, cols, chunk);
+    const auto kernel = walk_weighted ? (g.lists.wide ? dev::shared_sums_kernel<uint32_t, true>
+                                                      : dev::shared_sums_kernel<uint16_t, true>)
+                                      : (g.lists.wide ? dev::shared_sums_kernel<uint32_t, false>
+                                                      : dev::shared_sums_kernel<uint16_t, false>);
+    kernel<<<grid, threads, smem, s>>>(g.lists, out, col0, cols, chunk);
     launches++;
     SSU_CK(cudaGetLastError());
     return 0;
@@ -2120,7 +2280,7 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
                           const std::vector<int32_t> &start_of_obs) {
     n_sparse = static_cast<uint32_t>(sp.row.size());
     sparse_unit = 1.0 / sp.scale;
-    if (!n_sparse && !path) return setup_sample_lists(set, start_of_obs);
+    if (!n_sparse && !path && !walk_weighted) return setup_sample_lists(set, start_of_obs);
     SSU_CK(alloc(&d_sparse_q, sizeof(unsigned long long) * n));
     SSU_CK(alloc(&d_list_unit, sizeof(double)));
     double *d_path = nullptr;
@@ -2149,10 +2309,11 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
             last_error = "too many table entries for the sparse nodes' lists";
             return kOutputError;
         }
-        // parts of at least a wave of blocks of the walk
+        // parts of at least a wave of blocks of the walk (for the weighted
+        // walk two thirds: its shared sums read ten bytes an entry)
         la.slots = static_cast<uint64_t>(tg) * n_sparse;
         la.parts = static_cast<uint32_t>(
-            std::max<uint64_t>(1, std::min<uint64_t>(dev::LIST_PARTS, g.ld / (8 * static_cast<uint64_t>(n_sms)))));
+            std::max<uint64_t>(1, std::min<uint64_t>(dev::LIST_PARTS, g.ld / ((walk_weighted ? 4 : 8) * static_cast<uint64_t>(n_sms)))));
         uint32_t n_max = 1;
         for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);
         while (dev::list_part_rows(n_max, la.parts) > kSharedCols) la.parts *= 2;  // (a part's columns fit a block)
@@ -2178,7 +2339,15 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
         la.count = reinterpret_cast<uint32_t *>(la.cursor + 1);
         SSU_CK(alloc(&la.idx, bytes));
         g.list_bytes = bytes;
+        if (walk_weighted)  // the sample side holds the dense nodes too
+            for (uint32_t t = g.t0; t < g.t1; t++) ids += static_cast<uint64_t>(tdesc[t].n) * n_dense_rows;
         SSU_CK(alloc(&la.node, sizeof(uint32_t) * std::max<uint64_t>(ids, 1)));
+        if (walk_weighted) {
+            SSU_CK(alloc(&la.node_all, sizeof(uint32_t) * g.ld));
+            SSU_CK(alloc(&la.idx_q, sizeof(unsigned long long) * std::max<uint64_t>(at, 1) * dev::LIST_ALIGN));
+            SSU_CK(alloc(&la.node_q, sizeof(unsigned long long) * std::max<uint64_t>(ids, 1)));
+            SSU_CK(alloc(&la.node_u, sizeof(double) * std::max<uint64_t>(ids, 1)));
+        }
         SSU_CK(alloc(&la.node_ptr, sizeof(unsigned long long) * g.ld));
         SSU_CK(alloc(&la.node_cnt, sizeof(uint32_t) * g.ld));
         SSU_CK(alloc(&la.rs, sizeof(unsigned long long) * g.ld));
@@ -2187,6 +2356,7 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
     if (const int rc = setup_sample_lists(set, start_of_obs)) return rc;
     for (Group &g : groups)  // the padding after each list reads as sample 0, which no row adds
         if (n_sparse) SSU_CK(cudaMemsetAsync(g.lists.idx, 0, std::max<size_t>(g.list_bytes, 1), stream));
+    if (walk_weighted) return list_attributes();
     unsigned long long *d_top = nullptr;
     if (path) {
         SSU_CK(alloc(&d_top, sizeof(unsigned long long)));
@@ -2198,9 +2368,14 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
     dev::fixed_lengths_kernel<<<(n + 255) / 256, 256, 0, stream>>>(d_len_of_col, n, d_top, sp.scale, d_sparse_q,
                                                                   d_list_unit);
     SSU_CK(cudaGetLastError());
-    constexpr int smem = static_cast<int>(2 * sizeof(uint32_t) * kSharedCols);
-    SSU_CK(cudaFuncSetAttribute(dev::shared_sums_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    SSU_CK(cudaFuncSetAttribute(dev::shared_sums_kernel<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    return list_attributes();
+}
+
+int PlanImpl::list_attributes() {
+    for (auto kernel : {dev::shared_sums_kernel<uint16_t, false>, dev::shared_sums_kernel<uint32_t, false>,
+                        dev::shared_sums_kernel<uint16_t, true>, dev::shared_sums_kernel<uint32_t, true>})
+        SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(2 * sizeof(uint32_t) * kSharedCols)));
     return 0;
 }
 
@@ -2271,6 +2446,219 @@ int PlanImpl::execute_gemm(cudaStream_t s, const dev::OutSpec &out) {
     return 0;
 }
 
+// ----------------------------------------------- weighted by sample lists
+
+// Nodes left to the sample lists by weighted methods.  A dense row costs 0.13 ps
+// (fp64) or 0.09 ps (fp32) a pair of all samples, at least 10 ns where the
+// tables do not fill the SMs; by lists a node costs 1.2 ps a pair of its samples
+// and 100 ps a sample.  Dense costs of 0.05, 0.09, 0.13, 0.20, 0.30 ps: 2,048
+// samples x 20,000 tips, fp64, 1,413, 1,309, 1,293, 1,317, 1,372 us; four
+// replicates of 5,000 samples, fp32, 13.31, 12.62, 12.67, 13.08, 13.73 ms.
+ListRule PlanImpl::weighted_list_rule(const TableSet &set) const {
+    ListRule r;
+    r.on = true;
+    double pairs = 0.0;
+    for (const Table *t : set.tables) pairs += 0.5 * t->n_samples * static_cast<double>(t->n_samples);
+    r.dense_s = std::max(pairs * (spec.fp64 ? 1.3e-13 : 9e-14), 1e-8);
+    r.pair_s = 1.2e-12;
+    r.entry_s = 1e-10;
+    r.min_div = 1;
+    return r;
+}
+
+template <typename T>
+int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
+    SetupTimer timer;
+    const WalkLayout lay =
+        walk_layout.valid() ? walk_layout.get() : build_walk_layout(set, tree, list_rule, spec.fp64);
+    const SparseNodes &sp = lay.sparse;
+    const uint32_t n_cols = lay.n_cols;
+    // a sample's sum of L u is at most its total times the longest path
+    double vmax = 1.0;
+    if (!spec.normalize)
+        for (const Group &g : groups)
+            for (double t : g.totals) vmax = std::max(vmax, t);
+    int x = 0;
+    std::frexp(std::max(lay.path_max * vmax * (1.0 + 1e-9), 1e-290), &x);
+    const double scale = std::ldexp(1.0, std::min(62 - x, 1000));
+    walk_unit = 1.0 / scale;
+    n_dense_rows = lay.n_dense;
+    timer.step("walk_layout");
+
+    PairKernel<T> &k = kern<T>();
+    k = PairKernel<T>();
+    k.BM = k.BN = dev::RB;
+    k.name = spec.method == Method::weighted_normalized ? "pair_hybrid<weighted_normalized>" : "pair_hybrid<weighted_unnormalized>";
+    k.shape = "128x128/4x8";
+    uint32_t max_tiles = 1;
+    hpartial_bytes = 0;
+    for (Group &g : groups) {
+        std::vector<uint4> tiles;
+        for (uint32_t t = g.t0; t < g.t1; t++) append_tiles(tiles, t, tdesc[t].base, tdesc[t].n, dev::RB, dev::RB, false, 0, 0);
+        g.n_tiles = static_cast<uint32_t>(tiles.size());
+        max_tiles = std::max(max_tiles, g.n_tiles);
+        SSU_CK(upload(&g.d_tiles, tiles.data(), sizeof(uint4) * tiles.size()));
+        // Row splits so the tiles fill the SMs (one CTA per SM), in us: a row
+        // of a tile takes 0.27 (fp64) or 0.16, its end 12; a split tile's sums
+        // are written and read again, 4 each way, by a launch of its own.
+        double best = 1e300;
+        const double row_us = spec.fp64 ? 0.27 : 0.16;
+        const uint32_t max_s = std::max<uint32_t>(1, std::min<uint32_t>(64, n_dense_rows / 32));
+        for (uint32_t q = 1; q <= max_s; q++) {
+            const double waves = std::ceil(static_cast<double>(g.n_tiles) * q / n_sms);
+            double cost = waves * (n_dense_rows * row_us / q + (q > 1 ? 4.0 : 12.0));
+            if (q > 1) cost += 5.0 + std::ceil(static_cast<double>(g.n_tiles) / n_sms) * (4.0 * q + 12.0);
+            if (cost < best) {
+                best = cost;
+                g.splits = q;
+            }
+        }
+        if (g.splits > 1)
+            hpartial_bytes = std::max(hpartial_bytes, sizeof(double) * dev::RB * dev::RB * g.n_tiles * g.splits);
+    }
+    double *d_len_c = nullptr;
+    int32_t *d_par = nullptr, *d_kids = nullptr;
+    int2 *d_child = nullptr;
+    uint32_t *d_level = nullptr;
+    SSU_CK(upload(&d_len_c, lay.len.data(), sizeof(double) * n_cols));
+    SSU_CK(upload(&d_par, lay.parent.data(), sizeof(int32_t) * n_cols));
+    SSU_CK(upload(&d_child, lay.child.data(), sizeof(int2) * n_cols));
+    SSU_CK(upload(&d_kids, lay.kids.data(), sizeof(int32_t) * lay.kids.size()));
+    SSU_CK(upload(&d_level, lay.level.data(), sizeof(uint32_t) * lay.level.size()));
+    if (const int rc = setup_lists(set, tree, sp, nullptr, 1, 0, nullptr, lay.start_of_obs)) return rc;
+    walk.parent = d_par;
+    walk.child = d_child;
+    walk.kids = d_kids;
+    walk.level = d_level;
+    walk.n_levels = static_cast<uint32_t>(lay.level.size() / 2);
+    walk.len = d_len_c;
+    walk.normalize = spec.normalize ? 1 : 0;
+    walk.n_words = n_cols / 32;
+    walk.sparse0 = lay.sparse0;
+    walk.dense0 = lay.dense0;
+    walk.n_dense = n_dense_rows;
+    walk.scale = scale;
+    // values in shared memory for samples of up to `cap` nodes (WALK_BLOCKS an
+    // SM), else in memory; no more than every column
+    const size_t fixed = sizeof(uint32_t) * (2ull * walk.n_words + 1 + 2ull * walk.n_levels + 4);
+    constexpr size_t block = 227 * 1024 / dev::WALK_BLOCKS - 1536;  // (1 KB of it the system's)
+    const size_t room = fixed + 8 * 1024 < block ? block - fixed : 8 * 1024;
+    walk.cap = std::min<uint32_t>(n_cols, static_cast<uint32_t>(room / 12));
+    walk_smem = static_cast<size_t>(walk.cap) * 12 + fixed + 8;
+    uint64_t spill = 0;  // nodes of all samples of a group, at most
+    for (const Group &g : groups) {
+        uint64_t m = 0;
+        for (uint32_t t = g.t0; t < g.t1; t++) {
+            for (uint32_t c : sp.entries[t]) m += c;
+            m += static_cast<uint64_t>(tdesc[t].n) * n_dense_rows + set.tables[t]->nnz();
+        }
+        spill = std::max(spill, m);
+    }
+    if (walk.cap >= n_cols) spill = 1;
+    SSU_CK(alloc(&walk.spill, sizeof(double) * spill));
+    SSU_CK(alloc(&walk.spill_id, sizeof(uint32_t) * spill));
+    SSU_CK(alloc(&walk.spill_cursor, sizeof(unsigned long long)));
+    SSU_CK(alloc(&d_U, sizeof(T) * ld * std::max(n_dense_rows, 1u)));
+    SSU_CK(cudaMemsetAsync(d_U, 0, sizeof(T) * ld * std::max(n_dense_rows, 1u), stream));
+    SSU_CK(alloc(&d_W, sizeof(T) * ld));
+    SSU_CK(alloc(&d_full, sizeof(T) * std::max<uint64_t>(full_elems, 1)));
+    if (sizeof(T) == sizeof(double))
+        d_Sq = static_cast<unsigned long long *>(d_full);  // written only after its sum is read
+    else
+        SSU_CK(alloc(&d_Sq, sizeof(unsigned long long) * std::max<uint64_t>(full_elems, 1)));
+    SSU_CK(alloc(&d_flags, sizeof(int) * max_tiles));
+    SSU_CK(alloc(&d_close, sizeof(uint32_t) * (dev::RB * dev::RB / 32) * max_tiles));
+    if (hpartial_bytes) SSU_CK(alloc(&d_hpartial, hpartial_bytes));
+    for (auto kernel : {dev::pair_rows_kernel<T, true>, dev::pair_rows_kernel<T, false>,
+                        dev::rows_finalize_kernel<T, true>, dev::rows_finalize_kernel<T, false>})
+        SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(dev::rows_smem<T>())));
+    SSU_CK(cudaFuncSetAttribute(dev::weighted_walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(tc::MAX_BITMAP_BYTES)));
+    tuning = "sample lists";
+    timer.step("walk_buffers");
+    return 0;
+}
+
+// One group: the walk (dense rows, lists, one-sided sums), the sparse nodes'
+// shared sums, the dense tile kernel (+ split finalize), then the close pairs.
+template <typename T>
+int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
+                                  uint32_t ntiles, uint32_t splits, bool first, bool last) {
+    if (const int rc = reset_lists(s, g)) return rc;
+    const dev::ListArgs &la = g.lists;
+    dev::WalkArgs w = walk;
+    w.sample_ptr = g.d_sample_ptr;
+    w.start = g.d_start_col;
+    w.start_val = g.d_start_val;
+    w.totals = g.d_totals;
+    w.ld = g.ld;
+    SSU_CK(cudaMemsetAsync(walk.spill_cursor, 0, sizeof(unsigned long long), s));
+    if (groups.size() > 1)  // (the entries of one group are the same in every pass)
+        SSU_CK(cudaMemsetAsync(d_U, 0, sizeof(T) * g.ld * std::max(n_dense_rows, 1u), s));
+    for (uint32_t p = 0; p < la.parts; p++) {
+        if (p)
+            SSU_CK(cudaMemcpyAsync(la.part_count + (p - 1) * la.slots, la.count, sizeof(uint32_t) * la.slots,
+                                   cudaMemcpyDeviceToDevice, s));
+        const uint32_t c0 = g.part_col[p], c1 = g.part_col[p + 1];
+        if (c1 <= c0) continue;
+        dev::weighted_walk_kernel<T><<<c1 - c0, 256, walk_smem, s>>>(w, static_cast<T *>(d_U), static_cast<T *>(d_W),
+                                                                    g.d_columns + c0, la);
+        launches++;
+    }
+    SSU_CK(cudaGetLastError());
+    if (first && timed()) SSU_CK(cudaEventRecord(ev[1], s));
+    if (ntiles) {
+        dev::SharedOut so;
+        so.S = d_Sq;
+        if (n_sparse) {
+            if (const int rc = shared_sums(s, g, so, 0, static_cast<uint32_t>(g.ld))) return rc;
+        } else {
+            for (uint32_t t = g.t0; t < g.t1; t++)
+                SSU_CK(cudaMemsetAsync(d_Sq + tdesc[t].out_off, 0,
+                                       sizeof(unsigned long long) * tdesc[t].n * static_cast<size_t>(tdesc[t].n), s));
+        }
+        SSU_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * ntiles, s));
+        dev::RowsArgs<T> h{};
+        h.tiles = tiles;
+        h.n_tiles = ntiles;
+        h.n_splits = std::max<uint32_t>(splits, 1);
+        h.tables = d_tdesc;
+        h.U = static_cast<const T *>(d_U);
+        h.n_rows = n_dense_rows;
+        h.ld = g.ld;
+        h.W = static_cast<const T *>(d_W);
+        h.S = d_Sq;
+        h.rs = la.rs;
+        h.unit = walk_unit;
+        h.tau = 0.02;
+        h.tile_flags = d_flags;
+        h.close = d_close;
+        h.partial = h.n_splits > 1 ? d_hpartial : nullptr;
+        h.out = out;
+        const bool norm = spec.method == Method::weighted_normalized;
+        const uint32_t ctas = static_cast<uint32_t>(
+            std::min<uint64_t>(static_cast<uint64_t>(ntiles) * h.n_splits, static_cast<uint64_t>(n_sms)));
+        constexpr size_t smem = dev::rows_smem<T>();
+        const auto pairs = norm ? dev::pair_rows_kernel<T, true> : dev::pair_rows_kernel<T, false>;
+        pairs<<<ctas, dev::RTHREADS, smem, s>>>(h);
+        launches++;
+        if (h.partial) {
+            const auto finalize = norm ? dev::rows_finalize_kernel<T, true> : dev::rows_finalize_kernel<T, false>;
+            finalize<<<ntiles, dev::RTHREADS, smem, s>>>(h);
+            launches++;
+        }
+        {
+            const auto close = norm ? dev::close_pairs_kernel<T, true> : dev::close_pairs_kernel<T, false>;
+            close<<<ntiles, 256, 0, s>>>(h, la, walk.len + walk.sparse0);
+            launches++;
+        }
+        SSU_CK(cudaGetLastError());
+    }
+    if (last && timed()) SSU_CK(cudaEventRecord(ev[2], s));
+    return 0;
+}
+
 // ------------------------------------------- fp64 unweighted by presence words
 
 // Nodes left to the sample lists in the whole-number form.  A dense node costs
@@ -2297,7 +2685,8 @@ ListRule PlanImpl::bits_list_rule(const TableSet &set) const {
 int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     SetupTimer timer;
     const ListRule rule = bits_list_rule(set);
-    const SparseNodes sp = find_sparse_nodes(set, tree, rule);
+    const std::vector<int32_t> parent_row = parent_rows(tree);
+    const SparseNodes sp = find_sparse_nodes(set, tree, parent_row, rule);
     // columns: the dense rows in order, padded to whole words, then the sparse nodes
     uint32_t n_dense = 0;
     std::vector<int32_t> col(tree.n_nodes, -1);
@@ -2309,7 +2698,7 @@ int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     n_words_all = n_words + (static_cast<uint32_t>(sp.row.size()) + 63) / 64;
     const uint32_t n_cols = std::max(1u, n_words_all * 64);
     std::vector<double> len(n_cols, 0.0), path(n_cols, 0.0);
-    std::vector<int32_t> parent(n_cols, -1), parent_row = parent_rows(tree);
+    std::vector<int32_t> parent(n_cols, -1);
     for (uint32_t r = E; r-- > 0;) {  // parents follow their children
         const int32_t p = parent_row[r];
         len[col[r]] = tree.length[r];
@@ -2529,24 +2918,56 @@ bool use_tensor_cores(const MethodSpec &spec, const TableSet &set, const FlatTre
     return want;
 }
 
-// fp64 unweighted results from presence words and sample lists: counts and
-// lengths that are not negative and finite (presence is then "some tip below
-// has a count", and lists hold whole-number lengths), one length per node for
-// all tables, a bitmap of the nodes in shared memory, and no request for the
-// plain stripe form.
-bool use_walk_bits(const MethodSpec &spec, const TableSet &set, const FlatTree &tree) {
-    if (!spec.fp64 || spec.vaw || spec.unweighted_stripe || !set.row_active.empty() ||
-        !(spec.method == Method::unweighted || spec.method == Method::unweighted_unnormalized))
-        return false;
-    if (tree.n_embedded / 8 + 64 > tc::MAX_BITMAP_BYTES) return false;
-    for (uint32_t e = 0; e < tree.n_embedded; e++)
+// What the walks over each sample's tips need: counts and lengths that are not
+// negative and finite (a node is then present where some tip below has a
+// count), one length per node for all tables, one tip per observation, and
+// `bits` bits of shared memory per node.
+bool can_walk(const TableSet &set, const FlatTree &tree, uint64_t bits) {
+    if (!set.row_active.empty() || (tree.n_nodes + 2048) * bits / 8 > tc::MAX_BITMAP_BYTES - 16 * 1024) return false;
+    for (uint32_t e = 0; e < tree.n_nodes; e++)
         if (!(tree.length[e] >= 0.0 && std::isfinite(tree.length[e]))) return false;
     for (const Table *t : set.tables) {
         if (!t->nonneg) return false;
         for (double x : t->totals)
             if (!std::isfinite(x)) return false;
     }
+    std::vector<uint8_t> seen;
+    for (uint32_t r : tree.leaf_rows) {
+        const int32_t o = tree.leaf_obs[r];
+        if (o < 0) continue;
+        if (static_cast<size_t>(o) >= seen.size()) seen.resize(std::max<size_t>(2 * seen.size(), o + 1), 0);
+        if (seen[o]) return false;
+        seen[o] = 1;
+    }
     return true;
+}
+
+// fp64 unweighted results in whole numbers, unless the plain stripe form is
+// asked for.
+bool use_walk_bits(const MethodSpec &spec, const TableSet &set, const FlatTree &tree) {
+    return spec.fp64 && !spec.vaw && !spec.unweighted_stripe &&
+           (spec.method == Method::unweighted || spec.method == Method::unweighted_unnormalized) &&
+           can_walk(set, tree, 1);
+}
+
+// Weighted results by sample lists, unless the dense kernel or the tile walk
+// is asked for.
+bool use_walk_weighted(const MethodSpec &spec, const TableSet &set, const FlatTree &tree) {
+    if (spec.vaw || !(spec.method == Method::weighted_normalized || spec.method == Method::weighted_unnormalized))
+        return false;
+    if (const char *m = std::getenv("UNIFRAC_B200_WEIGHTED_MODE"))
+        if (std::string(m) == "dense") return false;
+    if (!env_int("UNIFRAC_B200_HYBRID_SCATTER", 1)) return false;
+    // an explicit zero of a sample without counts is 0 / 0, and its distances
+    // are NaN: the embedding's business
+    if (spec.normalize)
+        for (const Table *t : set.tables) {
+            bool empty = false;
+            for (double x : t->totals) empty = empty || x == 0.0;
+            for (uint64_t q = 0; empty && q < t->nnz(); q++)
+                if (t->totals[t->indices[q]] == 0.0) return false;
+        }
+    return can_walk(set, tree, 2) && tree.level_ptr.size() <= 4096;  // presence and ranks; the levels' ranks
 }
 
 }  // namespace
@@ -2564,11 +2985,15 @@ int Plan::create(const Table &table, const FlatTree &tree, const MethodSpec &spe
     set.embedded.push_back(tree.n_embedded);
     m.gemm = use_tensor_cores(spec, set, tree, false);
     m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
+    m.walk_weighted = use_walk_weighted(spec, set, tree);
     if (m.gemm) m.start_gemm_layout(set, tree);
+    if (m.walk_weighted) m.start_walk_layout(set, tree);
     int rc = m.setup(set, tree, BatchOptions{});
     if (!rc)
         rc = m.gemm        ? m.setup_gemm(set, tree)
              : m.walk_bits ? m.setup_walk_bits(set, tree)
+             : m.walk_weighted
+                 ? (spec.fp64 ? m.setup_walk_weighted<double>(set, tree) : m.setup_walk_weighted<float>(set, tree))
              : spec.fp64   ? m.setup_method<double>()
                            : m.setup_method<float>();
     if (rc) {
@@ -2597,11 +3022,15 @@ int Plan::create_batch(const TableSet &set, const FlatTree &tree, const MethodSp
     m.autotune = resolve_autotune(opts.autotune, true);
     m.gemm = use_tensor_cores(spec, set, tree, true);
     m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
+    m.walk_weighted = use_walk_weighted(spec, set, tree);
     if (m.gemm) m.start_gemm_layout(set, tree);
+    if (m.walk_weighted) m.start_walk_layout(set, tree);
     int rc = m.setup(set, tree, opts);
     if (!rc)
         rc = m.gemm        ? m.setup_gemm(set, tree)
              : m.walk_bits ? m.setup_walk_bits(set, tree)
+             : m.walk_weighted
+                 ? (spec.fp64 ? m.setup_walk_weighted<double>(set, tree) : m.setup_walk_weighted<float>(set, tree))
              : spec.fp64   ? m.setup_method<double>()
                            : m.setup_method<float>();
     if (rc) {

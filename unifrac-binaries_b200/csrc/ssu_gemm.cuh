@@ -533,12 +533,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 // device: table row i (one warp) whose observation starts at column
 // row_start[i] >= 0 gives every sample j with a positive count one entry in
 // operand row base + j.  Counting pass (fill == nullptr): count[base + j]++;
-// placing pass: start_col[fill[base + j]++] = row_start[i].  The order within
+// placing pass: start_col[fill[base + j]++] = row_start[i] (and the count into
+// start_val, unless null).  The order within
 // a sample's list varies; the rows kernel only takes the union of the paths.
 __global__ void sample_lists_kernel(const uint32_t *__restrict__ indptr, const uint32_t *__restrict__ indices,
                                     const double *__restrict__ data, const int32_t *__restrict__ row_start,
                                     uint32_t n_rows, uint32_t base, uint32_t *__restrict__ count,
-                                    uint32_t *__restrict__ fill, int32_t *__restrict__ start_col) {
+                                    uint32_t *__restrict__ fill, int32_t *__restrict__ start_col,
+                                    double *__restrict__ start_val) {
     const uint64_t w = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
     const uint32_t lane = threadIdx.x % 32;
     if (w >= n_rows) return;
@@ -547,10 +549,13 @@ __global__ void sample_lists_kernel(const uint32_t *__restrict__ indptr, const u
     for (uint32_t q = indptr[w] + lane; q < indptr[w + 1]; q += 32) {
         if (!(data[q] > 0.0)) continue;
         const uint32_t col = base + indices[q];
-        if (fill)
-            start_col[atomicAdd(fill + col, 1u)] = st;
-        else
+        if (fill) {
+            const uint32_t at = atomicAdd(fill + col, 1u);
+            start_col[at] = st;
+            if (start_val) start_val[at] = data[q];
+        } else {
             atomicAdd(count + col, 1u);
+        }
     }
 }
 

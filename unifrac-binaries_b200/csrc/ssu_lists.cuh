@@ -1,6 +1,6 @@
-// Unweighted sums over nodes that few samples have, through sample lists.
+// Sums over nodes that few samples have, through sample lists.
 //
-// For a set S of sparse nodes and a pair (k, l),
+// Unweighted.  For a set S of sparse nodes and a pair (k, l),
 //   sum_{n in S, k has n and l not} L_n = rs_k - shared_kl,
 //   rs_k = sum_{n in S, k has n} L_n,  shared_kl = sum_{n in S, both have n} L_n,
 // and shared_kl only needs, for sample k, the lists of the samples of k's own
@@ -10,6 +10,14 @@
 // so the differences above are exact sums of the q: no cancellation (two
 // samples with the same nodes differ by exactly 0), and no dependence on the
 // order of the additions.
+//
+// Weighted.  With q_n(k) = round(L_n u_n(k) 2^s), u the node's proportion in
+// the sample (or its counts),
+//   sum_{n in S} L |u(k) - u(l)| 2^s = rs_k + rs_l - 2 sum min(q_n(k), q_n(l)),
+// rs_k = sum q_n(k): the same sums with min(q(k), q(l)) in place of q, exact in
+// the same way (rounding keeps the order, so the smaller q is the smaller
+// value's).  A sample's rs never exceeds its total times the longest path from
+// the root to a tip, which sets the scale.
 //
 // Lists (built by the walk over each sample's tips, per execute):
 //   node side:   per (table, node) the table's samples that have it, 16 or 32
@@ -53,6 +61,11 @@ struct ListArgs {
     uint32_t parts = 1;                  // parts of a table's samples, each list_part_rows long
     uint32_t *part_count = nullptr;      // [parts - 1][slots]: entries before part 1, 2, ...
     uint64_t slots = 0;
+    // weighted: q of each entry, node side and sample side; on the sample side
+    // u too, and the dense nodes behind the sparse ones (node_all of both)
+    unsigned long long *idx_q = nullptr, *node_q = nullptr;
+    double *node_u = nullptr;
+    uint32_t *node_all = nullptr;
 };
 
 // Samples per part of a table of n samples.
@@ -243,7 +256,7 @@ __device__ __forceinline__ void shared_carry_below(uint32_t addr, uint32_t v, ui
 // the first one's old value add 64 bits at about 1e12 entries/s over the
 // chip, a 64-bit shared atomic at 4.4e11/s.  A block reads only the parts of
 // its chunk, from k's own on.
-template <typename IDX>
+template <typename IDX, bool WEIGHTED>
 __global__ void __launch_bounds__(768, 2)
     shared_sums_kernel(const ListArgs la, const SharedOut out, uint32_t col0, uint32_t cols, uint32_t chunk) {
     extern __shared__ uint32_t acc_s[];  // lo[cols], hi[cols]
@@ -289,20 +302,28 @@ __global__ void __launch_bounds__(768, 2)
             // down to a whole step's boundary (entries of other parts are not in the chunk)
             v.p0 = before ? before[e] & ~(LIST_ALIGN - 1) : 0u;
             v.off = la.off[slot0 + e];
-            v.q = la.q[e];
+            if (!WEIGHTED) v.q = la.q[e];
             return v;
         };
+        const unsigned long long *own = WEIGHTED ? la.node_q + la.node_ptr[j] : nullptr;
         uint32_t i = grp;
         Node next{};
         uint32_t id = 0;
-        if (i < n_ids) next = bounds(ids[i]);
+        if (i < n_ids) {
+            next = bounds(ids[i]);
+            if (WEIGHTED) next.q = own[i];
+        }
         if (i + groups < n_ids) id = ids[i + groups];
         for (; i < n_ids; i += groups) {
             const Node cur = next;
-            if (i + groups < n_ids) next = bounds(id);
+            if (i + groups < n_ids) {
+                next = bounds(id);
+                if (WEIGHTED) next.q = own[i + groups];
+            }
             if (i + 2 * groups < n_ids) id = ids[i + 2 * groups];
             const uint32_t m = cur.m, p0 = cur.p0;
             const IDX *list = idx + static_cast<uint64_t>(cur.off) * LIST_ALIGN;
+            const unsigned long long *list_q = WEIGHTED ? la.idx_q + static_cast<uint64_t>(cur.off) * LIST_ALIGN : nullptr;
             const uint32_t ql = static_cast<uint32_t>(cur.q), qh = static_cast<uint32_t>(cur.q >> 32);
             for (uint32_t p = p0 + gl * QE; p < m; p += GL * QE) {
                 uint32_t l[QE];
@@ -322,15 +343,33 @@ __global__ void __launch_bounds__(768, 2)
                 // (entries past the list's end are 0, never > k; those of other
                 // parts are outside the chunk)
                 uint32_t at[QE], old[QE];
+                uint32_t vl[QE], vh[QE];  // what each entry adds
+                if constexpr (WEIGHTED) {
+                    const ulonglong2 *qp = reinterpret_cast<const ulonglong2 *>(list_q + p);
+                    const ulonglong2 q01 = qp[0], q23 = qp[1];
+                    const unsigned long long qe[QE] = {q01.x, q01.y, q23.x, q23.y};
+#pragma unroll
+                    for (uint32_t x = 0; x < QE; x++) {
+                        const unsigned long long v = qe[x] < cur.q ? qe[x] : cur.q;
+                        vl[x] = static_cast<uint32_t>(v);
+                        vh[x] = static_cast<uint32_t>(v >> 32);
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t x = 0; x < QE; x++) {
+                        vl[x] = ql;
+                        vh[x] = qh;
+                    }
+                }
 #pragma unroll
                 for (uint32_t x = 0; x < QE; x++) {
                     l[x] -= c0;
                     at[x] = lo_s + l[x] * static_cast<uint32_t>(sizeof(uint32_t));
-                    old[x] = shared_add_below(at[x], ql, l[x], nc);
+                    old[x] = shared_add_below(at[x], vl[x], l[x], nc);
                 }
 #pragma unroll
                 for (uint32_t x = 0; x < QE; x++)
-                    shared_carry_below(at[x] + hi_off, qh + (old[x] > ~ql ? 1u : 0u), l[x], nc);
+                    shared_carry_below(at[x] + hi_off, vh[x] + (old[x] > ~vl[x] ? 1u : 0u), l[x], nc);
             }
         }
     }
@@ -368,6 +407,215 @@ static __global__ void __launch_bounds__(256)
     }
     double unused = 0.0;
     write_lists(la, j, bits + 2 * dense_words, 2 * (n_words - dense_words), len + 64ull * dense_words, sum, unused);
+}
+
+// Node values of one sample per block of 256 threads (weighted methods), in
+// place of an embedding of every node for every sample: the sample's tips,
+// then level by level the sums of a node's children that the sample has, left
+// child first as the reference sums them (src/unifrac_internal.cpp:240-257).
+// Node columns: value-only tips (bypassed), sparse nodes, dense nodes, each
+// section from a multiple of 32 and by height, so every child's column comes
+// before its parent's.  Written: the sparse nodes' lists, the dense nodes' rows
+// of L u (U), the one-sided sums W (every embedded node) and rs (sparse nodes).
+struct WalkArgs {
+    const uint32_t *sample_ptr;  // per column j: its entries
+    const int32_t *start;        // per entry: the tip's node column
+    const double *start_val;     // and count
+    const int32_t *parent;       // per node column
+    const int2 *child;           // per node column: children, -1 none; y == -2: a list at kids + x (count, columns)
+    const int32_t *kids;
+    const uint32_t *level;       // node columns where a level of internal nodes starts; n_levels pairs (start, end)
+    uint32_t n_levels;
+    const double *len;           // per node column
+    const double *totals;        // per column j
+    int normalize;
+    uint32_t n_words;            // 32-bit words of the bitmap
+    uint32_t sparse0, dense0, n_dense;  // section starts
+    double scale;                // 2^s
+    uint32_t cap;                // nodes held in shared memory
+    double *spill;               // values (and ids) of samples with more
+    uint32_t *spill_id;
+    unsigned long long *spill_cursor;
+    uint64_t ld;
+};
+
+constexpr int WALK_BLOCKS = 6;  // blocks an SM: the walk waits on loads and barriers, so samples in flight set its pace
+
+template <typename T>
+__global__ void __launch_bounds__(256, WALK_BLOCKS)
+    weighted_walk_kernel(const WalkArgs a, T *__restrict__ U, T *__restrict__ W, const uint32_t *__restrict__ column,
+                         const ListArgs la) {
+    extern __shared__ double walk_s[];
+    double *vals = walk_s;                                         // [cap]
+    uint32_t *ids = reinterpret_cast<uint32_t *>(vals + a.cap);    // [cap]
+    uint32_t *bits = ids + a.cap;                                  // [n_words]
+    uint32_t *pre = bits + a.n_words;                              // [n_words + 1] nodes before each word
+    uint32_t *level_s = pre + a.n_words + 1;                       // [2 n_levels + 4] ranks where levels start and end
+    __shared__ uint32_t warp_tot[8];
+    __shared__ double warp_w[8];
+    __shared__ unsigned long long warp_q[8];
+    __shared__ unsigned long long first[2];
+    const uint32_t j = column[blockIdx.x], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (uint32_t w = tid; w < a.n_words; w += 256) bits[w] = 0u;
+    __syncthreads();
+    const uint32_t e0 = a.sample_ptr[j], n_e = a.sample_ptr[j + 1] - e0;
+    // (the thread's first tip, for the values below)
+    const int32_t tip = tid < n_e ? a.start[e0 + tid] : 0;
+    const double count = tid < n_e ? a.start_val[e0 + tid] : 0.0, total_count = a.totals[j];
+    mark_paths(a.start + e0, n_e, a.parent, bits);
+    __syncthreads();
+    // ranks
+    const uint32_t per = (a.n_words + 255) / 256;
+    const uint32_t w0 = min(a.n_words, tid * per), w1 = min(a.n_words, w0 + per);
+    uint32_t c = 0;
+    for (uint32_t w = w0; w < w1; w++) c += __popc(bits[w]);
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= static_cast<uint32_t>(o)) incl += y;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; w++) {
+        if (w < warp) before += warp_tot[w];
+        total += warp_tot[w];
+    }
+    before += incl - c;
+    if (total > a.cap) {  // uniform over the block
+        if (tid == 0) first[0] = atomicAdd(a.spill_cursor, static_cast<unsigned long long>(total));
+        __syncthreads();
+        vals = a.spill + first[0];
+        ids = a.spill_id + first[0];
+    }
+    {
+        uint32_t at = before;
+        for (uint32_t w = w0; w < w1; w++) {
+            pre[w] = at;
+            uint32_t m = bits[w];
+            while (m) {
+                ids[at++] = w * 32 + __ffs(m) - 1;
+                m &= m - 1;
+            }
+        }
+        if (tid == 255) pre[a.n_words] = total;
+    }
+    __syncthreads();
+    auto rank = [&](uint32_t col) { return pre[col >> 5] + __popc(bits[col >> 5] & ((1u << (col & 31)) - 1u)); };
+    auto value = [&](int32_t col) {
+        return (bits[col >> 5] >> (col & 31)) & 1u ? vals[rank(static_cast<uint32_t>(col))] : 0.0;
+    };
+    for (uint32_t i = tid; i < 2 * a.n_levels + 4; i += 256) level_s[i] = i < 2 * a.n_levels ? rank(a.level[i]) : total;
+    for (uint32_t e = tid; e < n_e; e += 256) {
+        const double v = e == tid ? count : a.start_val[e0 + e];
+        vals[rank(static_cast<uint32_t>(e == tid ? tip : a.start[e0 + e]))] = a.normalize ? v / total_count : v;
+    }
+    __syncthreads();
+    // (a thread's first nodes of the next two levels have their children on
+    // their way while the current level is summed)
+    auto children = [&](uint32_t lv) {
+        const uint32_t r = level_s[2 * lv] + tid;
+        return r < level_s[2 * lv + 1] ? a.child[ids[r]] : make_int2(-1, -1);
+    };
+    int2 ch = children(0), next = children(1);
+    for (uint32_t lv = 0; lv < a.n_levels; lv++) {
+        const int2 after = lv + 2 < a.n_levels ? children(lv + 2) : make_int2(-1, -1);
+        const uint32_t r0 = level_s[2 * lv], r1 = level_s[2 * lv + 1];
+        if (r0 != r1) {  // uniform over the block
+            for (uint32_t r = r0 + tid; r < r1; r += 256) {
+                if (r >= r0 + 256) ch = a.child[ids[r]];
+                double s = 0.0;
+                if (ch.y != -2) {
+                    if (ch.x >= 0) s += value(ch.x);
+                    if (ch.y >= 0) s += value(ch.y);
+                } else {
+                    const int32_t *k = a.kids + ch.x;
+                    for (int32_t q = 1; q <= k[0]; q++) s += value(k[q]);
+                }
+                vals[r] = s;
+            }
+            __syncthreads();
+        }
+        ch = next;
+        next = after;
+    }
+    const uint32_t rs0 = rank(a.sparse0), rd0 = rank(a.dense0);
+    const uint32_t n_sp = rd0 - rs0;
+    if (tid == 0) {
+        first[1] = total > rs0 ? atomicAdd(la.cursor, static_cast<unsigned long long>(total - rs0)) : 0ull;
+        la.node_ptr[j] = first[1];
+        la.node_cnt[j] = n_sp;
+        la.node_all[j] = total - rs0;
+    }
+    __syncthreads();
+    // dense rows
+    double wsum = 0.0;
+    for (uint32_t r = rd0 + tid; r < total; r += 256) {
+        const uint32_t c = ids[r];
+        const double u = vals[r], lu = a.len[c] * u;
+        wsum += lu;
+        U[static_cast<uint64_t>(c - a.dense0) * a.ld + j] = static_cast<T>(lu);
+        la.node[first[1] + r - rs0] = c - a.sparse0;
+        la.node_u[first[1] + r - rs0] = u;
+    }
+    // lists
+    const uint32_t t = la.block_table[j >> 7];
+    const uint32_t pos = j - la.tables[t].base;
+    const uint64_t slot0 = static_cast<uint64_t>(t - la.t0) * la.n_nodes;
+    unsigned long long qsum = 0;
+    constexpr int UN = 4;  // entries of a thread in flight
+    for (uint32_t i0 = tid; i0 < n_sp; i0 += UN * 256) {
+        uint32_t e[UN], at[UN], off[UN];
+        double v[UN], lu[UN];
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            const uint32_t i = i0 + u * 256;
+            const bool on = i < n_sp;
+            e[u] = on ? ids[rs0 + i] - a.sparse0 : 0xFFFFFFFFu;
+            at[u] = on ? atomicAdd(la.count + slot0 + e[u], 1u) : 0u;
+            off[u] = on ? la.off[slot0 + e[u]] : 0u;
+            v[u] = on ? vals[rs0 + i] : 0.0;
+            lu[u] = on ? a.len[a.sparse0 + e[u]] * v[u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            if (e[u] == 0xFFFFFFFFu) continue;
+            wsum += lu[u];
+            const unsigned long long q = static_cast<unsigned long long>(__double2ll_rn(lu[u] * a.scale));
+            qsum += q;
+            const uint64_t to = static_cast<uint64_t>(off[u]) * LIST_ALIGN + at[u];
+            if (la.wide)
+                static_cast<uint32_t *>(la.idx)[to] = pos;
+            else
+                static_cast<uint16_t *>(la.idx)[to] = static_cast<uint16_t>(pos);
+            la.idx_q[to] = q;
+            la.node[first[1] + i0 + u * 256] = e[u];
+            la.node_q[first[1] + i0 + u * 256] = q;
+            la.node_u[first[1] + i0 + u * 256] = v[u];
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+        qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
+    }
+    if (lane == 0) {
+        warp_w[warp] = wsum;
+        warp_q[warp] = qsum;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double w = 0.0;
+        unsigned long long q = 0;
+        for (int i = 0; i < 8; i++) {
+            w += warp_w[i];
+            q += warp_q[i];
+        }
+        if (W) W[j] = static_cast<T>(w);
+        la.rs[j] = q;
+    }
 }
 
 }  // namespace dev
