@@ -189,21 +189,9 @@ ComputeStatus validate(const ssu::Table &table, const ssu::BPTree &tree) {
     return m.rows_matched == table.distinct_names ? okay : table_and_tree_do_not_overlap;
 }
 
-// SYNC_TREE_TABLE (src/api.cpp:90-92) + flattening for the device.  The kept
-// tips carry their table rows; when every tip is in the table the shear is
-// the tree itself, and a tree without single-child nodes collapses to itself.
+// SYNC_TREE_TABLE (src/api.cpp:90-92), flattened for the device.
 ssu::FlatTree sync_tree(const ssu::Table &table, const ssu::BPTree &tree, bool bypass_tips) {
-    const ssu::TipMatch &m = tip_match(table, tree);
-    bool single = false;
-    if (m.all_tips) {
-        ssu::FlatTree f = ssu::flatten(tree, bypass_tips, &m.tags, &single);
-        if (!single) return f;
-        return ssu::flatten(tree.collapse(&m.tags), bypass_tips);
-    }
-    const ssu::BPTree sheared = tree.shear_matched(m);
-    ssu::FlatTree f = ssu::flatten(sheared, bypass_tips, nullptr, &single);
-    if (!single) return f;
-    return ssu::flatten(sheared.collapse(), bypass_tips);
+    return ssu::flatten(tree, tip_match(table, tree).tags, bypass_tips);
 }
 
 // UNIFRAC_B200_UNWEIGHTED_MODE: "gemm" runs unweighted methods on the
@@ -555,15 +543,13 @@ ComputeStatus batch_prepare(const std::vector<const ssu::Table *> &tables, const
     // VALIDATE_TREE_TABLE (src/api.cpp:94-100) for every table: each of its
     // observations names a tip
     std::vector<uint8_t> in_tree(n_union, 0);
-    for (uint32_t i = 0; i + 1 < tree.size(); i++) {
-        if (!tree.leaf(i)) continue;
-        const int64_t u = uni.find(tree.name[i]);
+    const ssu::TipMatch match = tree.match_tips(uni, n_union);
+    for (int32_t u : match.tags)
         if (u >= 0) in_tree[u] = 1;
-    }
     for (size_t t = 0; t < tables.size(); t++)
         for (uint32_t u : uid[t])
             if (!in_tree[u]) return table_and_tree_do_not_overlap;
-    bh.flat = ssu::flatten(tree.shear_to(uni, n_union, nullptr).collapse(), bypass);
+    bh.flat = ssu::flatten(tree, match.tags, bypass);
     bh.set.tables = tables;
     bh.set.obs_row.assign(tables.size(), std::vector<int32_t>(n_union, -1));
     bh.set.embedded.resize(tables.size());

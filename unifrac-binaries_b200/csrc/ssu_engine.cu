@@ -412,8 +412,7 @@ struct SparseNodes {
     std::vector<std::vector<uint32_t>> entries;
     double scale = 1.0;              // 2^s, exact sums below 2^62
 };
-SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const std::vector<int32_t> &parent,
-                              const ListRule &rule, const std::vector<uint32_t> *height = nullptr);
+SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule, bool by_height = false);
 
 // Host-built layout of the weighted walk (see build_walk_layout).
 struct WalkLayout {
@@ -1732,25 +1731,16 @@ int PlanImpl::tune_band() {
 }
 
 // Row of every row's parent, or -1 under the root.
-std::vector<int32_t> parent_rows(const FlatTree &tree) {
-    std::vector<int32_t> parent(tree.n_nodes, -1);
-    for (uint32_t r = 0; r < tree.n_nodes; r++)
-        for (uint32_t c = tree.child_ptr[r]; c < tree.child_ptr[r + 1]; c++)
-            parent[tree.child_rows[c]] = static_cast<int32_t>(r);
-    return parent;
-}
-
 // Starting column of each tree observation: its tip's, or the tip's parent's
 // when tips are bypassed; -1 where neither is embedded.
-std::vector<int32_t> path_starts(const FlatTree &tree, const std::vector<int32_t> &parent_row,
-                                 const std::vector<int32_t> &col_of_row) {
+std::vector<int32_t> path_starts(const FlatTree &tree, const std::vector<int32_t> &col_of_row) {
     uint32_t n_obs = 0;
     for (uint32_t r : tree.leaf_rows) n_obs = std::max<uint32_t>(n_obs, tree.leaf_obs[r] + 1);
     std::vector<int32_t> start(n_obs, -1);
     for (uint32_t r : tree.leaf_rows) {
         const int32_t obs = tree.leaf_obs[r];
         if (obs < 0) continue;
-        const int32_t node = r < tree.n_embedded ? static_cast<int32_t>(r) : parent_row[r];
+        const int32_t node = r < tree.n_embedded ? static_cast<int32_t>(r) : tree.parent[r];
         start[obs] = (node >= 0 && static_cast<uint32_t>(node) < tree.n_embedded) ? col_of_row[node] : -1;
     }
     return start;
@@ -1771,9 +1761,9 @@ void add_entry_counts(const TableSet &set, const FlatTree &tree, size_t t, std::
 
 // Every internal row's count becomes the sum over its tips (tip rows hold
 // theirs): bypassed tips lie behind the embedded rows, which are in postorder.
-void sum_over_clades(const FlatTree &tree, const std::vector<int32_t> &parent, std::vector<uint32_t> &counts) {
+void sum_over_clades(const FlatTree &tree, std::vector<uint32_t> &counts) {
     auto up = [&](uint32_t r) {
-        const int32_t p = parent[r];
+        const int32_t p = tree.parent[r];
         if (p < 0) return;
         const uint64_t sum = static_cast<uint64_t>(counts[p]) + counts[r];
         counts[p] = static_cast<uint32_t>(std::min<uint64_t>(sum, UINT32_MAX));  // (repeated tip names)
@@ -1787,8 +1777,7 @@ void sum_over_clades(const FlatTree &tree, const std::vector<int32_t> &parent, s
 // counts twice), so the choice needs the tables' offsets alone.  A row whose
 // length is below 2^(min_bits - 1) units of the fixed point stays out (its
 // rounding would be coarser than the dense form's).
-SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const std::vector<int32_t> &parent,
-                              const ListRule &rule, const std::vector<uint32_t> *height) {
+SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const ListRule &rule, bool by_height) {
     SparseNodes sp;
     const uint32_t E = tree.n_embedded;
     sp.id_of_row.assign(E, -1);
@@ -1804,7 +1793,7 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const s
         samples += set.tables[t]->n_samples;
         counts[t].assign(tree.n_nodes, 0);
         add_entry_counts(set, tree, t, counts[t]);
-        sum_over_clades(tree, parent, counts[t]);
+        sum_over_clades(tree, counts[t]);
     }
     if (n_tables > 1) {
         sum.assign(E, 0);
@@ -1845,13 +1834,13 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const s
     for (uint64_t i = 1; i < at.size(); i++) at[i] += at[i - 1];
     sp.row.resize(rows.size());
     for (uint32_t e : rows) sp.row[at[samples - bound(e)]++] = e;
-    if (height) {
+    if (by_height) {
         uint32_t top = 0;
-        for (uint32_t e : rows) top = std::max(top, (*height)[e]);
+        for (uint32_t e : rows) top = std::max(top, tree.height[e]);
         at.assign(top + 2, 0);
-        for (uint32_t e : rows) at[(*height)[e] + 1]++;
+        for (uint32_t e : rows) at[tree.height[e] + 1]++;
         for (uint32_t i = 1; i < at.size(); i++) at[i] += at[i - 1];
-        for (uint32_t e : sp.row) rows[at[(*height)[e]]++] = e;
+        for (uint32_t e : sp.row) rows[at[tree.height[e]]++] = e;
         sp.row.swap(rows);
     }
     for (size_t i = 0; i < sp.row.size(); i++) sp.id_of_row[sp.row[i]] = static_cast<int32_t>(i);
@@ -1869,17 +1858,9 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const s
 WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule, bool fp64) {
     WalkLayout lay;
     const uint32_t E = tree.n_embedded, K = tree.n_nodes;
-    const std::vector<int32_t> parent_row = parent_rows(tree);
-    std::vector<uint32_t> height(K, 0);
-    uint32_t top = 0;
-    auto lift = [&](uint32_t r) {
-        const int32_t p = parent_row[r];
-        if (p >= 0) height[p] = std::max(height[p], height[r] + 1);
-        top = std::max(top, height[r]);
-    };
-    for (uint32_t r = E; r < K; r++) lift(r);
-    for (uint32_t r = 0; r < E; r++) lift(r);
-    lay.sparse = find_sparse_nodes(set, tree, parent_row, rule, &height);
+    const std::vector<uint32_t> &height = tree.height;
+    const uint32_t top = tree.level_ptr.empty() ? 0 : static_cast<uint32_t>(tree.level_ptr.size()) - 1;
+    lay.sparse = find_sparse_nodes(set, tree, rule, true);
     const SparseNodes &sp = lay.sparse;
     std::vector<uint32_t> dense(E - sp.row.size()), at(top + 2, 0);
     for (uint32_t e = 0; e < E; e++)
@@ -1913,7 +1894,7 @@ WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const Li
     lay.len.assign(lay.n_cols, 0.0);
     std::vector<double> path(K);
     auto down = [&](uint32_t r) {  // parents before children
-        const int32_t p = parent_row[r];
+        const int32_t p = tree.parent[r];
         const uint32_t c = static_cast<uint32_t>(col[r]);
         if (p >= 0) lay.parent[c] = col[p];
         if (r < E) lay.len[c] = fp64 ? tree.length[r] : static_cast<double>(static_cast<float>(tree.length[r]));
@@ -1953,8 +1934,7 @@ WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const Li
 GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule) {
     GemmLayout lay;
     const uint32_t E = tree.n_embedded;
-    const std::vector<int32_t> parent_row = parent_rows(tree);
-    lay.sparse = find_sparse_nodes(set, tree, parent_row, rule);
+    lay.sparse = find_sparse_nodes(set, tree, rule);
     const std::vector<int32_t> &sparse_of = lay.sparse.id_of_row;
     uint32_t n_dense = 0;  // contracted rows
     // order by binary exponent of |length|, largest first, by row within an
@@ -2054,10 +2034,10 @@ GemmLayout build_gemm_layout(const TableSet &set, const FlatTree &tree, const Li
     // parents among embedded nodes
     lay.parent_col.assign(lay.lsorted.size(), -1);
     for (uint32_t r = 0; r < E; r++) {
-        const int32_t p = parent_row[r];
+        const int32_t p = tree.parent[r];
         lay.parent_col[col_of_row[r]] = (p >= 0 && static_cast<uint32_t>(p) < E) ? col_of_row[p] : -1;
     }
-    lay.start_of_obs = path_starts(tree, parent_row, col_of_row);
+    lay.start_of_obs = path_starts(tree, col_of_row);
     return lay;
 }
 
@@ -2685,8 +2665,7 @@ ListRule PlanImpl::bits_list_rule(const TableSet &set) const {
 int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     SetupTimer timer;
     const ListRule rule = bits_list_rule(set);
-    const std::vector<int32_t> parent_row = parent_rows(tree);
-    const SparseNodes sp = find_sparse_nodes(set, tree, parent_row, rule);
+    const SparseNodes sp = find_sparse_nodes(set, tree, rule);
     // columns: the dense rows in order, padded to whole words, then the sparse nodes
     uint32_t n_dense = 0;
     std::vector<int32_t> col(tree.n_nodes, -1);
@@ -2700,7 +2679,7 @@ int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     std::vector<double> len(n_cols, 0.0), path(n_cols, 0.0);
     std::vector<int32_t> parent(n_cols, -1);
     for (uint32_t r = E; r-- > 0;) {  // parents follow their children
-        const int32_t p = parent_row[r];
+        const int32_t p = tree.parent[r];
         len[col[r]] = tree.length[r];
         if (p >= 0 && static_cast<uint32_t>(p) < E) parent[col[r]] = col[p];
         path[col[r]] = (parent[col[r]] >= 0 ? path[parent[col[r]]] : 0.0) + tree.length[r];
@@ -2736,7 +2715,7 @@ int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     SSU_CK(alloc(&d_flags, sizeof(int) * max_tiles));
     SSU_CK(upload(&d_parent_col, parent.data(), sizeof(int32_t) * n_cols));
     SSU_CK(upload(&d_len_cols, len.data(), sizeof(double) * n_cols));
-    if (const int rc = setup_lists(set, tree, sp, d_len_cols, n_cols, first, &path, path_starts(tree, parent_row, col)))
+    if (const int rc = setup_lists(set, tree, sp, d_len_cols, n_cols, first, &path, path_starts(tree, col)))
         return rc;
     timer.step("bits_lists");
     lut_stride = 0;
