@@ -691,3 +691,97 @@ def test_weighted_by_lists_leaves_other_inputs_to_the_embedding(ssu, monkeypatch
         got = call()
         np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
         check_fp64(np.nan_to_num(got), np.nan_to_num(ref))
+
+
+# ---- generalized by sample lists (the nodes that both samples have)
+
+def _union_dense(monkeypatch, call):
+    """`call` with the dense pair kernel over the embedding (the general path)."""
+    monkeypatch.setenv("UNIFRAC_B200_UNION_MODE", "dense")
+    try:
+        return call()
+    finally:
+        monkeypatch.delenv("UNIFRAC_B200_UNION_MODE")
+
+
+@pytest.mark.parametrize("alpha", [0.0, 0.25, 0.5, 1.0, 2.0])
+@pytest.mark.parametrize("n,n_tips,density", [(1, 40, 0.2), (2, 40, 0.2), (33, 1200, 0.01), (65, 700, 0.6), (300, 900, 0.03),
+                                              (1220, 150, 0.05)])
+def test_generalized_by_lists_matches_the_dense_form(ssu, monkeypatch, alpha, n, n_tips, density):
+    """Every alpha kind, both tile shapes, nodes by lists, by rows and by both,
+    a walk in two parts, polytomies, explicit zeros: full matrix, bypassed tips,
+    condensed, window; raw counts stay on the other kernels."""
+    rng = np.random.default_rng(n)
+    tree, table = _case(900 + n, n_tips=n_tips, n_samples=n, density=density, drop=5)
+    tree = _polytomy(tree, rng)
+    table.data[rng.random(table.data.shape[0]) < 0.1] = 0.0
+    # a table with a sample whose entries are all explicit zeros (0 / 0) stays on
+    # the embedding's union kernel: NaN, or where both samples are few items the
+    # sparse form's 1, the dense form's NaN
+    total = np.bincount(table.indices, weights=table.data, minlength=n)
+    void = (total == 0) & (np.bincount(table.indices, minlength=n) > 0)
+    k, l = np.triu_indices(n, 1)
+    stop = (n + 1) // 2
+    s = np.arange(stop // 3, max(stop, stop // 3 + 1))[:, None]
+    j = np.arange(n)[None, :]
+    m = "generalized_fp64"
+    full = void[:, None] | void[None, :]
+    calls = [(full, lambda: ssu.one_off_matrix(tree, table, m, alpha=alpha)[0]),
+             (full, lambda: ssu.one_off_matrix(tree, table, m, alpha=alpha, bypass_tips=True)[0]),
+             (full & False, lambda: ssu.one_off_matrix(tree, table, m, alpha=alpha, normalize=False)[0]),
+             (void[k] | void[l], lambda: ssu.one_off(tree, table, m, alpha=alpha)[0]),
+             (void[j + 0 * s] | void[(j + s + 1) % n], lambda: ssu.partial(tree, table, m, stop // 3, stop, alpha=alpha)[0])]
+    for skip, call in calls if n > 1 else calls[:4]:
+        got, ref = call(), _union_dense(monkeypatch, call)
+        got, ref = np.where(skip, 0.0, got), np.where(skip, 0.0, ref)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+        check_fp64(np.nan_to_num(got), np.nan_to_num(ref))
+    if void.any():
+        others = calls[0][1]()[void][:, total > 0]
+        assert np.all(np.isnan(others) | (others == 1.0))
+
+
+@pytest.mark.parametrize("alpha", [0.0, 0.25, 0.5, 2.0])
+def test_generalized_by_lists_close_pairs(ssu, oracle_mod, alpha):
+    """Near-duplicate samples (their tiles' marked pairs are summed again) meet 1e-12."""
+    tree, table = _near_duplicates(62)
+    for method in ("generalized_fp64", "generalized"):
+        gpu, _ = ssu.one_off_matrix(tree, table, method, alpha=alpha)
+        ref = oracle_mod.oracle_one_off(tree, table, "generalized_fp64", alpha=alpha)["matrix"]
+        if method.endswith("fp64"):
+            check_fp64(gpu, ref)
+        else:  # fp64 terms and sums, rounded to single precision once
+            np.testing.assert_allclose(gpu, ref, rtol=2.0 ** -23, atol=1e-30)
+
+
+def test_generalized_by_lists_with_tiny_proportions(ssu, oracle_mod):
+    """Proportions down to 1e-30: the branch-free reciprocal square root and the
+    lists' fixed point against the oracle."""
+    tree, table = _case(91, n_tips=200, n_samples=40, density=0.2)
+    rng = np.random.default_rng(4)
+    table.data = 10.0 ** rng.uniform(-30, 6, size=table.data.shape)
+    for alpha in (0.0, 0.5, 2.0):
+        gpu, _ = ssu.one_off_matrix(tree, table, "generalized_fp64", alpha=alpha)
+        check_fp64(gpu, oracle_mod.oracle_one_off(tree, table, "generalized_fp64", alpha=alpha)["matrix"])
+
+
+def test_generalized_by_lists_in_a_batch_as_a_graph(ssu, monkeypatch):
+    tree = ssu_synth.random_binary_tree(800, 0.1, 5)
+    tips = tree.tip_names()
+    tables = [ssu_synth.geometric_table(tips[3 * i:700 + 20 * i], n, 0.05, 10.0, 60 + i)
+              for i, n in enumerate((5, 64, 200, 33))]
+
+    def run(group_bytes=0):
+        plan = ssu.BatchPlan(tree, tables, "generalized_fp64", alpha=0.5, group_bytes=group_bytes, autotune=0)
+        plan.execute()
+        first = plan.results()
+        plan.set_graph(True)
+        for _ in range(2):
+            plan.execute()
+        for a, b in zip(plan.results(), first):
+            np.testing.assert_array_equal(a, b)
+        plan.close()
+        return first
+    for a, b, c in zip(run(), run(group_bytes=1), _union_dense(monkeypatch, run)):
+        check_fp64(a, c)
+        check_fp64(b, c)

@@ -17,6 +17,7 @@
 #include <thread>
 
 #include "ssu_gemm.cuh"
+#include "ssu_gen.cuh"
 #include "ssu_host.hpp"
 #include "ssu_kernels.cuh"
 #include "ssu_lists.cuh"
@@ -398,7 +399,7 @@ struct ListRule {
     double pair_s = 0.0;      // lists: per pair of a node's samples
     double entry_s = 0.0;     // and per sample of a node
     double fixed_s = 0.0;     // and once; less than this is not worth the lists
-    uint32_t min_div = 8;     // at most 1 / min_div of the samples
+    double most = 1.0;        // at most this share of the samples
     int min_bits = 0;         // bits that a length keeps in the fixed point
     bool wide = false;        // 32-bit list entries whatever the tables' sizes
 };
@@ -610,12 +611,20 @@ struct PlanImpl {
     // nodes that few samples have by sample lists, the others by the dense
     // tile kernel over their rows alone
     bool walk_weighted = false;
+    // generalized UniFrac the same way, over the nodes that both samples have
+    // (alpha 1 is weighted normalized); walk_weighted too
+    bool walk_gen = false;
+    bool gen_small = false;                 // 64 x 64 tiles
+    unsigned long long *d_gen_num = nullptr, *d_gen_den = nullptr;
+    int walk_gen_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles, uint32_t ntiles,
+                       uint32_t splits, uint32_t rows);
     dev::WalkArgs walk{};
     uint32_t n_dense_rows = 0;
     double walk_unit = 1.0;
     uint32_t *d_close = nullptr;
     size_t walk_smem = 0;
     ListRule weighted_list_rule(const TableSet &set) const;
+    void split_rows(Group &g, const PairKernel<double> &k) const;
     template <typename T>
     int setup_walk_weighted(const TableSet &set, const FlatTree &tree);
     template <typename T>
@@ -795,7 +804,7 @@ int PlanImpl::setup(const TableSet &set, const FlatTree &tree, const BatchOption
         if (std::string(m) == "dense") hybrid = false;
     // generalized and variance-adjusted methods: only the union of the two
     // samples' supports adds to a pair (needs u >= 0 so presence is u > 0)
-    union_mode = !faith && !gemm && nonneg_data && set.row_active.empty() &&
+    union_mode = !faith && !gemm && !walk_weighted && nonneg_data && set.row_active.empty() &&
                  (spec.vaw || spec.method == Method::generalized);
     if (const char *m = std::getenv("UNIFRAC_B200_UNION_MODE"))
         if (std::string(m) == "dense") union_mode = false;
@@ -1794,6 +1803,7 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
         counts[t].assign(tree.n_nodes, 0);
         add_entry_counts(set, tree, t, counts[t]);
         sum_over_clades(tree, counts[t]);
+        for (uint32_t &c : counts[t]) c = std::min(c, set.tables[t]->n_samples);  // (no list is longer)
     }
     if (n_tables > 1) {
         sum.assign(E, 0);
@@ -1805,6 +1815,7 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
             }
     }
     auto bound = [&](uint32_t e) -> uint64_t { return n_tables > 1 ? sum[e] : counts[0][e]; };
+    const uint64_t limit = static_cast<uint64_t>(rule.most * static_cast<double>(samples));
     std::vector<uint32_t> rows;
     rows.reserve(E);
     double total = 0.0, gain = -rule.fixed_s;
@@ -1812,7 +1823,7 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
         const uint64_t m = bound(e);
         const double x = static_cast<double>(m);
         const double by_lists = 0.5 * (n_tables > 1 ? square[e] : x * x) * rule.pair_s + x * rule.entry_s;
-        if (m * rule.min_div > samples || by_lists >= rule.dense_s) continue;
+        if (m > limit || by_lists >= rule.dense_s) continue;
         rows.push_back(e);
         gain += rule.dense_s - by_lists;
         total += tree.length[e];
@@ -1829,11 +1840,11 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
     // numbered by decreasing length of their lists (within a height, where the
     // walk needs children first), by counting sorts: a sample's nodes then come
     // in that order, and the lists that lanes read side by side end together
-    std::vector<uint32_t> at(samples + 2, 0);
-    for (uint32_t e : rows) at[samples - bound(e) + 1]++;
+    std::vector<uint32_t> at(limit + 2, 0);
+    for (uint32_t e : rows) at[limit - bound(e) + 1]++;
     for (uint64_t i = 1; i < at.size(); i++) at[i] += at[i - 1];
     sp.row.resize(rows.size());
-    for (uint32_t e : rows) sp.row[at[samples - bound(e)]++] = e;
+    for (uint32_t e : rows) sp.row[at[limit - bound(e)]++] = e;
     if (by_height) {
         uint32_t top = 0;
         for (uint32_t e : rows) top = std::max(top, tree.height[e]);
@@ -1847,7 +1858,7 @@ SparseNodes find_sparse_nodes(const TableSet &set, const FlatTree &tree, const L
     for (size_t t = 0; t < n_tables; t++) {
         sp.entries[t].resize(sp.row.size());
         for (size_t i = 0; i < sp.row.size(); i++)
-            sp.entries[t][i] = std::min(counts[t][sp.row[i]], set.tables[t]->n_samples);
+            sp.entries[t][i] = counts[t][sp.row[i]];
     }
     return sp;
 }
@@ -2118,6 +2129,7 @@ ListRule PlanImpl::tc_list_rule(const TableSet &set, uint32_t n_rows) const {
     r.pair_s = 1e-12;
     r.entry_s = 6e-11;
     r.fixed_s = 20e-6;
+    r.most = 0.125;
     r.min_bits = tc::QBITS;  // as many as the contraction's digits hold
     if (mode >= 1) {
         r.dense_s = 1.0;
@@ -2296,7 +2308,8 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
             std::max<uint64_t>(1, std::min<uint64_t>(dev::LIST_PARTS, g.ld / ((walk_weighted ? 4 : 8) * static_cast<uint64_t>(n_sms)))));
         uint32_t n_max = 1;
         for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);
-        while (dev::list_part_rows(n_max, la.parts) > kSharedCols) la.parts *= 2;  // (a part's columns fit a block)
+        const uint32_t most = walk_gen ? dev::kGenCols : kSharedCols;
+        while (dev::list_part_rows(n_max, la.parts) > most) la.parts *= 2;  // (a part's columns fit a block)
         std::vector<std::vector<uint32_t>> by_part(la.parts);
         for (uint32_t t = g.t0; t < g.t1; t++) {
             const uint32_t n_t = tdesc[t].n, rows = dev::list_part_rows(std::max(n_t, 1u), la.parts);
@@ -2324,6 +2337,11 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
         SSU_CK(alloc(&la.node, sizeof(uint32_t) * std::max<uint64_t>(ids, 1)));
         if (walk_weighted) {
             SSU_CK(alloc(&la.node_all, sizeof(uint32_t) * g.ld));
+            if (walk_gen) {
+                SSU_CK(alloc(&la.idx_u, sizeof(double) * std::max<uint64_t>(at, 1) * dev::LIST_ALIGN));
+                // (read, not used, past each list's end)
+                SSU_CK(cudaMemsetAsync(la.idx_u, 0, sizeof(double) * std::max<uint64_t>(at, 1) * dev::LIST_ALIGN, stream));
+            }
             SSU_CK(alloc(&la.idx_q, sizeof(unsigned long long) * std::max<uint64_t>(at, 1) * dev::LIST_ALIGN));
             SSU_CK(alloc(&la.node_q, sizeof(unsigned long long) * std::max<uint64_t>(ids, 1)));
             SSU_CK(alloc(&la.node_u, sizeof(double) * std::max<uint64_t>(ids, 1)));
@@ -2441,9 +2459,37 @@ ListRule PlanImpl::weighted_list_rule(const TableSet &set) const {
     for (const Table *t : set.tables) pairs += 0.5 * t->n_samples * static_cast<double>(t->n_samples);
     r.dense_s = std::max(pairs * (spec.fp64 ? 1.3e-13 : 9e-14), 1e-8);
     r.pair_s = 1.2e-12;
+    if (walk_gen) {
+        // terms of about 25 fp64 instructions in both forms, the lists' with
+        // four atomics (dense costs of 0.3, 0.6, 1.0, 1.5, 2.5 ps, eight uneven
+        // tables on 50,000 tips: 5.97, 5.18, 4.86, 4.74, 4.77 ms); a general
+        // alpha's pow costs eight times as much, and takes the dense kernel's
+        // few blocks of a small table far longer (128 samples: 786 us with the
+        // 20 ns floor of the others, 160 us so)
+        const bool pow = alpha_kind(spec.alpha) == 0;
+        r.dense_s = std::max(pairs * (pow ? 1.2e-11 : 1.5e-12), pow ? 4e-6 : 2e-8);
+        r.pair_s = pow ? 1.2e-11 : 4e-12;
+    }
     r.entry_s = 1e-10;
-    r.min_div = 1;
     return r;
+}
+
+// Row splits of the generalized dense kernel: waves of its blocks over the
+// dense rows, no fewer than 64 rows a split.
+void PlanImpl::split_rows(Group &g, const PairKernel<double> &k) const {
+    const uint32_t q = static_cast<uint32_t>(k.row_quantum), slots = static_cast<uint32_t>(n_sms * k.blocks_per_sm);
+    double best = 1e300;
+    const uint32_t max_s = std::max<uint32_t>(1, std::min<uint32_t>(64, n_dense_rows / 64));
+    for (uint32_t s = 1; s <= max_s; s++) {
+        const double cost = std::ceil(static_cast<double>(g.n_tiles) * s / slots) / s * (1.0 + 0.01 * (s - 1));
+        if (cost < best - 1e-12) {
+            best = cost;
+            g.splits = s;
+        }
+    }
+    g.rows_per_split = ((n_dense_rows + g.splits - 1) / g.splits + q - 1) / q * q;
+    g.splits = g.rows_per_split ? (n_dense_rows + g.rows_per_split - 1) / g.rows_per_split : 1;
+    if (g.splits == 0) g.splits = 1;
 }
 
 template <typename T>
@@ -2458,9 +2504,14 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     if (!spec.normalize)
         for (const Group &g : groups)
             for (double t : g.totals) vmax = std::max(vmax, t);
+    double bound = lay.path_max * vmax;
+    if (walk_gen) {  // u^alpha <= 1 for proportions: at most every length
+        bound = 0.0;
+        for (double L : lay.len) bound += L;
+    }
     int x = 0;
-    std::frexp(std::max(lay.path_max * vmax * (1.0 + 1e-9), 1e-290), &x);
-    const double scale = std::ldexp(1.0, std::min(62 - x, 1000));
+    std::frexp(std::max(2.0 * bound * (1.0 + 1e-9), 1e-290), &x);  // (r_k + r_l stays below 2^63)
+    const double scale = std::ldexp(1.0, std::min(63 - x, 1000));
     walk_unit = 1.0 / scale;
     n_dense_rows = lay.n_dense;
     timer.step("walk_layout");
@@ -2468,16 +2519,40 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     PairKernel<T> &k = kern<T>();
     k = PairKernel<T>();
     k.BM = k.BN = dev::RB;
-    k.name = spec.method == Method::weighted_normalized ? "pair_hybrid<weighted_normalized>" : "pair_hybrid<weighted_unnormalized>";
+    k.name = spec.method == Method::generalized           ? "pair_union_lists<generalized>"
+             : spec.method == Method::weighted_normalized ? "pair_hybrid<weighted_normalized>"
+                                                          : "pair_hybrid<weighted_unnormalized>";
     k.shape = "128x128/4x8";
+    if (walk_gen) {
+        uint64_t big = 0;  // 128 x 64 tiles
+        for (const dev::TableDesc &d : tdesc) big += static_cast<uint64_t>((d.n + 127) / 128) * ((d.n + 127) / 128 + 1);
+        gen_small = big < 2ull * static_cast<uint64_t>(n_sms);
+        PairKernel<double> c = dev::gen_rows_candidates(alpha_kind(spec.alpha))[gen_small ? 1 : 0];
+        int bps = 0;
+        if (c.configure(c.smem) != cudaSuccess || c.occupancy(&bps, c.threads, c.smem) != cudaSuccess || bps < 1) {
+            last_error = "pair kernel does not fit on the device";
+            return kOutputError;
+        }
+        c.blocks_per_sm = bps;
+        kd = c;
+        k.BM = kf.BM = c.BM;
+        k.BN = kf.BN = c.BN;
+        kf.name = c.name;
+        kf.shape = kd.shape;
+    }
     uint32_t max_tiles = 1;
     hpartial_bytes = 0;
     for (Group &g : groups) {
         std::vector<uint4> tiles;
-        for (uint32_t t = g.t0; t < g.t1; t++) append_tiles(tiles, t, tdesc[t].base, tdesc[t].n, dev::RB, dev::RB, false, 0, 0);
+        for (uint32_t t = g.t0; t < g.t1; t++) append_tiles(tiles, t, tdesc[t].base, tdesc[t].n, k.BM, k.BN, false, 0, 0);
         g.n_tiles = static_cast<uint32_t>(tiles.size());
         max_tiles = std::max(max_tiles, g.n_tiles);
         SSU_CK(upload(&g.d_tiles, tiles.data(), sizeof(uint4) * tiles.size()));
+        if (walk_gen) {  // the dense kernel always leaves its sums in memory
+            split_rows(g, kd);
+            partial_bytes = std::max(partial_bytes, sizeof(double) * kd.partial_per_tile * g.n_tiles * g.splits);
+            continue;
+        }
         // Row splits so the tiles fill the SMs (one CTA per SM), in us: a row
         // of a tile takes 0.27 (fp64) or 0.16, its end 12; a split tile's sums
         // are written and read again, 4 each way, by a launch of its own.
@@ -2504,6 +2579,11 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     SSU_CK(upload(&d_par, lay.parent.data(), sizeof(int32_t) * n_cols));
     SSU_CK(upload(&d_child, lay.child.data(), sizeof(int2) * n_cols));
     SSU_CK(upload(&d_kids, lay.kids.data(), sizeof(int32_t) * lay.kids.size()));
+    if (walk_gen) {
+        SSU_CK(upload(reinterpret_cast<double **>(&d_len), lay.len.data() + lay.dense0,
+                      sizeof(double) * (lay.n_cols - lay.dense0)));
+        SSU_CK(dev::gen_configure());
+    }
     SSU_CK(upload(&d_level, lay.level.data(), sizeof(uint32_t) * lay.level.size()));
     if (const int rc = setup_lists(set, tree, sp, nullptr, 1, 0, nullptr, lay.start_of_obs)) return rc;
     walk.parent = d_par;
@@ -2518,13 +2598,16 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     walk.dense0 = lay.dense0;
     walk.n_dense = n_dense_rows;
     walk.scale = scale;
+    walk.gen = walk_gen ? 1 : 0;
+    walk.alpha = spec.alpha;
     // values in shared memory for samples of up to `cap` nodes (WALK_BLOCKS an
-    // SM), else in memory; no more than every column
-    const size_t fixed = sizeof(uint32_t) * (2ull * walk.n_words + 1 + 2ull * walk.n_levels + 4);
+    // SM), else in memory (eight tables on 50,000 tips, 4,500 nodes a sample: the
+    // walk takes the same with fewer blocks and all of them in shared memory)
+    const size_t fixed = sizeof(uint32_t) * (2ull * walk.n_words + 1 + 2ull * walk.n_levels + 4) + 8;
     constexpr size_t block = 227 * 1024 / dev::WALK_BLOCKS - 1536;  // (1 KB of it the system's)
     const size_t room = fixed + 8 * 1024 < block ? block - fixed : 8 * 1024;
     walk.cap = std::min<uint32_t>(n_cols, static_cast<uint32_t>(room / 12));
-    walk_smem = static_cast<size_t>(walk.cap) * 12 + fixed + 8;
+    walk_smem = static_cast<size_t>(walk.cap) * 12 + fixed;
     uint64_t spill = 0;  // nodes of all samples of a group, at most
     for (const Group &g : groups) {
         uint64_t m = 0;
@@ -2538,23 +2621,31 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     SSU_CK(alloc(&walk.spill, sizeof(double) * spill));
     SSU_CK(alloc(&walk.spill_id, sizeof(uint32_t) * spill));
     SSU_CK(alloc(&walk.spill_cursor, sizeof(unsigned long long)));
-    SSU_CK(alloc(&d_U, sizeof(T) * ld * std::max(n_dense_rows, 1u)));
-    SSU_CK(cudaMemsetAsync(d_U, 0, sizeof(T) * ld * std::max(n_dense_rows, 1u), stream));
-    SSU_CK(alloc(&d_W, sizeof(T) * ld));
+    const size_t el = walk_gen ? sizeof(double) : sizeof(T);  // generalized rows and sums are fp64 in both precisions
+    SSU_CK(alloc(&d_U, el * ld * std::max(n_dense_rows, 1u)));
+    SSU_CK(cudaMemsetAsync(d_U, 0, el * ld * std::max(n_dense_rows, 1u), stream));
+    SSU_CK(alloc(&d_W, el * ld));
     SSU_CK(alloc(&d_full, sizeof(T) * std::max<uint64_t>(full_elems, 1)));
     if (sizeof(T) == sizeof(double))
         d_Sq = static_cast<unsigned long long *>(d_full);  // written only after its sum is read
     else
         SSU_CK(alloc(&d_Sq, sizeof(unsigned long long) * std::max<uint64_t>(full_elems, 1)));
+    if (walk_gen) {
+        d_gen_num = d_Sq;
+        SSU_CK(alloc(&d_gen_den, sizeof(unsigned long long) * std::max<uint64_t>(full_elems, 1)));
+        SSU_CK(alloc(&d_partial, std::max<size_t>(partial_bytes, 256)));
+    }
     SSU_CK(alloc(&d_flags, sizeof(int) * max_tiles));
-    SSU_CK(alloc(&d_close, sizeof(uint32_t) * (dev::RB * dev::RB / 32) * max_tiles));
+    SSU_CK(alloc(&d_close, sizeof(uint32_t) * (static_cast<size_t>(k.BM) * k.BN / 32) * max_tiles));
     if (hpartial_bytes) SSU_CK(alloc(&d_hpartial, hpartial_bytes));
     for (auto kernel : {dev::pair_rows_kernel<T, true>, dev::pair_rows_kernel<T, false>,
                         dev::rows_finalize_kernel<T, true>, dev::rows_finalize_kernel<T, false>})
         SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(dev::rows_smem<T>())));
-    SSU_CK(cudaFuncSetAttribute(dev::weighted_walk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(tc::MAX_BITMAP_BYTES)));
+    for (const void *kernel : {reinterpret_cast<const void *>(dev::weighted_walk_kernel<T>),
+                               reinterpret_cast<const void *>(dev::weighted_walk_kernel<double>)})
+        SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(tc::MAX_BITMAP_BYTES)));
     tuning = "sample lists";
     timer.step("walk_buffers");
     return 0;
@@ -2575,20 +2666,26 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
     w.ld = g.ld;
     SSU_CK(cudaMemsetAsync(walk.spill_cursor, 0, sizeof(unsigned long long), s));
     if (groups.size() > 1)  // (the entries of one group are the same in every pass)
-        SSU_CK(cudaMemsetAsync(d_U, 0, sizeof(T) * g.ld * std::max(n_dense_rows, 1u), s));
+        SSU_CK(cudaMemsetAsync(d_U, 0, (walk_gen ? sizeof(double) : sizeof(T)) * g.ld * std::max(n_dense_rows, 1u), s));
     for (uint32_t p = 0; p < la.parts; p++) {
         if (p)
             SSU_CK(cudaMemcpyAsync(la.part_count + (p - 1) * la.slots, la.count, sizeof(uint32_t) * la.slots,
                                    cudaMemcpyDeviceToDevice, s));
         const uint32_t c0 = g.part_col[p], c1 = g.part_col[p + 1];
         if (c1 <= c0) continue;
-        dev::weighted_walk_kernel<T><<<c1 - c0, 256, walk_smem, s>>>(w, static_cast<T *>(d_U), static_cast<T *>(d_W),
-                                                                    g.d_columns + c0, la);
+        if (walk_gen)
+            dev::weighted_walk_kernel<double><<<c1 - c0, 256, walk_smem, s>>>(
+                w, static_cast<double *>(d_U), static_cast<double *>(d_W), g.d_columns + c0, la);
+        else
+            dev::weighted_walk_kernel<T><<<c1 - c0, 256, walk_smem, s>>>(w, static_cast<T *>(d_U),
+                                                                        static_cast<T *>(d_W), g.d_columns + c0, la);
         launches++;
     }
     SSU_CK(cudaGetLastError());
     if (first && timed()) SSU_CK(cudaEventRecord(ev[1], s));
-    if (ntiles) {
+    if (ntiles && walk_gen) {
+        if (const int rc = walk_gen_stage(s, g, out, tiles, ntiles, g.splits, g.rows_per_split)) return rc;
+    } else if (ntiles) {
         dev::SharedOut so;
         so.S = d_Sq;
         if (n_sparse) {
@@ -2616,7 +2713,7 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
         h.close = d_close;
         h.partial = h.n_splits > 1 ? d_hpartial : nullptr;
         h.out = out;
-        const bool norm = spec.method == Method::weighted_normalized;
+        const bool norm = spec.method != Method::weighted_unnormalized;
         const uint32_t ctas = static_cast<uint32_t>(
             std::min<uint64_t>(static_cast<uint64_t>(ntiles) * h.n_splits, static_cast<uint64_t>(n_sms)));
         constexpr size_t smem = dev::rows_smem<T>();
@@ -2639,6 +2736,62 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
     return 0;
 }
 
+// The generalized pair stage after the walk: the brackets of the list nodes,
+// the dense kernel's sums, the distances, the close pairs.
+int PlanImpl::walk_gen_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
+                             uint32_t ntiles, uint32_t splits, uint32_t rows) {
+    const dev::ListArgs &la = g.lists;
+    const dev::GenLaunch gl{alpha_kind(spec.alpha), spec.alpha, walk.scale, walk.len + walk.sparse0};
+    if (n_sparse) {
+        uint32_t n_max = 1;
+        for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);
+        const uint32_t part_rows = dev::list_part_rows(n_max, la.parts);
+        const uint32_t chunk = std::max(1u, dev::kGenCols / part_rows);  // parts per chunk
+        const uint32_t chunks = (la.parts + chunk - 1) / chunk;
+        const uint32_t cols = std::min<uint32_t>(n_max, std::min(dev::kGenCols, chunk * part_rows));
+        SSU_CK(dev::gen_sums_launch(gl, la, dev::GenSums{d_gen_num, d_gen_den}, static_cast<uint32_t>(g.ld), cols,
+                                    chunk, chunks, s));
+        launches++;
+    }
+    dev::PairArgs<double> a{};
+    a.tiles = tiles;
+    a.n_tiles = ntiles;
+    a.n_splits = std::max(1u, splits);
+    a.tables = d_tdesc;
+    a.U = static_cast<const double *>(d_U);
+    a.len = static_cast<const double *>(d_len);
+    a.E = n_dense_rows;
+    a.ld = g.ld;
+    a.rows_per_split = splits > 1 ? rows : n_dense_rows;
+    a.alpha = spec.alpha;
+    a.out = out;
+    a.partial = static_cast<double *>(d_partial);
+    const uint64_t slots = static_cast<uint64_t>(std::max(1, n_sms * kd.blocks_per_sm));
+    kd.launch(a, static_cast<uint32_t>(std::min<uint64_t>(static_cast<uint64_t>(ntiles) * a.n_splits, slots)), kd.smem, s);
+    launches++;
+    SSU_CK(cudaMemsetAsync(d_flags, 0, sizeof(int) * ntiles, s));
+    SSU_CK(cudaMemsetAsync(d_close, 0, sizeof(uint32_t) * (static_cast<size_t>(kd.BM) * kd.BN / 32) * ntiles, s));
+    dev::GenFinish f{};
+    f.tiles = tiles;
+    f.n_tiles = ntiles;
+    f.n_splits = a.n_splits;
+    f.tables = d_tdesc;
+    f.partial = a.partial;
+    f.num = n_sparse ? d_gen_num : nullptr;
+    f.den = d_gen_den;
+    f.rs = la.rs;
+    f.W = static_cast<const double *>(d_W);
+    f.unit = walk_unit;
+    f.tau = 0.02;
+    f.tile_flags = d_flags;
+    f.close = d_close;
+    f.out = out;
+    SSU_CK(spec.fp64 ? dev::gen_finish_launch<double>(gl, la, f, gen_small, s)
+                     : dev::gen_finish_launch<float>(gl, la, f, gen_small, s));
+    launches += 2;
+    return 0;
+}
+
 // ------------------------------------------- fp64 unweighted by presence words
 
 // Nodes left to the sample lists in the whole-number form.  A dense node costs
@@ -2658,7 +2811,6 @@ ListRule PlanImpl::bits_list_rule(const TableSet &set) const {
     r.dense_s = std::max(pairs * 8e-14, 1e-8);
     r.pair_s = 1e-12;
     r.entry_s = 6e-11;
-    r.min_div = 1;
     return r;
 }
 
@@ -2932,11 +3084,20 @@ bool use_walk_bits(const MethodSpec &spec, const TableSet &set, const FlatTree &
 // Weighted results by sample lists, unless the dense kernel or the tile walk
 // is asked for.
 bool use_walk_weighted(const MethodSpec &spec, const TableSet &set, const FlatTree &tree) {
-    if (spec.vaw || !(spec.method == Method::weighted_normalized || spec.method == Method::weighted_unnormalized))
+    if (spec.vaw) return false;
+    if (spec.method == Method::generalized) {
+        if (const char *m = std::getenv("UNIFRAC_B200_UNION_MODE"))
+            if (std::string(m) == "dense") return false;
+        // (u^alpha stays at most 1, and alpha 0.0 to 2 leaves the sums well
+        // conditioned away from close pairs)
+        if (!spec.normalize || !(spec.alpha >= 0.0 && spec.alpha <= 2.0)) return false;
+    } else if (spec.method == Method::weighted_normalized || spec.method == Method::weighted_unnormalized) {
+        if (const char *m = std::getenv("UNIFRAC_B200_WEIGHTED_MODE"))
+            if (std::string(m) == "dense") return false;
+        if (!env_int("UNIFRAC_B200_HYBRID_SCATTER", 1)) return false;
+    } else {
         return false;
-    if (const char *m = std::getenv("UNIFRAC_B200_WEIGHTED_MODE"))
-        if (std::string(m) == "dense") return false;
-    if (!env_int("UNIFRAC_B200_HYBRID_SCATTER", 1)) return false;
+    }
     // an explicit zero of a sample without counts is 0 / 0, and its distances
     // are NaN: the embedding's business
     if (spec.normalize)
@@ -2965,6 +3126,7 @@ int Plan::create(const Table &table, const FlatTree &tree, const MethodSpec &spe
     m.gemm = use_tensor_cores(spec, set, tree, false);
     m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
     m.walk_weighted = use_walk_weighted(spec, set, tree);
+    m.walk_gen = m.walk_weighted && spec.method == Method::generalized && spec.alpha != 1.0;
     if (m.gemm) m.start_gemm_layout(set, tree);
     if (m.walk_weighted) m.start_walk_layout(set, tree);
     int rc = m.setup(set, tree, BatchOptions{});
@@ -3002,6 +3164,7 @@ int Plan::create_batch(const TableSet &set, const FlatTree &tree, const MethodSp
     m.gemm = use_tensor_cores(spec, set, tree, true);
     m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
     m.walk_weighted = use_walk_weighted(spec, set, tree);
+    m.walk_gen = m.walk_weighted && spec.method == Method::generalized && spec.alpha != 1.0;
     if (m.gemm) m.start_gemm_layout(set, tree);
     if (m.walk_weighted) m.start_walk_layout(set, tree);
     int rc = m.setup(set, tree, opts);

@@ -66,6 +66,7 @@ struct ListArgs {
     unsigned long long *idx_q = nullptr, *node_q = nullptr;
     double *node_u = nullptr;
     uint32_t *node_all = nullptr;
+    double *idx_u = nullptr;  // generalized: u of each entry
 };
 
 // Samples per part of a table of n samples.
@@ -432,6 +433,8 @@ struct WalkArgs {
     uint32_t n_words;            // 32-bit words of the bitmap
     uint32_t sparse0, dense0, n_dense;  // section starts
     double scale;                // 2^s
+    int gen;                     // generalized: q = round(L u^alpha 2^s), rows of u, W = sum L u^alpha
+    double alpha;
     uint32_t cap;                // nodes held in shared memory
     double *spill;               // values (and ids) of samples with more
     uint32_t *spill_id;
@@ -550,13 +553,16 @@ __global__ void __launch_bounds__(256, WALK_BLOCKS)
         la.node_all[j] = total - rs0;
     }
     __syncthreads();
+    auto power = [&](double u) {
+        return !a.gen || a.alpha == 1.0 ? u : a.alpha == 0.5 ? sqrt(u) : a.alpha == 0.0 ? 1.0 : pow(u, a.alpha);
+    };
     // dense rows
     double wsum = 0.0;
     for (uint32_t r = rd0 + tid; r < total; r += 256) {
         const uint32_t c = ids[r];
-        const double u = vals[r], lu = a.len[c] * u;
+        const double u = vals[r], lu = a.len[c] * power(u);
         wsum += lu;
-        U[static_cast<uint64_t>(c - a.dense0) * a.ld + j] = static_cast<T>(lu);
+        U[static_cast<uint64_t>(c - a.dense0) * a.ld + j] = static_cast<T>(a.gen ? u : lu);
         la.node[first[1] + r - rs0] = c - a.sparse0;
         la.node_u[first[1] + r - rs0] = u;
     }
@@ -577,7 +583,7 @@ __global__ void __launch_bounds__(256, WALK_BLOCKS)
             at[u] = on ? atomicAdd(la.count + slot0 + e[u], 1u) : 0u;
             off[u] = on ? la.off[slot0 + e[u]] : 0u;
             v[u] = on ? vals[rs0 + i] : 0.0;
-            lu[u] = on ? a.len[a.sparse0 + e[u]] * v[u] : 0.0;
+            lu[u] = on ? a.len[a.sparse0 + e[u]] * power(v[u]) : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < UN; u++) {
@@ -591,6 +597,7 @@ __global__ void __launch_bounds__(256, WALK_BLOCKS)
             else
                 static_cast<uint16_t *>(la.idx)[to] = static_cast<uint16_t>(pos);
             la.idx_q[to] = q;
+            if (a.gen) la.idx_u[to] = v[u];
             la.node[first[1] + i0 + u * 256] = e[u];
             la.node_q[first[1] + i0 + u * 256] = q;
             la.node_u[first[1] + i0 + u * 256] = v[u];
