@@ -785,3 +785,35 @@ def test_generalized_by_lists_in_a_batch_as_a_graph(ssu, monkeypatch):
     for a, b, c in zip(run(), run(group_bytes=1), _union_dense(monkeypatch, run)):
         check_fp64(a, c)
         check_fp64(b, c)
+
+
+# ---- Faith PD by the walk
+
+@pytest.mark.parametrize("n,n_tips,density", [(1, 3, 1.0), (2, 17, 0.5), (33, 150, 0.3), (70, 400, 0.01), (257, 16, 0.9)])
+def test_faith_by_the_walk(ssu, oracle_mod, n, n_tips, density):
+    """Bitmaps of one word to many, samples of all tips and of none (explicit
+    zeros), chains and polytomies, tips without a table row."""
+    rng = np.random.default_rng(n)
+    tree, table = _case(700 + n, n_tips=n_tips, n_samples=n, density=density, drop=n_tips // 8)
+    tree = _polytomy(tree, rng)
+    table.data[rng.random(table.data.shape[0]) < 0.1] = 0.0
+    vals, ids = ssu.faith_pd(tree, table)
+    ref = oracle_mod.oracle_faith_pd(tree, table)
+    np.testing.assert_allclose(vals, ref["values"], rtol=1e-12)
+
+
+@pytest.mark.parametrize("what", ["negative length", "negative count", "two tips of one name"])
+def test_faith_leaves_other_inputs_to_the_embedding(ssu, oracle_mod, what):
+    tree, table = _case(84, n_tips=120, n_samples=30, density=0.2)
+    if what == "negative length":
+        tree.lengths = tree.lengths.copy()
+        tree.lengths[np.flatnonzero(tree.structure)[5]] = -0.01
+    elif what == "negative count":
+        table.data[3] = -0.25 * table.data[3]
+    else:
+        names = [i for i, x in enumerate(tree.names) if x]
+        tree.names = list(tree.names)
+        tree.names[names[-1]] = tree.names[names[0]]  # (the last tip is not in the table)
+    vals, _ = ssu.faith_pd(tree, table)
+    ref = oracle_mod.oracle_faith_pd(tree, table)
+    np.testing.assert_allclose(vals, ref["values"], rtol=1e-12)

@@ -137,6 +137,46 @@ static __device__ __forceinline__ void mark_paths(const int32_t *__restrict__ st
     }
 }
 
+// Faith PD by the walk: one block per sample marks its tips' paths in a bitmap
+// over the tree's rows (columns are rows here), then a warp per bitmap word
+// adds the lengths of its nodes, coalesced.  Bound: the walk's loads of
+// parents.  (2,048 samples with 5% of 20,000 tips: 54 us and 64 us for the samples'
+// tips; embedding every row for every sample and summing the rows, 655 MB
+// written and read, 690 us.)
+static __global__ void __launch_bounds__(256)
+    faith_walk_kernel(const uint32_t *__restrict__ sample_ptr, const int32_t *__restrict__ start,
+                      const int32_t *__restrict__ parent, const double *__restrict__ len, uint32_t n_rows,
+                      double *__restrict__ out) {
+    extern __shared__ uint32_t faith_bits[];
+    __shared__ double warp_sum[8];
+    const uint32_t j = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t n_words = (n_rows + 31) / 32;
+    for (uint32_t w = tid; w < n_words; w += 256) faith_bits[w] = 0u;
+    __syncthreads();
+    const uint32_t e0 = sample_ptr[j];
+    mark_paths(start + e0, sample_ptr[j + 1] - e0, parent, faith_bits);
+    __syncthreads();
+    double sum = 0.0;
+    constexpr uint32_t UN = 4;
+    for (uint32_t w = warp; w < n_words; w += 8 * UN) {
+        double v[UN];
+#pragma unroll
+        for (uint32_t u = 0; u < UN; u++) {
+            const uint32_t x = w + 8 * u;
+            // (bits past the last row are never set)
+            v[u] = x < n_words && (faith_bits[x] >> lane) & 1u ? len[x * 32 + lane] : 0.0;
+        }
+        sum += (v[0] + v[1]) + (v[2] + v[3]);
+    }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) warp_sum[warp] = sum;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < 8; w++) sum += warp_sum[w];
+        out[j] = sum;
+    }
+}
+
 // Both sides of the lists for column j, from its presence bitmap over the
 // sparse nodes (words 32-bit words in shared memory), by the whole block of
 // 256 threads; writes rs[j], the threads' `sum` included, and adds their
