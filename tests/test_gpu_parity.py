@@ -817,3 +817,21 @@ def test_faith_leaves_other_inputs_to_the_embedding(ssu, oracle_mod, what):
     vals, _ = ssu.faith_pd(tree, table)
     ref = oracle_mod.oracle_faith_pd(tree, table)
     np.testing.assert_allclose(vals, ref["values"], rtol=1e-12)
+
+
+@pytest.mark.parametrize("method", ["unweighted_fp64", "unweighted", "weighted_normalized_fp64", "weighted_unnormalized",
+                                    "generalized_fp64"])
+def test_plans_refused_the_lists_memory_are_built_without(ssu, oracle_mod, monkeypatch, method):
+    """One table and a batch: the embedding's forms (every node contracted) take over."""
+    tree, table = _case(88, n_tips=300, n_samples=150, density=0.1)
+    ref = oracle_mod.oracle_one_off(tree, table, method.replace("_fp64", "") + "_fp64", alpha=0.5)["matrix"]
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    monkeypatch.setenv("UNIFRAC_B200_TC_LISTS", "1")
+    plan = ssu.BatchPlan(tree, [table, table], method, alpha=0.5, autotune=0)
+    plan.execute()
+    for got in [ssu.one_off_matrix(tree, table, method, alpha=0.5)[0], *plan.results()]:
+        if method.endswith("fp64"):
+            check_fp64(got, ref)
+        else:
+            np.testing.assert_allclose(got, ref, rtol=1e-6, atol=1e-6)
+    plan.close()

@@ -486,6 +486,7 @@ struct PlanImpl {
     }
     void start_gemm_layout(const TableSet &set, const FlatTree &tree) {
         list_rule = tc_list_rule(set, tree.n_embedded);
+        if (!use_lists) list_rule.on = false;
         try {
             gemm_layout = std::async(std::launch::async, build_gemm_layout, std::cref(set), std::cref(tree), list_rule);
         } catch (const std::exception &) {
@@ -589,6 +590,7 @@ struct PlanImpl {
     double *d_list_unit = nullptr;           // the same, as the lists' kernels left it
     int setup_sample_lists(const TableSet &set, const std::vector<int32_t> &start_of_obs);
     int setup_walk_faith(const TableSet &set, const FlatTree &tree);
+    int build(const TableSet &set, const FlatTree &tree, const BatchOptions &opts);
     // Fixed-point lengths of n columns, the sparse nodes' from column `first`
     // on.  `path`: per column the length from it upward (the scale is then
     // the finest that every sample's sum allows); nullptr: sp.scale
@@ -660,12 +662,15 @@ struct PlanImpl {
     std::vector<void *> allocations;
 
     cudaMemPool_t pool = nullptr;
+    bool out_of_memory = false;  // an allocation was refused
+    bool use_lists = true;       // false: the embedding's forms, every node contracted
 
     template <typename P>
     cudaError_t alloc(P **p, size_t bytes) {
         void *q = nullptr;
         cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, std::max<size_t>(bytes, 256), pool, stream)
                              : cudaMallocAsync(&q, std::max<size_t>(bytes, 256), stream);
+        if (e == cudaErrorMemoryAllocation) out_of_memory = true;
         if (e == cudaSuccess) {
             allocations.push_back(q);
             *p = static_cast<P *>(q);
@@ -2286,6 +2291,11 @@ int PlanImpl::shared_sums(cudaStream_t s, const Group &g, const dev::SharedOut &
 int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const SparseNodes &sp,
                           const double *d_len_of_col, uint32_t n, uint32_t first, const std::vector<double> *path,
                           const std::vector<int32_t> &start_of_obs) {
+    if (use_lists && env_int("UNIFRAC_B200_TEST_LIST_MEMORY", 0)) {  // as if an allocation were refused (tests)
+        out_of_memory = true;
+        last_error = "device allocation failed";
+        return kOutputError;
+    }
     n_sparse = static_cast<uint32_t>(sp.row.size());
     sparse_unit = 1.0 / sp.scale;
     if (!n_sparse && !path && !walk_weighted) return setup_sample_lists(set, start_of_obs);
@@ -3128,38 +3138,57 @@ bool use_walk_weighted(const MethodSpec &spec, const TableSet &set, const FlatTr
 
 }  // namespace
 
+// The form of a plan's calls and its buffers.
+int PlanImpl::build(const TableSet &set, const FlatTree &tree, const BatchOptions &opts) {
+    gemm = use_tensor_cores(spec, set, tree, batch);
+    walk_bits = use_lists && !gemm && use_walk_bits(spec, set, tree);
+    walk_weighted = use_lists && use_walk_weighted(spec, set, tree);
+    walk_gen = walk_weighted && spec.method == Method::generalized && spec.alpha != 1.0;
+    if (gemm) start_gemm_layout(set, tree);
+    if (walk_weighted) start_walk_layout(set, tree);
+    if (const int rc = setup(set, tree, opts)) return rc;
+    return gemm          ? setup_gemm(set, tree)
+           : walk_bits     ? setup_walk_bits(set, tree)
+           : walk_weighted ? (spec.fp64 ? setup_walk_weighted<double>(set, tree) : setup_walk_weighted<float>(set, tree))
+           : spec.fp64     ? setup_method<double>()
+                           : setup_method<float>();
+}
+
+// Lists hold sums per pair, which for many samples on a small tree are more
+// than the embedding that they replace: where the device refuses them, the
+// plan is built again without lists.
+int Plan::build(const TableSet &set, const FlatTree &tree, const MethodSpec &spec, const BatchOptions &opts, bool batch,
+                void *stream, Plan **out, std::string &err) {
+    for (bool lists : {true, false}) {
+        Plan *p = new Plan();
+        p->impl_ = new PlanImpl();
+        PlanImpl &m = *p->impl_;
+        m.spec = spec;
+        m.batch = batch;
+        m.use_lists = lists;
+        m.stream = static_cast<cudaStream_t>(stream);
+        m.autotune = resolve_autotune(batch ? opts.autotune : -1, batch);
+        const int rc = m.build(set, tree, opts);
+        if (!rc) {
+            *out = p;
+            return 0;
+        }
+        err = m.last_error;
+        const bool again =
+            lists && m.out_of_memory && (m.walk_bits || m.walk_weighted || (m.gemm && m.list_rule.on));
+        delete p;
+        if (!again) return rc;
+        cudaGetLastError();
+    }
+    return kOutputError;
+}
+
 int Plan::create(const Table &table, const FlatTree &tree, const MethodSpec &spec, void *stream, Plan **out,
                  std::string &err) {
-    Plan *p = new Plan();
-    p->impl_ = new PlanImpl();
-    PlanImpl &m = *p->impl_;
-    m.spec = spec;
-    m.stream = static_cast<cudaStream_t>(stream);
-    m.autotune = resolve_autotune(-1, false);
     TableSet set;
     set.tables.push_back(&table);
     set.embedded.push_back(tree.n_embedded);
-    m.gemm = use_tensor_cores(spec, set, tree, false);
-    m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
-    m.walk_weighted = use_walk_weighted(spec, set, tree);
-    m.walk_gen = m.walk_weighted && spec.method == Method::generalized && spec.alpha != 1.0;
-    if (m.gemm) m.start_gemm_layout(set, tree);
-    if (m.walk_weighted) m.start_walk_layout(set, tree);
-    int rc = m.setup(set, tree, BatchOptions{});
-    if (!rc)
-        rc = m.gemm        ? m.setup_gemm(set, tree)
-             : m.walk_bits ? m.setup_walk_bits(set, tree)
-             : m.walk_weighted
-                 ? (spec.fp64 ? m.setup_walk_weighted<double>(set, tree) : m.setup_walk_weighted<float>(set, tree))
-             : spec.fp64   ? m.setup_method<double>()
-                           : m.setup_method<float>();
-    if (rc) {
-        err = m.last_error;
-        delete p;
-        return rc;
-    }
-    *out = p;
-    return 0;
+    return build(set, tree, spec, BatchOptions{}, false, stream, out, err);
 }
 
 int Plan::create_batch(const TableSet &set, const FlatTree &tree, const MethodSpec &spec, const BatchOptions &opts,
@@ -3170,34 +3199,7 @@ int Plan::create_batch(const TableSet &set, const FlatTree &tree, const MethodSp
         err = "bad table set";
         return kOutputError;
     }
-    Plan *p = new Plan();
-    p->impl_ = new PlanImpl();
-    PlanImpl &m = *p->impl_;
-    m.spec = spec;
-    m.batch = true;
-    m.stream = static_cast<cudaStream_t>(stream);
-    m.autotune = resolve_autotune(opts.autotune, true);
-    m.gemm = use_tensor_cores(spec, set, tree, true);
-    m.walk_bits = !m.gemm && use_walk_bits(spec, set, tree);
-    m.walk_weighted = use_walk_weighted(spec, set, tree);
-    m.walk_gen = m.walk_weighted && spec.method == Method::generalized && spec.alpha != 1.0;
-    if (m.gemm) m.start_gemm_layout(set, tree);
-    if (m.walk_weighted) m.start_walk_layout(set, tree);
-    int rc = m.setup(set, tree, opts);
-    if (!rc)
-        rc = m.gemm        ? m.setup_gemm(set, tree)
-             : m.walk_bits ? m.setup_walk_bits(set, tree)
-             : m.walk_weighted
-                 ? (spec.fp64 ? m.setup_walk_weighted<double>(set, tree) : m.setup_walk_weighted<float>(set, tree))
-             : spec.fp64   ? m.setup_method<double>()
-                           : m.setup_method<float>();
-    if (rc) {
-        err = m.last_error;
-        delete p;
-        return rc;
-    }
-    *out = p;
-    return 0;
+    return build(set, tree, spec, opts, true, stream, out, err);
 }
 
 int Plan::create_faith(const Table &table, const FlatTree &tree, void *stream, Plan **out, std::string &err) {

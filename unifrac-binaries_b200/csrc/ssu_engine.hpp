@@ -82,7 +82,7 @@ class Plan {
     // the other in device memory.
     static int create_batch(const TableSet &set, const FlatTree &tree, const MethodSpec &spec,
                             const BatchOptions &opts, void *stream, Plan **out, std::string &err);
-    // Faith PD plan: embedding of every non-root node in fp64, no pair stage.
+    // Faith PD plan: no pair stage.
     static int create_faith(const Table &table, const FlatTree &tree, void *stream, Plan **out, std::string &err);
     ~Plan();
 
@@ -143,6 +143,8 @@ class Plan {
 
   private:
     Plan() = default;
+    static int build(const TableSet &set, const FlatTree &tree, const MethodSpec &spec, const BatchOptions &opts,
+                     bool batch, void *stream, Plan **out, std::string &err);
     PlanImpl *impl_ = nullptr;
 };
 
