@@ -53,8 +53,6 @@ WORKLOADS = {
 # normalized fp64 method (accumulator read-modify-write of two fp64 stripes
 # per 112-node batch: 2 * 2 * 8 / 112)
 ALGO_BYTES_PER_UPDATE = 2 * 2 * 8 / 112.0
-PROFILE_TRAFFIC = os.path.join(ROOT, "profiles", "pair_hybrid_weighted_normalized_fp64_20k_tips_2048_samples.md")
-PROFILE_TC = os.path.join(ROOT, "profiles", "unweighted_tc_kernel_100k_tips_25k_presence.md")
 
 
 def parse():
@@ -230,22 +228,6 @@ class ClockSampler:
                 continue
             rows.append((s, m, [name for name, val in zip(cls.NAMES, f[5:9]) if val.lower() == "active"]))
         return rows
-
-
-def read_profile_value(path, key):
-    """A `key: value ...` figure from a committed ncu summary (first token)."""
-    try:
-        for line in open(path):
-            if line.startswith(key + ":"):
-                return float(line.split(":", 1)[1].split()[0])
-    except (OSError, ValueError):
-        pass
-    return None
-
-
-def read_traffic():
-    """dram bytes per hybrid pair-kernel launch from the committed ncu summary."""
-    return read_profile_value(PROFILE_TRAFFIC, "dram_bytes_per_launch_full_size")
 
 
 def peaks():
@@ -438,13 +420,6 @@ def _step_loop(torch, plan, stream, steps, barrier, flush):
     return step_ms, pair_ms
 
 
-def tc_work_units(n):
-    """Work units of the tensor-core kernel for one table of n samples: the
-    (256-row, 128-column) blocks holding a pair k < l."""
-    nkb, nlb = (n + 255) // 256, (n + 127) // 128
-    return sum(1 for kb in range(nkb) for lb in range(nlb) if kb * 256 < min(n, (lb + 1) * 128) - 1)
-
-
 def run_presence(args):
     """The default line: unweighted fp64 on the 100,000-tip / 25,000-sample
     presence table through the tcgen05 contraction, with the plain stripe
@@ -551,8 +526,6 @@ def run_presence(args):
         algo_flops = 2.0 * units
         achieved = algo_flops / (mean_tc_ms / 1e3) / 1e12
         issued = flops_issued / (mean_tc_ms / 1e3) / 1e12  # int8 tensor ops
-        traffic_per_unit = read_profile_value(PROFILE_TC, "dram_bytes_per_work_unit")
-        n_units = tc_work_units(n)
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
@@ -562,22 +535,22 @@ def run_presence(args):
             "data": "synthetic (seeded generator presence_100k_tips_25k_samples)",
             "config": {"workload": PRESENCE_WORKLOAD, "method": method, "pair_kernel": "unweighted_tc_kernel",
                        "n_samples": n, "embedded_branches": gp_units_e(units, n), "per_gpu_units": units,
-                       "l2": "flushed between steps (256 MiB write outside the step events); operands 30 GB > L2",
+                       "l2": "flushed between steps (256 MiB write outside the step events)",
                        "generation_s": gen_s},
             "tc_kernel_ms": mean_tc_ms,
             **extra,
-            "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak_sus, "unit": "TFLOP/s",
-                         "frac": achieved / peak_sus, "traffic": traffic_per_unit * n_units if traffic_per_unit else None,
-                         "peak_kind": f"{peak_kind} bf16 sustained (the kernel runs ~0.2 s per launch, back to back)",
-                         "frac_of_burst": achieved / peak_burst,
+            "roofline": {"bound": "tensor", "achieved": issued, "peak": 2.0 * peak_sus, "unit": "TOP/s (int8)",
+                         "frac": issued / (2.0 * peak_sus), "traffic": None,
+                         "peak_kind": f"2 x {peak_kind} bf16 sustained (dense int8 : bf16 = 2 : 1 on B200)",
+                         "frac_of_burst": issued / (2.0 * peak_burst),
                          "algorithmic_flops_per_launch": algo_flops, "issued_int8_ops_per_launch": flops_issued,
-                         "issued_int8_tops": issued, "issued_frac": issued / (2.0 * peak_sus),
-                         "issued_peak": f"2 x {peak_kind} bf16 sustained (dense int8 : bf16 = 2 : 1 on B200)",
-                         "note": "algorithmic flops = 2 x pair-branch updates (one multiply-add per pair and "
-                                 "branch), against the bf16 peak; the kernel issues ~2x that in int8 ops (two "
-                                 "digit products per length, padding of the length chunks and of 256 x 128 work "
-                                 "units on the diagonal) at twice the bf16 rate; traffic = ncu DRAM bytes per work unit x work "
-                                 "units"},
+                         "algorithmic_tflops": achieved,
+                         "note": "over the pair stage: the sums over nodes that few samples have (by lists of their "
+                                 "samples, no tensor work) and the contraction of the other nodes (two int8 digit "
+                                 "products per length, padding of the length chunks and of 256 x 128 work units on "
+                                 "the diagonal); the contraction is bound by shared-memory operand bandwidth; "
+                                 "algorithmic flops = 2 x pair-branch updates over every node, so they are not "
+                                 "work that the tensor cores do"},
             "e2e": {"value": all_units * len(e2e_ms) / (e2e_total / 1e3) if e2e_ms else None, "unit": UNIT,
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "ms_per_step": e2e_total / len(e2e_ms) if e2e_ms else None,
@@ -944,15 +917,15 @@ def measure_weighted(args, world, rank, local, stream=None, flush=None, cpu=True
         "data": "synthetic (seeded generator lognormal_20k_tips_2048_samples)",
         "config": {"workload": WEIGHTED_WORKLOAD, "method": args.method, "n_samples": args.samples,
                    "n_tips": args.tips, "embedded_branches": n_emb, "pair_kernel": kernel,
-                   "l2": "flushed between steps (256 MiB write outside the step events); embedding 655 MB > L2",
+                   "l2": "flushed between steps (256 MiB write outside the step events)",
                    "per_gpu_units": units},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": read_traffic(), "peak_kind": peak_kind,
+                     "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
                      "algorithmic_bytes_per_launch": algo_bytes,
                      "note": "reference-form bytes (2 fp64 accumulators RMW per 112-node batch) over the "
-                             "pair stage; the hybrid kernel keeps its accumulators on chip (traffic = its "
-                             "measured DRAM bytes per launch), so the binding bound is instruction issue: "
-                             "see fp64_dense_equivalent and the profile summary",
+                             "pair stage; accumulators stay on chip and nodes that few samples have are summed "
+                             "by lists of their samples, so this is an accounting figure: the stage is bound by "
+                             "the fp64 pipe over the dense rows and by shared-memory atomics over the lists",
                      "fp64_dense_equivalent": {"achieved_tflops": fp64_achieved,
                                                "peak_tflops_at_clock": fp64_peak,
                                                "frac": fp64_achieved / fp64_peak}},
