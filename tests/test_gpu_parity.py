@@ -5,11 +5,13 @@ Bars: fp64 methods within 1e-12 relative of the oracle (1e-13 absolute where
 the oracle value is 0); fp32 methods within 4x the reference fp32 build's own
 error against fp64 on the same input (measured with the oracle's fp32 mode),
 floored at 1e-6; NaN patterns identical."""
+import os
+
 import numpy as np
 import pytest
 
 import ssu_synth
-from conftest import matrix_from_stripes, rel_err, stripes_from_golden
+from conftest import ROOT, matrix_from_stripes, rel_err, stripes_from_golden
 
 pytestmark = pytest.mark.gpu
 
@@ -835,3 +837,28 @@ def test_plans_refused_the_lists_memory_are_built_without(ssu, oracle_mod, monke
         else:
             np.testing.assert_allclose(got, ref, rtol=1e-6, atol=1e-6)
     plan.close()
+
+
+# ---- fp32 methods whose results leave as doubles
+
+CRAWFORD = [os.path.join(ROOT, "tests", "golden", "fixtures", f) for f in ("crawford.biom", "crawford.tre")]
+
+
+@pytest.mark.parametrize("method", ["unweighted", "unweighted_unnormalized", "weighted_normalized", "weighted_unnormalized",
+                                    "generalized"])
+def test_doubles_of_fp32_methods_keep_the_form_without_lists(ssu, monkeypatch, method):
+    """Condensed, stripes, a pair and a file's matrix of an fp32 method are the
+    embedding's values bit for bit (as with the lists refused), also where a
+    plan of the same table sums its nodes by lists."""
+    tree, table = _case(89, n_tips=300, n_samples=150, density=0.1)
+    monkeypatch.setenv("UNIFRAC_B200_TC_LISTS", "1")
+    monkeypatch.setenv("UNIFRAC_B200_DETERMINISTIC", "1")
+    dense = table.dense()
+    calls = [lambda: ssu.one_off(tree, table, method, alpha=0.5)[0],
+             lambda: ssu.partial(tree, table, method, 10, 40, alpha=0.5)[0],
+             lambda: ssu.dense_pair(tree, table.obs_ids, dense[:, 0], dense[:, 1], method, alpha=0.5),
+             lambda: ssu.file_matrix("one_off_matrix_v3", *CRAWFORD, method, alpha=0.5)[0]]
+    got = [call() for call in calls]
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    for a, call in zip(got, calls):
+        np.testing.assert_array_equal(a, call())

@@ -211,7 +211,18 @@ struct Request {
     double alpha;
     bool bypass;
     bool normalize;
+    // The result can leave as doubles whatever the method's precision.  fp32
+    // methods then keep to the embedding's forms: a sum in another form moves
+    // each distance by a rounding of a single (2-norm of the change 3.6e-8 of
+    // the result's), which a caller who has doubles would see.
+    bool doubles = false;
 };
+
+// The same request, its result in doubles.
+Request as_doubles(Request r) {
+    r.doubles = true;
+    return r;
+}
 
 ComputeStatus make_plan(const ssu::Table &table, const ssu::BPTree &tree, const Request &r,
                         std::unique_ptr<ssu::Plan> &plan, StepTimer &timer) {
@@ -221,6 +232,7 @@ ComputeStatus make_plan(const ssu::Table &table, const ssu::BPTree &tree, const 
     spec.alpha = r.alpha;
     spec.bypass_tips = r.bypass;
     spec.normalize = r.normalize;
+    spec.lists = spec.fp64 || !r.doubles;
     unweighted_mode(spec);
     std::string err;
     if (!select_device(err)) {
@@ -695,7 +707,7 @@ ComputeStatus subsample_batch_v3(const support_biom_t *table_data, const support
 ComputeStatus condensed(const ssu::Table &table, const ssu::BPTree &tree, const Request &r, mat_t **result) {
     StepTimer timer("one_off");
     std::unique_ptr<ssu::Plan> plan;
-    ComputeStatus st = make_plan(table, tree, r, plan, timer);
+    ComputeStatus st = make_plan(table, tree, as_doubles(r), plan, timer);
     if (st != okay) return st;
     const uint64_t n = table.n_samples;
     mat_t *m = static_cast<mat_t *>(std::malloc(sizeof(mat_t)));
@@ -726,7 +738,7 @@ ComputeStatus partial_stripes(const ssu::Table &table, const ssu::BPTree &tree, 
         return output_error;
     }
     std::unique_ptr<ssu::Plan> plan;
-    ComputeStatus st = make_plan(table, tree, r, plan, timer);
+    ComputeStatus st = make_plan(table, tree, as_doubles(r), plan, timer);
     if (st != okay) return st;
     partial_mat_t *p = static_cast<partial_mat_t *>(std::malloc(sizeof(partial_mat_t)));
     p->n_samples = table.n_samples;
@@ -1131,7 +1143,7 @@ static ComputeStatus dense_pair(unsigned int n_obs, const char **obs_ids, const 
         }
     } else {
         mat_full_fp32_t *m = nullptr;
-        st = full_matrix<float, mat_full_fp32_t>(table, tree, r, nullptr, &m);
+        st = full_matrix<float, mat_full_fp32_t>(table, tree, as_doubles(r), nullptr, &m);
         if (st == okay) {
             *result = m->matrix[1];
             destroy_mat_full_fp32(&m);
@@ -1214,10 +1226,12 @@ ComputeStatus one_off_wtree(const char *biom_filename, const opaque_bptree_t *tr
 namespace {
 
 // one_off_matrix_v3_T over a loaded table (src/api.cpp:700-717): optional
-// rarefaction, the method's precision for the arithmetic, TReal for the result.
+// rarefaction, the method's precision for the arithmetic, TReal for the result
+// (an fp32 method gives the same values as singles and as doubles).
 template <class TReal, class TMat>
-ComputeStatus file_matrix(ComputeStatus loaded, const ssu::Table &table, const ssu::BPTree &tree, const Request &r,
+ComputeStatus file_matrix(ComputeStatus loaded, const ssu::Table &table, const ssu::BPTree &tree, const Request &request,
                           unsigned int subsample_depth, bool with_replacement, const char *mmap_dir, TMat **result) {
+    const Request r = as_doubles(request);
     if (loaded != okay) return loaded;
     if (!result) return output_error;
     if (mmap_dir && mmap_dir[0] == 0) mmap_dir = nullptr;

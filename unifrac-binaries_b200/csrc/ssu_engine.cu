@@ -3160,6 +3160,7 @@ int PlanImpl::build(const TableSet &set, const FlatTree &tree, const BatchOption
 int Plan::build(const TableSet &set, const FlatTree &tree, const MethodSpec &spec, const BatchOptions &opts, bool batch,
                 void *stream, Plan **out, std::string &err) {
     for (bool lists : {true, false}) {
+        if (lists && !spec.lists) continue;
         Plan *p = new Plan();
         p->impl_ = new PlanImpl();
         PlanImpl &m = *p->impl_;

@@ -32,6 +32,8 @@ struct MethodSpec {
     // results too, unweighted_stripe keeps the presence-word stripe kernel
     bool unweighted_gemm = false;
     bool unweighted_stripe = false;
+    // false: no sample lists (the embedding's forms, every node contracted)
+    bool lists = true;
 };
 
 // Method-name table of the reference (src/api.cpp:55-88): bare names are fp32.
