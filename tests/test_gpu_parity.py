@@ -862,3 +862,54 @@ def test_doubles_of_fp32_methods_keep_the_form_without_lists(ssu, monkeypatch, m
     monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
     for a, call in zip(got, calls):
         np.testing.assert_array_equal(a, call())
+
+
+# ---- tables of common features
+
+def _prevalent(seed, n, n_tips, kind):
+    """Features that most samples have: prevalences Beta(2, 2) or Beta(5, 2), or
+    95% of them at 95% and a few at 5%; every sample has a count."""
+    tree = ssu_synth.random_binary_tree(n_tips, 0.1, seed)
+    rng = np.random.default_rng(seed)
+    p = {"beta22": lambda: rng.beta(2, 2, n_tips), "beta52": lambda: rng.beta(5, 2, n_tips),
+         "few rare": lambda: np.where(rng.random(n_tips) < 0.05, 0.05, 0.95)}[kind]()
+    dense = np.where(rng.random((n_tips, n)) < p[:, None], rng.geometric(0.1, (n_tips, n)), 0).astype(float)
+    dense[rng.integers(n_tips), :] = 2.0
+    return tree, ssu_synth.Table.from_dense(dense, tree.tip_names(), ["S%d" % j for j in range(n)])
+
+
+@pytest.mark.parametrize("kind", ["beta22", "beta52", "few rare"])
+@pytest.mark.parametrize("n", [129, 640, 1000, 2048])
+def test_whole_number_unweighted_of_common_features(ssu, monkeypatch, kind, n):
+    """Nearly all length in dense nodes, a few sparse ones: the fixed point's
+    scale follows what a sample sums.  Full matrix, condensed, window, batch."""
+    tree, table = _prevalent(n, n, 300, kind)
+    stop = (n + 1) // 2
+
+    def batch():
+        plan = ssu.BatchPlan(tree, [table, table], "unweighted_fp64", autotune=0)
+        plan.execute()
+        got = plan.results()[1]
+        plan.close()
+        return got
+    for method in ("unweighted_fp64", "unweighted_unnormalized_fp64"):
+        calls = [lambda: ssu.one_off_matrix(tree, table, method)[0], lambda: ssu.one_off(tree, table, method)[0],
+                 lambda: ssu.partial(tree, table, method, stop // 3, stop // 3 + 20)[0], batch]
+        for call in calls if n == 640 else calls[:1]:
+            check_fp64(call(), _stripe_mode(monkeypatch, call))
+
+
+def test_whole_number_unweighted_with_one_long_stem(ssu, oracle_mod):
+    """A small clade under a stem of a thousand times the other lengths, which
+    every sample has; the rest of the tree is rare."""
+    tree, table = _case(93, n_tips=200, n_samples=300, density=0.05, drop=0)
+    inner = [i for i in range(1, len(tree.structure) - 1) if tree.structure[i] and tree.structure[i + 1]]
+    dense = table.dense()
+    first = table.obs_ids.index(next(nm for nm in tree.names[inner[0]:] if nm))
+    dense[first, :] = 1.0
+    tree.lengths = tree.lengths.copy()
+    tree.lengths[inner[0]] = 1000.0 * tree.lengths.max()
+    table = ssu_synth.Table.from_dense(dense, table.obs_ids, table.sample_ids)
+    for method in ("unweighted_fp64", "unweighted_unnormalized_fp64"):
+        gpu, _ = ssu.one_off_matrix(tree, table, method)
+        check_fp64(gpu, oracle_mod.oracle_one_off(tree, table, method)["matrix"])

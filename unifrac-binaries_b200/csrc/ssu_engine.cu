@@ -2382,15 +2382,17 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
         if (n_sparse) SSU_CK(cudaMemsetAsync(g.lists.idx, 0, std::max<size_t>(g.list_bytes, 1), stream));
     if (walk_weighted) return list_attributes();
     unsigned long long *d_top = nullptr;
+    double all = 0.0;
     if (path) {
+        for (uint32_t e = 0; e < E; e++) all += tree.length[e];
         SSU_CK(alloc(&d_top, sizeof(unsigned long long)));
         SSU_CK(cudaMemsetAsync(d_top, 0, sizeof(unsigned long long), stream));
         for (const Group &g : groups)
             dev::list_bound_kernel<<<static_cast<uint32_t>((g.ld + 7) / 8), 256, 0, stream>>>(
                 g.d_sample_ptr, g.d_start_col, static_cast<uint32_t>(g.ld), d_path, d_top);
     }
-    dev::fixed_lengths_kernel<<<(n + 255) / 256, 256, 0, stream>>>(d_len_of_col, n, d_top, sp.scale, d_sparse_q,
-                                                                  d_list_unit);
+    dev::fixed_lengths_kernel<<<(n + 255) / 256, 256, 0, stream>>>(d_len_of_col, n, d_top, all, sp.scale,
+                                                                  d_sparse_q, d_list_unit);
     SSU_CK(cudaGetLastError());
     return list_attributes();
 }

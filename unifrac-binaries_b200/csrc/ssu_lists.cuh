@@ -92,17 +92,19 @@ static __global__ void __launch_bounds__(256)
 }
 
 // q = round(L 2^s), unit = 2^-s.  The scale is `least`, at which the sum of
-// every sparse length stays below 2^62 units, or (top != nullptr) the finest
-// at which the largest sample's does.
+// every sparse length stays below 2^62 units, or (top != nullptr: every column
+// is summed as q) the finest at which no sample's sum reaches 2^63: it is at
+// most *top, and at most `all`, the sum of every length.  (`least` counts the
+// sparse lengths alone, and would wrap the sums of samples that are mostly dense nodes.)
 static __global__ void fixed_lengths_kernel(const double *__restrict__ len, uint32_t n,
-                                            const unsigned long long *__restrict__ top, double least,
+                                            const unsigned long long *__restrict__ top, double all, double least,
                                             unsigned long long *__restrict__ q, double *__restrict__ unit) {
     double scale = least;
     if (top) {
-        const double m = __longlong_as_double(static_cast<long long>(*top));
+        const double m = fmin(__longlong_as_double(static_cast<long long>(*top)), all);
         int x = 0;
-        frexp(m * (1.0 + 1e-9), &x);  // m < 2^x
-        if (m > 0.0) scale = fmax(ldexp(1.0, min(62 - x, 1000)), least);
+        frexp(m * (1.0 + 1e-9), &x);  // m < 2^x, by more than the roundings add
+        scale = m > 0.0 ? ldexp(1.0, min(63 - x, 1000)) : 1.0;
     }
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *unit = 1.0 / scale;
