@@ -913,3 +913,29 @@ def test_whole_number_unweighted_with_one_long_stem(ssu, oracle_mod):
     for method in ("unweighted_fp64", "unweighted_unnormalized_fp64"):
         gpu, _ = ssu.one_off_matrix(tree, table, method)
         check_fp64(gpu, oracle_mod.oracle_one_off(tree, table, method)["matrix"])
+
+
+@pytest.mark.parametrize("alpha", [0.0, 0.5, 1.0, 1.5, 2.0])
+@pytest.mark.parametrize("n", [20, 300])
+def test_generalized_with_one_long_stem(ssu, oracle_mod, alpha, n):
+    """Three quarters of the tree's length (95 of 127) in a stem that every
+    sample has whole, so that s^alpha = 2^alpha on it, over eight tips of length
+    4 of which a sample has one or two: the denominator is 2.2 (alpha 1.5) and
+    3.1 (alpha 2) times the tree's length, and few pairs are close.  (Two more
+    tips beside the stem are not in the table.)"""
+    structure, lengths, names = [True, True], [0.0, 95.0], ["", ""]
+    for i in range(10):
+        if i == 8:
+            structure.append(False), lengths.append(0.0), names.append("")
+        structure += [True, False]
+        lengths += [4.0, 0.0]
+        names += ["T%d" % i, ""]
+    structure.append(False), lengths.append(0.0), names.append("")
+    tree = ssu_synth.BPTree(np.array(structure), np.array(lengths), names)
+    rng = np.random.default_rng(n)
+    dense = np.zeros((8, n))
+    for j in range(n):
+        dense[rng.integers(8, size=rng.integers(1, 3)), j] = rng.integers(1, 9)
+    table = ssu_synth.Table.from_dense(dense, ["T%d" % i for i in range(8)], ["S%d" % j for j in range(n)])
+    gpu, _ = ssu.one_off_matrix(tree, table, "generalized_fp64", alpha=alpha)
+    check_fp64(gpu, oracle_mod.oracle_one_off(tree, table, "generalized_fp64", alpha=alpha)["matrix"])

@@ -2533,9 +2533,13 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
         for (const Group &g : groups)
             for (double t : g.totals) vmax = std::max(vmax, t);
     double bound = lay.path_max * vmax;
-    if (walk_gen) {  // u^alpha <= 1 for proportions: at most every length
+    if (walk_gen && spec.alpha < 1.0) {  // u^alpha <= 1 for proportions: at most every length
         bound = 0.0;
         for (double L : lay.len) bound += L;
+    } else if (walk_gen) {
+        // u^alpha <= u, but (u_k + u_l)^alpha <= 2^(alpha - 1) (u_k + u_l): the
+        // denominator, and a term of it, reaches that many times r_k + r_l
+        bound *= std::pow(2.0, spec.alpha - 1.0);
     }
     int x = 0;
     std::frexp(std::max(2.0 * bound * (1.0 + 1e-9), 1e-290), &x);  // (r_k + r_l stays below 2^63)
@@ -3117,7 +3121,8 @@ bool use_walk_weighted(const MethodSpec &spec, const TableSet &set, const FlatTr
         if (const char *m = std::getenv("UNIFRAC_B200_UNION_MODE"))
             if (std::string(m) == "dense") return false;
         // (u^alpha stays at most 1, and alpha 0.0 to 2 leaves the sums well
-        // conditioned away from close pairs)
+        // conditioned away from close pairs; their scale allows for s^alpha up
+        // to 2^alpha)
         if (!spec.normalize || !(spec.alpha >= 0.0 && spec.alpha <= 2.0)) return false;
     } else if (spec.method == Method::weighted_normalized || spec.method == Method::weighted_unnormalized) {
         if (const char *m = std::getenv("UNIFRAC_B200_WEIGHTED_MODE"))
