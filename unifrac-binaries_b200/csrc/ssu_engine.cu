@@ -2632,14 +2632,8 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     walk.scale = scale;
     walk.gen = walk_gen ? 1 : 0;
     walk.alpha = spec.alpha;
-    // values in shared memory for samples of up to `cap` nodes (WALK_BLOCKS an
-    // SM), else in memory (eight tables on 50,000 tips, 4,500 nodes a sample: the
-    // walk takes the same with fewer blocks and all of them in shared memory)
-    const size_t fixed = sizeof(uint32_t) * (2ull * walk.n_words + 1 + 2ull * walk.n_levels + 4) + 8;
-    constexpr size_t block = 227 * 1024 / dev::WALK_BLOCKS - 1536;  // (1 KB of it the system's)
-    const size_t room = fixed + 8 * 1024 < block ? block - fixed : 8 * 1024;
-    walk.cap = std::min<uint32_t>(n_cols, static_cast<uint32_t>(room / 12));
-    walk_smem = static_cast<size_t>(walk.cap) * 12 + fixed;
+    walk.cap = ssu::walk::capacity(n_cols, walk.n_levels);
+    walk_smem = ssu::walk::shared_bytes(n_cols, walk.n_levels);
     uint64_t spill = 0;  // nodes of all samples of a group, at most
     for (const Group &g : groups) {
         uint64_t m = 0;
@@ -2677,7 +2671,7 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     for (const void *kernel : {reinterpret_cast<const void *>(dev::weighted_walk_kernel<T>),
                                reinterpret_cast<const void *>(dev::weighted_walk_kernel<double>)})
         SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(tc::MAX_BITMAP_BYTES)));
+                                    static_cast<int>(ssu::walk::kSharedMost)));
     tuning = "sample lists";
     timer.step("walk_buffers");
     return 0;
@@ -3140,7 +3134,9 @@ bool use_walk_weighted(const MethodSpec &spec, const TableSet &set, const FlatTr
             for (uint64_t q = 0; empty && q < t->nnz(); q++)
                 if (t->totals[t->indices[q]] == 0.0) return false;
         }
-    return can_walk(set, tree, 2) && tree.level_ptr.size() <= 4096;  // presence and ranks; the levels' ranks
+    // (presence and ranks, and the levels' ranks: a deep tree of many nodes stays on the embedding)
+    return can_walk(set, tree, 2) && tree.level_ptr.size() <= 4096 &&
+           ssu::walk::fits(tree.n_nodes, tree.level_ptr.empty() ? 0 : tree.level_ptr.size() - 1);
 }
 
 }  // namespace

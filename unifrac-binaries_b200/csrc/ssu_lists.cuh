@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include "ssu_kernels.cuh"
+#include "ssu_walk_size.hpp"
 
 namespace ssu {
 namespace dev {
@@ -484,10 +485,8 @@ struct WalkArgs {
     uint64_t ld;
 };
 
-constexpr int WALK_BLOCKS = 6;  // blocks an SM: the walk waits on loads and barriers, so samples in flight set its pace
-
 template <typename T>
-__global__ void __launch_bounds__(256, WALK_BLOCKS)
+__global__ void __launch_bounds__(256, walk::kBlocks)
     weighted_walk_kernel(const WalkArgs a, T *__restrict__ U, T *__restrict__ W, const uint32_t *__restrict__ column,
                          const ListArgs la) {
     extern __shared__ double walk_s[];
