@@ -867,12 +867,12 @@ def test_doubles_of_fp32_methods_keep_the_form_without_lists(ssu, monkeypatch, m
 # ---- tables of common features
 
 def _prevalent(seed, n, n_tips, kind):
-    """Features that most samples have: prevalences Beta(2, 2) or Beta(5, 2), or
-    95% of them at 95% and a few at 5%; every sample has a count."""
+    """Features that most samples have: prevalences Beta(2, 2) or Beta(5, 2),
+    95% of them at 95% and a few at 5%, or all at 90%; every sample has a count."""
     tree = ssu_synth.random_binary_tree(n_tips, 0.1, seed)
     rng = np.random.default_rng(seed)
     p = {"beta22": lambda: rng.beta(2, 2, n_tips), "beta52": lambda: rng.beta(5, 2, n_tips),
-         "few rare": lambda: np.where(rng.random(n_tips) < 0.05, 0.05, 0.95)}[kind]()
+         "few rare": lambda: np.where(rng.random(n_tips) < 0.05, 0.05, 0.95), "common": lambda: np.full(n_tips, 0.9)}[kind]()
     dense = np.where(rng.random((n_tips, n)) < p[:, None], rng.geometric(0.1, (n_tips, n)), 0).astype(float)
     dense[rng.integers(n_tips), :] = 2.0
     return tree, ssu_synth.Table.from_dense(dense, tree.tip_names(), ["S%d" % j for j in range(n)])
@@ -939,3 +939,16 @@ def test_generalized_with_one_long_stem(ssu, oracle_mod, alpha, n):
     table = ssu_synth.Table.from_dense(dense, ["T%d" % i for i in range(8)], ["S%d" % j for j in range(n)])
     gpu, _ = ssu.one_off_matrix(tree, table, "generalized_fp64", alpha=alpha)
     check_fp64(gpu, oracle_mod.oracle_one_off(tree, table, "generalized_fp64", alpha=alpha)["matrix"])
+
+
+@pytest.mark.parametrize("method", ["unweighted_fp64", "weighted_normalized_fp64"])
+def test_without_sparse_nodes_the_walk_is_one_launch(ssu, method):
+    """2,500 samples that have nearly every tip: the walk, the pair kernel (and
+    its split sums), the flagged tiles or close pairs, however many parts a
+    list would have."""
+    tree, table = _prevalent(7, 2500, 120, "common")
+    plan = ssu.Plan(tree, table, method)
+    plan.execute()
+    plan.result()
+    assert plan.launches() <= 4
+    plan.close()

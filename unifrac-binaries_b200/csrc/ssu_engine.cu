@@ -2330,12 +2330,14 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
         // parts of at least a wave of blocks of the walk (for the weighted
         // walk two thirds: its shared sums read ten bytes an entry)
         la.slots = static_cast<uint64_t>(tg) * n_sparse;
+        // (no sparse node, nothing to read in parts)
         la.parts = static_cast<uint32_t>(
             std::max<uint64_t>(1, std::min<uint64_t>(dev::LIST_PARTS, g.ld / ((walk_weighted ? 4 : 8) * static_cast<uint64_t>(n_sms)))));
+        if (!n_sparse) la.parts = 1;
         uint32_t n_max = 1;
         for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);
         const uint32_t most = walk_gen ? dev::kGenCols : kSharedCols;
-        while (dev::list_part_rows(n_max, la.parts) > most) la.parts *= 2;  // (a part's columns fit a block)
+        while (n_sparse && dev::list_part_rows(n_max, la.parts) > most) la.parts *= 2;  // (a part's columns fit a block)
         std::vector<std::vector<uint32_t>> by_part(la.parts);
         for (uint32_t t = g.t0; t < g.t1; t++) {
             const uint32_t n_t = tdesc[t].n, rows = dev::list_part_rows(std::max(n_t, 1u), la.parts);
