@@ -952,3 +952,62 @@ def test_without_sparse_nodes_the_walk_is_one_launch(ssu, method):
     plan.result()
     assert plan.launches() <= 4
     plan.close()
+
+
+# ---- tables of near duplicates (every pair is summed again over its own nodes)
+
+def _all_near(seed, n, n_tips, density):
+    """One community with a percent of noise in its counts and a feature or two gained or lost."""
+    tree = ssu_synth.random_binary_tree(n_tips, 0.1, seed)
+    rng = np.random.default_rng(seed)
+    base = rng.random(n_tips) < density
+    base[0] = True
+    on = base[:, None] ^ (rng.random((n_tips, n)) < 1.0 / n_tips)
+    on[0] = True
+    counts = np.exp(2 + 1.5 * rng.standard_normal(n_tips))[:, None] * np.exp(0.01 * rng.standard_normal((n_tips, n)))
+    dense = np.where(on, np.round(50 * counts) + 1, 0.0)
+    return tree, ssu_synth.Table.from_dense(dense, tree.tip_names(), ["S%d" % j for j in range(n)])
+
+
+@pytest.mark.parametrize("n,n_tips,density", [(2, 30, 0.9), (17, 60, 0.5), (129, 300, 0.2), (150, 9000, 0.002), (300, 700, 0.9)])
+@pytest.mark.parametrize("method,alpha", [("weighted_normalized_fp64", 1.0), ("weighted_unnormalized_fp64", 1.0),
+                                          ("generalized_fp64", 0.0), ("generalized_fp64", 0.5), ("generalized_fp64", 1.5)])
+def test_near_duplicates_are_summed_over_their_own_nodes(ssu, oracle_mod, method, alpha, n, n_tips, density):
+    """Strips with every row and column involved and with few, the last ones
+    short; samples of fewer and of more nodes than are laid out at once, long
+    runs of nodes that none has; full matrix, window, condensed."""
+    tree, table = _all_near(n, n, n_tips, density)
+    if n == 129:  # half of the samples are like no other
+        dense = table.dense()
+        rng = np.random.default_rng(5)
+        dense[:, ::2] = np.where(rng.random(dense[:, ::2].shape) < 0.3, rng.geometric(0.1, dense[:, ::2].shape), 0.0)
+        dense[0] = 4.0
+        table = ssu_synth.Table.from_dense(dense, table.obs_ids, table.sample_ids)
+    kw = {"alpha": alpha}
+    ref = oracle_mod.oracle_one_off(tree, table, method, **kw)["matrix"]
+    check_fp64(ssu.one_off_matrix(tree, table, method, **kw)[0], ref)
+    if n > 2:
+        check_fp64(ssu.one_off(tree, table, method, **kw)[0], ref[np.triu_indices(n, 1)])
+        stop = (n + 1) // 2
+        s, k = np.arange(stop // 3, stop)[:, None], np.arange(n)[None, :]
+        check_fp64(ssu.partial(tree, table, method, stop // 3, stop, **kw)[0], ref[k, (k + s + 1) % n])
+
+
+@pytest.mark.parametrize("method", ["weighted_normalized_fp64", "generalized_fp64"])
+def test_a_table_of_near_duplicates_costs_little_more_than_another(ssu, method):
+    """500 samples, every pair close, against 500 unrelated ones with as many
+    features: less than eight times as long (a thread a pair took over 60 times)."""
+    near = _all_near(11, 500, 4000, 0.05)
+    other = _case(11, n_tips=4000, n_samples=500, density=0.05, drop=0)
+    best = []
+    for tree, table in (near, other):
+        plan = ssu.Plan(tree, table, method, alpha=0.5)
+        plan.set_timing(True)
+        ms = []
+        for _ in range(5):
+            plan.execute()
+            plan.result()
+            ms.append(sum(plan.stage_ms()))
+        best.append(min(ms))
+        plan.close()
+    assert best[0] < 8 * best[1], best

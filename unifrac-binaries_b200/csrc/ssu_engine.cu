@@ -2670,6 +2670,10 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
                         dev::rows_finalize_kernel<T, true>, dev::rows_finalize_kernel<T, false>})
         SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(dev::rows_smem<T>())));
+    for (auto kernel : {dev::close_strips_kernel<T, dev::OpCloseWeighted<true>, dev::RB, dev::RB>,
+                        dev::close_strips_kernel<T, dev::OpCloseWeighted<false>, dev::RB, dev::RB>})
+        SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(ssu::walk::kSharedMost)));
     for (const void *kernel : {reinterpret_cast<const void *>(dev::weighted_walk_kernel<T>),
                                reinterpret_cast<const void *>(dev::weighted_walk_kernel<double>)})
         SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2754,8 +2758,20 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
             launches++;
         }
         {
-            const auto close = norm ? dev::close_pairs_kernel<T, true> : dev::close_pairs_kernel<T, false>;
-            close<<<ntiles, 256, 0, s>>>(h, la, walk.len + walk.sparse0);
+            dev::CloseArgs c{};
+            c.tiles = tiles;
+            c.n_tiles = ntiles;
+            c.tables = d_tdesc;
+            c.tile_flags = d_flags;
+            c.close = d_close;
+            c.W = d_W;
+            c.len = walk.len + walk.sparse0;
+            c.n_words = walk.n_words - walk.sparse0 / 32;
+            c.out = out;
+            const auto close = norm ? dev::close_strips_kernel<T, dev::OpCloseWeighted<true>, dev::RB, dev::RB>
+                                    : dev::close_strips_kernel<T, dev::OpCloseWeighted<false>, dev::RB, dev::RB>;
+            const uint32_t strips = ntiles * dev::close_strips<dev::RB, dev::RB>();
+            close<<<std::min<uint32_t>(strips, 2 * n_sms), dev::CTHREADS, dev::close_smem(c.n_words), s>>>(c, la);
             launches++;
         }
         SSU_CK(cudaGetLastError());
@@ -2769,7 +2785,8 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
 int PlanImpl::walk_gen_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
                              uint32_t ntiles, uint32_t splits, uint32_t rows) {
     const dev::ListArgs &la = g.lists;
-    const dev::GenLaunch gl{alpha_kind(spec.alpha), spec.alpha, walk.scale, walk.len + walk.sparse0};
+    const dev::GenLaunch gl{alpha_kind(spec.alpha), spec.alpha, walk.scale, walk.len + walk.sparse0,
+                            walk.n_words - walk.sparse0 / 32, n_sms};
     if (n_sparse) {
         uint32_t n_max = 1;
         for (uint32_t t = g.t0; t < g.t1; t++) n_max = std::max(n_max, tdesc[t].n);

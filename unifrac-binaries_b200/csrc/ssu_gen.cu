@@ -17,13 +17,20 @@ void (*sums_of(int ak))(const ListArgs, const GenSums, const double *, double, d
 }
 
 template <typename T, int BM, int BN>
-void (*close_of(int ak))(const GenFinish, const ListArgs, const double *, double) {
+void (*close_of(int ak))(const CloseArgs, const ListArgs) {
     switch (ak) {
-    case 1: return gen_close_kernel<T, 1, BM, BN>;
-    case 2: return gen_close_kernel<T, 2, BM, BN>;
-    case 3: return gen_close_kernel<T, 3, BM, BN>;
-    default: return gen_close_kernel<T, 0, BM, BN>;
+    case 1: return close_strips_kernel<T, OpCloseGen<1>, BM, BN>;
+    case 2: return close_strips_kernel<T, OpCloseGen<2>, BM, BN>;
+    case 3: return close_strips_kernel<T, OpCloseGen<3>, BM, BN>;
+    default: return close_strips_kernel<T, OpCloseGen<0>, BM, BN>;
     }
+}
+
+template <typename T, int BM, int BN>
+cudaError_t close_launch(const GenLaunch &g, const ListArgs &la, const CloseArgs &c, cudaStream_t s) {
+    const uint32_t strips = c.n_tiles * close_strips<BM, BN>(), most = 2 * static_cast<uint32_t>(g.n_sms);
+    close_of<T, BM, BN>(g.ak)<<<strips < most ? strips : most, CTHREADS, close_smem(c.n_words), s>>>(c, la);
+    return cudaGetLastError();
 }
 
 template <int AK>
@@ -52,6 +59,13 @@ cudaError_t gen_configure() {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(16 * kGenCols));
             if (e != cudaSuccess) return e;
         }
+    for (int ak = 0; ak < 4; ak++)
+        for (auto kernel : {close_of<double, 128, 64>(ak), close_of<double, 64, 64>(ak), close_of<float, 128, 64>(ak),
+                            close_of<float, 64, 64>(ak)}) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(walk::kSharedMost));
+            if (e != cudaSuccess) return e;
+        }
     return cudaSuccess;
 }
 
@@ -64,14 +78,22 @@ cudaError_t gen_sums_launch(const GenLaunch &g, const ListArgs &la, const GenSum
 
 template <typename T>
 cudaError_t gen_finish_launch(const GenLaunch &g, const ListArgs &la, const GenFinish &f, bool small, cudaStream_t s) {
+    CloseArgs c{};
+    c.tiles = f.tiles;
+    c.n_tiles = f.n_tiles;
+    c.tables = f.tables;
+    c.tile_flags = f.tile_flags;
+    c.close = f.close;
+    c.len = g.len;
+    c.n_words = g.n_words;
+    c.alpha = g.alpha;
+    c.out = f.out;
     if (small) {
         gen_finalize_kernel<T, 64, 64, 4, 4><<<f.n_tiles, 256, 0, s>>>(f);
-        close_of<T, 64, 64>(g.ak)<<<f.n_tiles, 256, 0, s>>>(f, la, g.len, g.alpha);
-    } else {
-        gen_finalize_kernel<T, 128, 64, 8, 4><<<f.n_tiles, 256, 0, s>>>(f);
-        close_of<T, 128, 64>(g.ak)<<<f.n_tiles, 256, 0, s>>>(f, la, g.len, g.alpha);
+        return close_launch<T, 64, 64>(g, la, c, s);
     }
-    return cudaGetLastError();
+    gen_finalize_kernel<T, 128, 64, 8, 4><<<f.n_tiles, 256, 0, s>>>(f);
+    return close_launch<T, 128, 64>(g, la, c, s);
 }
 template cudaError_t gen_finish_launch<double>(const GenLaunch &, const ListArgs &, const GenFinish &, bool, cudaStream_t);
 template cudaError_t gen_finish_launch<float>(const GenLaunch &, const ListArgs &, const GenFinish &, bool, cudaStream_t);

@@ -18,6 +18,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "ssu_close.cuh"
 #include "ssu_kernels.cuh"
 #include "ssu_lists.cuh"
 #include "ssu_pairs.cuh"
@@ -236,40 +237,26 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gen_finalize_kernel(con
     }
 }
 
-// The close pairs again, one thread each, over the two samples' own nodes.
-template <typename T, int AK, int BM, int BN>
-__global__ void __launch_bounds__(256) gen_close_kernel(const GenFinish a, const ListArgs la,
-                                                        const double *__restrict__ len, double alpha) {
-    const uint32_t ti = blockIdx.x;
-    if (!a.tile_flags[ti]) return;
-    const uint4 tile = a.tiles[ti];
-    const TableDesc td = a.tables[tile.z];
-    OutSpec o = a.out;
-    if (o.mode == 0) o.ptr = static_cast<T *>(o.ptr) + td.out_off;
-    for (uint32_t e = threadIdx.x; e < BM * BN; e += 256) {
-        if (!((a.close[static_cast<uint64_t>(ti) * (BM * BN / 32) + e / 32] >> (e & 31)) & 1u)) continue;
-        const uint32_t kc = tile.x * BM + e / BN, lc = tile.y * BN + e % BN;
-        const uint32_t *ik = la.node + la.node_ptr[kc], *il = la.node + la.node_ptr[lc];
-        const double *uk = la.node_u + la.node_ptr[kc], *ul = la.node_u + la.node_ptr[lc];
-        const uint32_t nk = la.node_all[kc], nl = la.node_all[lc];
-        double acc[2] = {0.0, 0.0};
-        uint32_t x = 0, y = 0;
-        while (x < nk || y < nl) {
-            const uint32_t ex = x < nk ? ik[x] : 0xFFFFFFFFu, ey = y < nl ? il[y] : 0xFFFFFFFFu;
-            const double vx = ex <= ey ? uk[x] : 0.0, vy = ey <= ex ? ul[y] : 0.0;
-            OpGeneralized<double, AK>::term(acc, vx, vy, 0.0, 0.0, 0.0, len[min(ex, ey)], alpha);
-            x += ex <= ey;
-            y += ey <= ex;
-        }
-        emit_pair<T>(o, td.n, kc - td.base, lc - td.base, static_cast<T>(acc[0] / acc[1]));
+// The operator's terms, the pairs that the finalize pass marked close (close_strips_kernel).
+template <int AK>
+struct OpCloseGen {
+    static constexpr int NACC = 2;
+    __device__ static void term(double *acc, double a, double b, double L, double alpha) {
+        OpGenRows<AK>::term(acc, a, b, 0.0, 0.0, 0.0, L, alpha);
     }
-}
+    template <typename T>
+    __device__ static T value(const double *acc, const T *, uint32_t, uint32_t) {
+        return static_cast<T>(acc[0] / acc[1]);
+    }
+};
 
 // Method dispatch (ssu_gen.cu).
 struct GenLaunch {
     int ak;
     double alpha, scale;
     const double *len;  // per sparse node, then the dense nodes
+    uint32_t n_words;   // 32-bit words of a bitmap over them
+    int n_sms;
 };
 cudaError_t gen_configure();
 cudaError_t gen_sums_launch(const GenLaunch &g, const ListArgs &la, const GenSums &out, uint32_t columns, uint32_t cols,

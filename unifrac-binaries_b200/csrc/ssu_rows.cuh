@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "ssu_close.cuh"
 #include "ssu_kernels.cuh"
 #include "ssu_lists.cuh"
 
@@ -57,7 +58,7 @@ struct RowsArgs {
 // The tile's distances from its raw sums in shared memory, by the whole block.
 // A pair is close when its distance is below tau of its samples' one-sided sums,
 // where the rounding of L u (to fp64, and to half a unit in the lists) could
-// show; close_pairs_kernel sums it again.
+// show; close_strips_kernel sums it again.
 template <typename T, bool NORM>
 __device__ __forceinline__ void rows_epilogue(const RowsArgs<T> &a, uint32_t ti, double *Mt) {
     const uint4 tile = a.tiles[ti];
@@ -247,37 +248,16 @@ __global__ void __launch_bounds__(RTHREADS) rows_finalize_kernel(const RowsArgs<
     rows_epilogue<T, NORM>(a, ti, Mt);
 }
 
-// Pairs that the epilogue marked close, one thread each: sum L |u(k) - u(l)|
-// over every node in fp64, merging the two samples' lists (both in node order).
-// len: per node.
-template <typename T, bool NORM>
-__global__ void __launch_bounds__(256) close_pairs_kernel(const RowsArgs<T> a, const ListArgs la,
-                                                          const double *__restrict__ len) {
-    const uint32_t ti = blockIdx.x;
-    if (!a.tile_flags[ti]) return;
-    const uint4 tile = a.tiles[ti];
-    const TableDesc td = a.tables[tile.z];
-    OutSpec o = a.out;
-    if (o.mode == 0) o.ptr = static_cast<T *>(o.ptr) + td.out_off;
-    for (uint32_t e = threadIdx.x; e < RB * RB; e += 256) {
-        if (!((a.close[static_cast<uint64_t>(ti) * (RB * RB / 32) + e / 32] >> (e & 31)) & 1u)) continue;
-        const uint32_t kc = tile.x * RB + e / RB, lc = tile.y * RB + e % RB;
-        const uint32_t k = kc - td.base, l = lc - td.base;
-        const uint32_t *ik = la.node + la.node_ptr[kc], *il = la.node + la.node_ptr[lc];
-        const double *uk = la.node_u + la.node_ptr[kc], *ul = la.node_u + la.node_ptr[lc];
-        const uint32_t nk = la.node_all[kc], nl = la.node_all[lc];
-        double d = 0.0;
-        uint32_t x = 0, y = 0;
-        while (x < nk || y < nl) {
-            const uint32_t ex = x < nk ? ik[x] : 0xFFFFFFFFu, ey = y < nl ? il[y] : 0xFFFFFFFFu;
-            const double vx = ex <= ey ? uk[x] : 0.0, vy = ey <= ex ? ul[y] : 0.0;
-            d = fma(fabs(vx - vy), len[min(ex, ey)], d);
-            x += ex <= ey;
-            y += ey <= ex;
-        }
-        emit_pair<T>(o, td.n, k, l, NORM ? static_cast<T>(d) / (a.W[kc] + a.W[lc]) : static_cast<T>(d));
+// L |u(k) - u(l)|, the pairs that the epilogue marked close (close_strips_kernel).
+template <bool NORM>
+struct OpCloseWeighted {
+    static constexpr int NACC = 1;
+    __device__ static void term(double *acc, double a, double b, double L, double) { acc[0] = fma(fabs(a - b), L, acc[0]); }
+    template <typename T>
+    __device__ static T value(const double *acc, const T *W, uint32_t kc, uint32_t lc) {
+        return NORM ? static_cast<T>(acc[0]) / (W[kc] + W[lc]) : static_cast<T>(acc[0]);
     }
-}
+};
 
 }  // namespace dev
 }  // namespace ssu
