@@ -1011,3 +1011,53 @@ def test_a_table_of_near_duplicates_costs_little_more_than_another(ssu, method):
         best.append(min(ms))
         plan.close()
     assert best[0] < 8 * best[1], best
+
+
+# ---- digits of the list sums
+
+def _long_double_matrix(tree, table, method, alpha):
+    """Weighted and generalized distances with every step in long double."""
+    dense = table.dense()
+    row = {o: dense[i] for i, o in enumerate(table.obs_ids)}
+    counts, lengths, stack = [], [], [[]]
+    for i, o in enumerate(tree.structure):  # a node's counts when its parenthesis closes
+        if o:
+            stack.append([i, np.zeros(dense.shape[1])])
+            if not tree.structure[i + 1] and tree.names[i] in row:
+                stack[-1][1] = row[tree.names[i]].copy()
+        else:
+            at, c = stack.pop()
+            if len(stack) > 1:
+                stack[-1][1] += c
+                counts.append(c)
+                lengths.append(tree.lengths[at])
+    u = np.array(counts, dtype=np.longdouble) / dense.sum(0).astype(np.longdouble)
+    L = np.array(lengths, dtype=np.longdouble)
+    u, L = u[(u > 0).any(1)], L[(u > 0).any(1)]
+    n = dense.shape[1]
+    out = np.zeros((n, n), dtype=np.longdouble)
+    for k in range(n - 1):
+        s, d = u[:, k:k + 1] + u[:, k + 1:], np.abs(u[:, k:k + 1] - u[:, k + 1:])
+        if method.startswith("generalized"):
+            p = np.where(s > 0, np.where(s > 0, s, 1) ** np.longdouble(alpha), 0) * L[:, None]
+            num, den = (p * d / np.where(s > 0, s, 1)).sum(0), p.sum(0)
+        else:
+            num, den = (d * L[:, None]).sum(0), (s * L[:, None]).sum(0) if "_normalized" in method else np.longdouble(1)
+        out[k, k + 1:] = out[k + 1:, k] = num / den
+    return out
+
+
+@pytest.mark.parametrize("method,alpha", [("generalized_fp64", a) for a in (0.0, 0.25, 0.5, 0.75, 0.9, 1.25, 2.0)]
+                         + [("weighted_normalized_fp64", 1.0), ("weighted_unnormalized_fp64", 1.0)])
+def test_list_sums_keep_the_digits_of_direct_sums(ssu, monkeypatch, method, alpha):
+    """2-norm of the error against long double: no larger than that of the
+    embedding's form (the lists refused), give or take a rounding of the result."""
+    tree, table = _case(96, n_tips=3000, n_samples=40, density=0.3, drop=0)
+    ref = _long_double_matrix(tree, table, method, alpha)
+
+    def error():
+        got, _ = ssu.one_off_matrix(tree, table, method, alpha=alpha)
+        return np.sqrt(((got - ref) ** 2).sum() / (ref ** 2).sum())
+    lists = error()
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    assert lists <= error() + 2.0 ** -53

@@ -426,7 +426,7 @@ struct WalkLayout {
     std::vector<int32_t> kids;
     std::vector<uint32_t> level;
     std::vector<int32_t> start_of_obs;
-    double path_max = 0.0;               // longest path from the root to a tip
+    double path_max = 0.0;               // largest sparse length of a path from the root to a tip
 };
 WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const ListRule &rule, bool fp64);
 
@@ -633,6 +633,9 @@ struct PlanImpl {
     void split_rows(Group &g, const PairKernel<double> &k) const;
     template <typename T>
     int setup_walk_weighted(const TableSet &set, const FlatTree &tree);
+    template <typename T>
+    int walk_lists(cudaStream_t s, const Group &g);
+    int fit_gen_scale();
     template <typename T>
     int walk_weighted_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
                             uint32_t ntiles, uint32_t splits, bool first, bool last);
@@ -1918,7 +1921,7 @@ WalkLayout build_walk_layout(const TableSet &set, const FlatTree &tree, const Li
         const uint32_t c = static_cast<uint32_t>(col[r]);
         if (p >= 0) lay.parent[c] = col[p];
         if (r < E) lay.len[c] = fp64 ? tree.length[r] : static_cast<double>(static_cast<float>(tree.length[r]));
-        path[r] = (p >= 0 ? path[p] : 0.0) + lay.len[c];
+        path[r] = (p >= 0 ? path[p] : 0.0) + (r < E && sp.id_of_row[r] >= 0 ? lay.len[c] : 0.0);
         lay.path_max = std::max(lay.path_max, path[r]);
         const uint32_t k0 = tree.child_ptr[r], k1 = tree.child_ptr[r + 1];
         if (k1 - k0 <= 2) {
@@ -2529,15 +2532,16 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
         walk_layout.valid() ? walk_layout.get() : build_walk_layout(set, tree, list_rule, spec.fp64);
     const SparseNodes &sp = lay.sparse;
     const uint32_t n_cols = lay.n_cols;
-    // a sample's sum of L u is at most its total times the longest path
+    // a sample's sum of L u over the sparse nodes is at most its total times
+    // their largest sum along a path
     double vmax = 1.0;
     if (!spec.normalize)
         for (const Group &g : groups)
             for (double t : g.totals) vmax = std::max(vmax, t);
     double bound = lay.path_max * vmax;
-    if (walk_gen && spec.alpha < 1.0) {  // u^alpha <= 1 for proportions: at most every length
+    if (walk_gen && spec.alpha < 1.0) {  // u^alpha <= 1 for proportions: at most every sparse length
         bound = 0.0;
-        for (double L : lay.len) bound += L;
+        for (size_t i = 0; i < sp.row.size(); i++) bound += lay.len[lay.sparse0 + i];
     } else if (walk_gen) {
         // u^alpha <= u, but (u_k + u_l)^alpha <= 2^(alpha - 1) (u_k + u_l): the
         // denominator, and a term of it, reaches that many times r_k + r_l
@@ -2678,16 +2682,17 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
                                reinterpret_cast<const void *>(dev::weighted_walk_kernel<double>)})
         SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(ssu::walk::kSharedMost)));
+    if (walk_gen) {
+        if (const int rc = fit_gen_scale()) return rc;
+    }
     tuning = "sample lists";
     timer.step("walk_buffers");
     return 0;
 }
 
-// One group: the walk (dense rows, lists, one-sided sums), the sparse nodes'
-// shared sums, the dense tile kernel (+ split finalize), then the close pairs.
+// One group's walk: dense rows, lists, one-sided sums.
 template <typename T>
-int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
-                                  uint32_t ntiles, uint32_t splits, bool first, bool last) {
+int PlanImpl::walk_lists(cudaStream_t s, const Group &g) {
     if (const int rc = reset_lists(s, g)) return rc;
     const dev::ListArgs &la = g.lists;
     dev::WalkArgs w = walk;
@@ -2714,6 +2719,40 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
         launches++;
     }
     SSU_CK(cudaGetLastError());
+    return 0;
+}
+
+// The generalized lists' unit from the samples' own sums r_k over the sparse
+// nodes (one walk with the unit that every table allows, when the plan is made):
+// as s^alpha <= 2^max(alpha - 1, 0) (u_k^alpha + u_l^alpha), a pair's denominator is at
+// most that many times r_k + r_l.  (The unit by the lengths alone left the error
+// of alpha 0.75 at 13 times that of the direct sums, alpha 2 at 1.5 times.)
+int PlanImpl::fit_gen_scale() {
+    if (!n_sparse) return 0;
+    unsigned long long most = 0;
+    for (const Group &g : groups) {
+        if (const int rc = walk_lists<double>(stream, g)) return rc;
+        std::vector<unsigned long long> rs(g.ld);
+        SSU_CK(cudaMemcpyAsync(rs.data(), g.lists.rs, sizeof(unsigned long long) * g.ld, cudaMemcpyDeviceToHost, stream));
+        SSU_CK(cudaStreamSynchronize(stream));
+        for (unsigned long long r : rs) most = std::max(most, r);
+    }
+    // (each node's q was rounded by up to half a unit)
+    const double units = (static_cast<double>(most) + n_sparse) * (1.0 + 1e-9) * std::pow(2.0, std::max(spec.alpha, 1.0));
+    int x = 0;
+    std::frexp(units, &x);  // 2^max(alpha, 1) r_k < 2^x units
+    walk.scale = std::ldexp(walk.scale, std::max(0, std::min(63 - x, 40)));
+    walk_unit = 1.0 / walk.scale;
+    return 0;
+}
+
+// One group: the walk, the sparse nodes' shared sums, the dense tile kernel (+
+// split finalize), then the close pairs.
+template <typename T>
+int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
+                                  uint32_t ntiles, uint32_t splits, bool first, bool last) {
+    if (const int rc = walk_lists<T>(s, g)) return rc;
+    const dev::ListArgs &la = g.lists;
     if (first && timed()) SSU_CK(cudaEventRecord(ev[1], s));
     if (ntiles && walk_gen) {
         if (const int rc = walk_gen_stage(s, g, out, tiles, ntiles, g.splits, g.rows_per_split)) return rc;
