@@ -1061,3 +1061,18 @@ def test_list_sums_keep_the_digits_of_direct_sums(ssu, monkeypatch, method, alph
     lists = error()
     monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
     assert lists <= error() + 2.0 ** -53
+
+
+@pytest.mark.parametrize("method,alpha", [("generalized_fp64", 0.0), ("generalized_fp64", 0.5), ("weighted_normalized_fp64", 1.0)])
+def test_list_sums_of_near_duplicates_keep_the_digits_of_direct_sums(ssu, monkeypatch, method, alpha):
+    """The same on near duplicates, some pairs below the bound under which they are
+    summed again and some above; give or take two roundings of the result."""
+    tree, table = _all_near(97, 96, 2000, 0.05)
+    ref = _long_double_matrix(tree, table, method, alpha)
+
+    def error():
+        got, _ = ssu.one_off_matrix(tree, table, method, alpha=alpha)
+        return np.sqrt(((got - ref) ** 2).sum() / (ref ** 2).sum())
+    lists = error()
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    assert lists <= error() + 2.0 ** -52

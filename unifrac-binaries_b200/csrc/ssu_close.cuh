@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(CTHREADS, 2) close_strips_kernel(const CloseAr
             }
             __syncthreads();
             for (uint32_t w = 0; w < a.n_words;) {
-                // the next words with up to CROWS marked nodes, by the first warp
+                // the next words with up to CROWS marked nodes, by the first warp; the others clear the rows
                 if (warp == 0) {
                     uint32_t n = 0, nw = 0;
                     for (bool more = true; more;) {
@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(CTHREADS, 2) close_strips_kernel(const CloseAr
                         chunk_words = nw;
                         chunk_rows = n;
                     }
+                } else {
+                    for (int x = tid - 32; x < CROWS * LD; x += CTHREADS - 32) V[x] = 0.0;
                 }
                 __syncthreads();
                 const uint32_t nw = chunk_words, n = chunk_rows;  // (nw >= 2: a word has 32 nodes at most)
@@ -171,8 +173,6 @@ __global__ void __launch_bounds__(CTHREADS, 2) close_strips_kernel(const CloseAr
                     const uint32_t m = w + x / 32 < a.n_words ? bits[w + x / 32] : 0u, b = x & 31;
                     if ((m >> b) & 1u) row_len[base_s[x / 32] + __popc(m & ((1u << b) - 1u))] = a.len[w * 32 + x];
                 }
-                for (uint32_t x = tid; x < n * LD; x += CTHREADS) V[x] = 0.0;
-                __syncthreads();
                 const uint32_t end = (w + nw) * 32;
                 constexpr int U = 6;  // samples of a warp with loads in flight
                 for (uint32_t i0 = warp; i0 < who; i0 += WARPS * U) {
@@ -220,6 +220,8 @@ __global__ void __launch_bounds__(CTHREADS, 2) close_strips_kernel(const CloseAr
                 }
                 __syncthreads();
                 if (busy) {
+                    // (the chunk's terms apart, so that no sum runs over more than CROWS)
+                    double part[TM][TN][Op::NACC] = {};
                     const double *row = V;
                     for (uint32_t r = 0; r < n; r++, row += LD) {
                         const double L = row_len[r];
@@ -231,8 +233,14 @@ __global__ void __launch_bounds__(CTHREADS, 2) close_strips_kernel(const CloseAr
 #pragma unroll
                         for (int i = 0; i < TM; i++)
 #pragma unroll
-                            for (int j = 0; j < TN; j++) Op::term(acc[i][j], ak[i], bl[j], L, a.alpha);
+                            for (int j = 0; j < TN; j++) Op::term(part[i][j], ak[i], bl[j], L, a.alpha);
                     }
+#pragma unroll
+                    for (int i = 0; i < TM; i++)
+#pragma unroll
+                        for (int j = 0; j < TN; j++)
+#pragma unroll
+                            for (int c = 0; c < Op::NACC; c++) acc[i][j][c] += part[i][j][c];
                 }
                 w += nw;
                 __syncthreads();  // the next chunk's words and rows lie over these

@@ -2779,7 +2779,12 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
         h.S = d_Sq;
         h.rs = la.rs;
         h.unit = walk_unit;
-        h.tau = 0.02;
+        // fp64: at 0.005 the roundings of L u and of the lists' unit leave the error of
+        // near duplicates where the embedding's is (2-norm against long double, counts
+        // with 0.1 to 3% noise: 0.5 to 1.3 times; at 0.02 1.0 to 1.3, at 0.002 0.6 to
+        // 1.5); 700 of them on 5,000 tips take 0.52 ms (0.60 at 0.02, 0.35 at
+        // 0.002).  Rows in single precision want the wider bound.
+        h.tau = spec.fp64 ? 0.005 : 0.02;
         h.tile_flags = d_flags;
         h.close = d_close;
         h.partial = h.n_splits > 1 ? d_hpartial : nullptr;
@@ -2866,7 +2871,9 @@ int PlanImpl::walk_gen_stage(cudaStream_t s, const Group &g, const dev::OutSpec 
     f.rs = la.rs;
     f.W = static_cast<const double *>(d_W);
     f.unit = walk_unit;
-    f.tau = 0.02;
+    // (errors of near duplicates 0.5 to 1.2 times the direct form's, at 0.02 0.9 to
+    // 2.6 times; 700 of them on 5,000 tips 1.20 ms, at 0.02 1.48 ms)
+    f.tau = 0.005;
     f.tile_flags = d_flags;
     f.close = d_close;
     f.out = out;
