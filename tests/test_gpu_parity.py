@@ -1076,3 +1076,23 @@ def test_list_sums_of_near_duplicates_keep_the_digits_of_direct_sums(ssu, monkey
     lists = error()
     monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
     assert lists <= error() + 2.0 ** -52
+
+
+def test_fp32_rows_keep_the_digits_of_the_embedding(ssu, monkeypatch):
+    """Single precision, samples of 10 to a million reads: the error against long
+    double is no larger than that of the embedding's form."""
+    tree = ssu_synth.random_binary_tree(2000, 0.1, 98)
+    rng = np.random.default_rng(98)
+    dense = np.exp(2 + 1.5 * rng.standard_normal((2000, 96))) * 10 ** rng.uniform(0, 4, 96)
+    dense = np.where(rng.random(dense.shape) < 0.03, np.round(dense) + 1, 0.0)
+    dense[0] += 1.0
+    table = ssu_synth.Table.from_dense(dense, tree.tip_names(), ["S%d" % j for j in range(96)])
+    ref = _long_double_matrix(tree, table, "weighted_unnormalized", 1.0)
+    monkeypatch.setenv("UNIFRAC_B200_DETERMINISTIC", "1")
+
+    def error():
+        got = ssu.one_off_matrix(tree, table, "weighted_unnormalized")[0].astype(np.longdouble)
+        return np.sqrt(((got - ref) ** 2).sum() / (ref ** 2).sum())
+    lists = error()
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    assert lists <= error()
