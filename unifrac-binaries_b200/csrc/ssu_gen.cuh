@@ -31,8 +31,9 @@ namespace dev {
 // eight uneven tables took 4.45 ms, with this 1.89 ms): the single-precision
 // approximation y, and one step of Householder's third-order iteration for
 // y^-2 = s,  y (1 + e / 2 + 3 e^2 / 8) with e = 1 - s y^2.  e is at most 2^-21, the
-// step's own error 5 e^3 / 16 below 2^-64; the roundings leave about 1.5 units
-// in the last place.
+// step's own error 5 e^3 / 16 below 2^-64; the roundings leave at most 0.99 and on
+// average 0.28 units in the last place on a million values (rsqrt: up to 1).  With
+// y^2 first, which is exact, 0.50 and 0.25, but the dense rows take 3% longer and the distances' error stays.
 __device__ __forceinline__ double rsqrt_step(double s) {
     float f;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(static_cast<float>(s)));
@@ -44,7 +45,9 @@ __device__ __forceinline__ double rsqrt_step(double s) {
 // by the power of two that takes s to [1, 2) (a denormal s to 2^-51 or more), as
 // s may be far below the range of a single, and 1 / s is its single-precision
 // approximation (relative error e below 2^-22) and Newton's iteration to third order,
-// y (1 + e + e^2): error e^3 < 2^-66.
+// y (1 + e + e^2): error e^3 < 2^-66; at most 1.44 and on average 0.34 units in the
+// last place on a million pairs.  (The remainder in one more step takes that to 0.50
+// and 0.25, and 5% longer; the distances' error stays.)
 __device__ __forceinline__ double ratio_step(double d, double s) {
     const double up = __hiloint2double(0x7fe00000 - (__double2hiint(s) & 0x7ff00000), 0);
     const double ss = fma(s, up, 1e-37);
