@@ -1096,3 +1096,33 @@ def test_fp32_rows_keep_the_digits_of_the_embedding(ssu, monkeypatch):
     lists = error()
     monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
     assert lists <= error()
+
+
+# ---- lengths and counts far below the largest
+
+@pytest.mark.parametrize("scale", [1e-6, 1e-11, 1e-30])
+@pytest.mark.parametrize("method,alpha", [("unweighted_fp64", 1.0), ("unweighted_unnormalized_fp64", 1.0),
+                                          ("weighted_normalized_fp64", 1.0), ("weighted_unnormalized_fp64", 1.0),
+                                          ("generalized_fp64", 0.0), ("generalized_fp64", 0.5), ("generalized_fp64", 1.5)])
+def test_samples_in_a_clade_of_short_branches(ssu, oracle_mod, method, alpha, scale):
+    """Every third sample has only tips of a clade whose branches are 1e-6 to 1e-30
+    of the others': few or no units of the fixed point that the table's largest sample sets."""
+    tree, table = _case(99, n_tips=300, n_samples=70, density=0.3, drop=0)
+    # the first child of the root, its parenthesis and the tips inside
+    depth, end = 0, 1
+    for end in range(1, len(tree.structure)):
+        depth += 1 if tree.structure[end] else -1
+        if depth == 0:
+            break
+    tree.lengths = tree.lengths.copy()
+    tree.lengths[1:end] *= scale
+    inside = np.array([1 < tree.names.index(o) < end for o in table.obs_ids])
+    dense = table.dense()
+    dense[np.ix_(~inside, np.arange(70) % 3 == 0)] = 0.0
+    dense[np.flatnonzero(inside)[0]] += 2.0
+    table = ssu_synth.Table.from_dense(dense, table.obs_ids, table.sample_ids)
+    got = ssu.one_off_matrix(tree, table, method, alpha=alpha)[0]
+    ref = oracle_mod.oracle_one_off(tree, table, method, alpha=alpha)["matrix"]
+    assert np.all(np.isfinite(ref))
+    off = np.abs(got - ref) / np.where(ref == 0, 1.0, ref)
+    assert off.max() <= FP64_REL, off.max()

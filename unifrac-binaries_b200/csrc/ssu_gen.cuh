@@ -11,8 +11,8 @@
 // the sample lists as whole numbers of a fixed-point unit, the one-sided parts
 // by the same rounding, so both differences are exact (modulo 2^64: the brackets may be
 // negative for alpha > 1); the other nodes are summed for every pair by
-// the dense kernel.  Pairs whose numerator is below tau of r_k + r_l are
-// summed again over their own nodes.  Terms are fp64 for both precisions.
+// the dense kernel.  Pairs whose numerator is below tau of r_k + r_l, and those
+// whose r_k + r_l is few units, are summed again over their own nodes.  Terms are fp64 for both precisions.
 #pragma once
 
 #include <cstdint>
@@ -230,7 +230,8 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gen_finalize_kernel(con
                 n += static_cast<double>(static_cast<long long>(own - a.num[at])) * a.unit;
                 d += static_cast<double>(static_cast<long long>(own - a.den[at])) * a.unit;
             }
-            if (n < a.tau * (wk + a.W[td.base + l])) {
+            const double w = wk + a.W[td.base + l];
+            if (n < a.tau * w || (a.num && w < kSharedLeast * a.unit)) {
                 const uint32_t e = static_cast<uint32_t>(row * BN + col);
                 atomicOr(a.close + static_cast<uint64_t>(ti) * (BM * BN / 32) + e / 32, 1u << (e & 31));
                 a.tile_flags[ti] = 1;

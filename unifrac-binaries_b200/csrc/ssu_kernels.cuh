@@ -953,6 +953,11 @@ static __global__ void build_nibbles_kernel(const unsigned long long *__restrict
 // the half unit that each length was rounded by could show: its tile is
 // flagged and recomputed in the stripe form over every node.
 constexpr double kSharedTau = 0.02;
+// So it could where the two samples' lengths are this few units, which the
+// table's largest sample sets: 2^14 of what that one has at most (a clade of
+// branches far below the others').  A pair of m nodes is off by about
+// sqrt(m / 12) units: 1e-14 at 100 nodes.
+constexpr double kSharedLeast = 0x1p48;
 
 template <bool NORMALIZED, int BM, int BN, int TM, int TN>
 __device__ __forceinline__ void shared_bits_epilogue(const PairArgs<double> &a, uint32_t ti, int tx, int ty,
@@ -982,7 +987,7 @@ __device__ __forceinline__ void shared_bits_epilogue(const PairArgs<double> &a, 
             if (!(k < l && l < td.n)) continue;
             const unsigned long long own = rk + rl[j], sh = acc[i][j] + (row ? row[l] : 0ull);
             const double x = static_cast<double>(own - 2 * sh);
-            close = close || x < kSharedTau * static_cast<double>(own);
+            close = close || x < kSharedTau * static_cast<double>(own) || static_cast<double>(own) < kSharedLeast;
             emit_pair<double>(o, td.n, k, l, NORMALIZED ? x / static_cast<double>(own - sh) : x * unit);
         }
     }

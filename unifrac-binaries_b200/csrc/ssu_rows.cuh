@@ -57,7 +57,7 @@ struct RowsArgs {
 
 // The tile's distances from its raw sums in shared memory, by the whole block.
 // A pair is close when its distance is below tau of its samples' one-sided sums,
-// where the rounding of L u (to fp64, and to half a unit in the lists) could
+// or these are few units, where the rounding of L u (to fp64, and to half a unit in the lists) could
 // show; close_strips_kernel sums it again.
 template <typename T, bool NORM>
 __device__ __forceinline__ void rows_epilogue(const RowsArgs<T> &a, uint32_t ti, double *Mt) {
@@ -76,6 +76,7 @@ __device__ __forceinline__ void rows_epilogue(const RowsArgs<T> &a, uint32_t ti,
         wl[i] = l < td.n ? a.W[td.base + l] : T(0);
     }
     bool any = false;
+    const double least = (sizeof(T) == 8 ? kSharedLeast : 0x1p30) * a.unit;
     constexpr int G = 4;  // rows of a warp whose shared sums are in flight together
     for (int r0 = warp; r0 < RB; r0 += RWARPS * G) {
         unsigned long long sh[G][4], rk[G];
@@ -103,7 +104,7 @@ __device__ __forceinline__ void rows_epilogue(const RowsArgs<T> &a, uint32_t ti,
                 const unsigned long long own = rk[u] + rl[i];
                 const double d = x + static_cast<double>(own - 2 * sh[u][i]) * a.unit;
                 const T w = wk[u] + wl[i];
-                const bool close = on && d < a.tau * static_cast<double>(w);
+                const bool close = on && (d < a.tau * static_cast<double>(w) || static_cast<double>(w) < least);
                 const T v = NORM ? static_cast<T>(d) / w : static_cast<T>(d);
                 if (on && o.mode == 0) {
                     static_cast<T *>(o.ptr)[static_cast<uint64_t>(k) * td.n + l] = v;
