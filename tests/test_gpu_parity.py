@@ -1098,7 +1098,7 @@ def test_fp32_rows_keep_the_digits_of_the_embedding(ssu, monkeypatch):
     assert lists <= error()
 
 
-# ---- lengths and counts far below the largest
+# ---- lengths and counts far below the largest, and sums out of range
 
 @pytest.mark.parametrize("scale", [1e-6, 1e-11, 1e-30])
 @pytest.mark.parametrize("method,alpha", [("unweighted_fp64", 1.0), ("unweighted_unnormalized_fp64", 1.0),
@@ -1126,3 +1126,14 @@ def test_samples_in_a_clade_of_short_branches(ssu, oracle_mod, method, alpha, sc
     assert np.all(np.isfinite(ref))
     off = np.abs(got - ref) / np.where(ref == 0, 1.0, ref)
     assert off.max() <= FP64_REL, off.max()
+
+
+@pytest.mark.parametrize("method", ["unweighted_fp64", "weighted_unnormalized_fp64"])
+def test_sums_out_of_range_stay_on_the_embedding(ssu, monkeypatch, method):
+    """Lengths of 1e306 whose sum is not finite, raw counts: as with the lists refused."""
+    tree, table = _case(100, n_tips=300, n_samples=40, density=0.2)
+    tree.lengths = np.where(tree.lengths > 0, 1e306, 0.0)
+    call = lambda: ssu.one_off_matrix(tree, table, method, normalize=False)[0]  # noqa: E731
+    got = call()
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    np.testing.assert_array_equal(got, call())

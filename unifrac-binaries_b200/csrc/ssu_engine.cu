@@ -3141,13 +3141,17 @@ bool use_tensor_cores(const MethodSpec &spec, const TableSet &set, const FlatTre
 }
 
 // What the walks over each sample's tips need: counts and lengths that are not
-// negative and finite (a node is then present where some tip below has a
-// count), one length per node for all tables, one tip per observation, and
+// negative and finite, also in sum (a node is then present where some tip below has a
+// count, and a fixed point can hold a sample's sums), one length per node for all tables, one tip per observation, and
 // `bits` bits of shared memory per node.
 bool can_walk(const TableSet &set, const FlatTree &tree, uint64_t bits) {
     if (!set.row_active.empty() || (tree.n_nodes + 2048) * bits / 8 > tc::MAX_BITMAP_BYTES - 16 * 1024) return false;
-    for (uint32_t e = 0; e < tree.n_nodes; e++)
-        if (!(tree.length[e] >= 0.0 && std::isfinite(tree.length[e]))) return false;
+    double sum = 0.0;
+    for (uint32_t e = 0; e < tree.n_nodes; e++) {
+        if (!(tree.length[e] >= 0.0)) return false;
+        sum += tree.length[e];
+    }
+    if (!std::isfinite(sum)) return false;
     for (const Table *t : set.tables) {
         if (!t->nonneg) return false;
         for (double x : t->totals)
@@ -3190,6 +3194,12 @@ bool use_walk_weighted(const MethodSpec &spec, const TableSet &set, const FlatTr
     } else {
         return false;
     }
+    double most = 1.0, all = 0.0;
+    if (!spec.normalize)
+        for (const Table *t : set.tables)
+            for (double x : t->totals) most = std::max(most, x);
+    for (uint32_t e = 0; e < tree.n_nodes; e++) all += tree.length[e];
+    if (!std::isfinite(4.0 * most * all)) return false;
     // an explicit zero of a sample without counts is 0 / 0, and its distances
     // are NaN: the embedding's business
     if (spec.normalize)
