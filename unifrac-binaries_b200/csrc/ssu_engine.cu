@@ -2239,8 +2239,9 @@ int PlanImpl::setup_gemm(const TableSet &set, const FlatTree &tree) {
     }
     // the same limit for every plan: the attribute is the kernel's, not the
     // plan's, so a plan's own size would refuse the launches of other plans
-    SSU_CK(cudaFuncSetAttribute(tc::presence_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(tc::MAX_BITMAP_BYTES)));
+    for (auto kernel : {tc::presence_rows_kernel<true>, tc::presence_rows_kernel<false>})
+        SSU_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(tc::MAX_BITMAP_BYTES)));
     SSU_CK(alloc(&d_full, (spec.fp64 ? sizeof(double) : sizeof(float)) * std::max<uint64_t>(full_elems, 1)));
     SSU_CK(cudaStreamSynchronize(stream));
     timer.step("gemm_buffers");
@@ -2422,7 +2423,8 @@ int PlanImpl::gemm_rows(cudaStream_t s, const Group &g) {
             SSU_CK(cudaMemcpyAsync(la.part_count + (p - 1) * la.slots, la.count, sizeof(uint32_t) * la.slots,
                                    cudaMemcpyDeviceToDevice, s));
         if (c1 <= c0) continue;
-        tc::presence_rows_kernel<<<c1 - c0, 256, bits_smem, s>>>(
+        const auto kernel = n_sparse ? tc::presence_rows_kernel<true> : tc::presence_rows_kernel<false>;
+        kernel<<<c1 - c0, 256, bits_smem, s>>>(
             g.d_sample_ptr, g.d_start_col, d_parent_col, d_lq, d_lsorted, static_cast<uint32_t>(g.ld), k_pad,
             static_cast<uint64_t>(n_pad) * k_pad, d_A, d_B, d_r, n_sparse ? g.d_columns + c0 : nullptr, la);
         launches++;

@@ -607,8 +607,12 @@ __global__ void __launch_bounds__(1024) exclusive_scan_kernel(const uint32_t *__
 // 16 bytes per store; A1 and B1 `plane` bytes after A0 and B0), and
 // r = sum L of the present nodes (fp64, fixed reduction order), and the
 // sample's entries of the sparse nodes' lists.  lq holds the node digits u,
-// s, v, t: digit i at lq + i * k_pad.
-__global__ void __launch_bounds__(256)
+// s, v, t: digit i at lq + i * k_pad.  Without sparse nodes (LISTS false) eight
+// blocks to an SM: the lists' registers leave room for five (3,440 samples on
+// 5,482 tips: 65 us so, 53 us with an instance of its own).  With lists five:
+// 6,241 samples on 5,190 tips take 708, 675, 687, 699 us at four, five, six, eight.
+template <bool LISTS>
+__global__ void __launch_bounds__(256, LISTS ? 5 : 8)
     presence_rows_kernel(const uint32_t *__restrict__ sample_ptr, const int32_t *__restrict__ start_col,
                          const int32_t *__restrict__ parent_col, const uint8_t *__restrict__ lq,
                          const double *__restrict__ l_sorted, uint32_t n, uint32_t k_pad, uint64_t plane,
@@ -617,7 +621,7 @@ __global__ void __launch_bounds__(256)
     extern __shared__ uint32_t bits[];  // k_pad / 32 words, then the sparse nodes'
     __shared__ double red[256];
     const uint32_t j = column ? column[blockIdx.x] : blockIdx.x;
-    const uint32_t sp_words = (la.n_nodes + 31) / 32;
+    const uint32_t sp_words = LISTS ? (la.n_nodes + 31) / 32 : 0;
     const uint32_t words = k_pad / 32 + sp_words;
     for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) bits[w] = 0u;
     __syncthreads();
@@ -647,7 +651,7 @@ __global__ void __launch_bounds__(256)
         for (int t = 0; t < 16; t++)
             if ((b >> t) & 1u) part += l_sorted[c16 + t];
     }
-    if (la.n_nodes) dev::write_lists(la, j, bits + k_pad / 32, sp_words, l_sorted + k_pad, 0ull, part);
+    if constexpr (LISTS) dev::write_lists(la, j, bits + k_pad / 32, sp_words, l_sorted + k_pad, 0ull, part);
     red[threadIdx.x] = part;
     __syncthreads();
     if (threadIdx.x == 0) {
