@@ -119,6 +119,15 @@ static __global__ void fixed_lengths_kernel(const double *__restrict__ len, uint
 constexpr int WALKS = 4;
 static __device__ __forceinline__ void mark_paths(const int32_t *__restrict__ start, uint32_t n,
                                                   const int32_t *__restrict__ parent, uint32_t *bits) {
+    if (n <= blockDim.x) {  // one path a thread: nothing beside it in a step
+        int32_t c = threadIdx.x < n ? start[threadIdx.x] : -1;
+        while (c >= 0) {
+            const uint32_t m = 1u << (c & 31);
+            const int32_t up = parent[c];
+            c = atomicOr(&bits[c >> 5], m) & m ? -1 : up;
+        }
+        return;
+    }
     for (uint32_t e = threadIdx.x; e < n; e += WALKS * blockDim.x) {
         int32_t c[WALKS];
 #pragma unroll
