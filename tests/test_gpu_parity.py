@@ -1137,3 +1137,18 @@ def test_sums_out_of_range_stay_on_the_embedding(ssu, monkeypatch, method):
     got = call()
     monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
     np.testing.assert_array_equal(got, call())
+
+
+@pytest.mark.parametrize("alpha", [0.0, 0.5, 1.0, 1.5])
+def test_fp32_generalized_keeps_the_digits_of_the_union_form(ssu, monkeypatch, alpha):
+    """Single precision: the error against long double is no larger than the union
+    kernel's over the embedding, whose sums are fp64 (alpha 1 too)."""
+    tree, table = _case(101, n_tips=1500, n_samples=60, density=0.05, drop=0)
+    ref = _long_double_matrix(tree, table, "generalized", alpha)
+
+    def error():
+        got = ssu.one_off_matrix(tree, table, "generalized", alpha=alpha)[0].astype(np.longdouble)
+        return np.sqrt(((got - ref) ** 2).sum() / (ref ** 2).sum())
+    lists = error()
+    monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
+    assert lists <= error()

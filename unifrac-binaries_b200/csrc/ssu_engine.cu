@@ -618,7 +618,7 @@ struct PlanImpl {
     // tile kernel over their rows alone
     bool walk_weighted = false;
     // generalized UniFrac the same way, over the nodes that both samples have
-    // (alpha 1 is weighted normalized); walk_weighted too
+    // (alpha 1 in fp64 is weighted normalized); walk_weighted too
     bool walk_gen = false;
     bool gen_small = false;                 // 64 x 64 tiles
     unsigned long long *d_gen_num = nullptr, *d_gen_den = nullptr;
@@ -3223,7 +3223,9 @@ int PlanImpl::build(const TableSet &set, const FlatTree &tree, const BatchOption
     gemm = use_tensor_cores(spec, set, tree, batch);
     walk_bits = use_lists && !gemm && use_walk_bits(spec, set, tree);
     walk_weighted = use_lists && use_walk_weighted(spec, set, tree);
-    walk_gen = walk_weighted && spec.method == Method::generalized && spec.alpha != 1.0;
+    // (alpha 1 is weighted normalized, but in single precision the generalized form's
+    // sums are fp64 and rounded once, as the union kernel's were)
+    walk_gen = walk_weighted && spec.method == Method::generalized && (spec.alpha != 1.0 || !spec.fp64);
     if (gemm) start_gemm_layout(set, tree);
     if (walk_weighted) start_walk_layout(set, tree);
     if (const int rc = setup(set, tree, opts)) return rc;
