@@ -1152,3 +1152,42 @@ def test_fp32_generalized_keeps_the_digits_of_the_union_form(ssu, monkeypatch, a
     lists = error()
     monkeypatch.setenv("UNIFRAC_B200_TEST_LIST_MEMORY", "1")
     assert lists <= error()
+
+
+def _duplicates(seed, n, n_tips, density, copies=2):
+    """Samples in random order, each with a duplicate (`copies` 1: none) that lacks one of its features half of the time."""
+    tree = ssu_synth.random_binary_tree(n_tips, 0.1, seed)
+    rng = np.random.default_rng(seed)
+    dense = np.where(rng.random((n_tips, n // copies)) < density, rng.geometric(0.1, (n_tips, n // copies)), 0).astype(float)
+    dense[0] = 1.0
+    dense = np.tile(dense, (1, copies))
+    for j in range(n // 2, n, 2):
+        dense[rng.choice(np.flatnonzero(dense[1:, j])) + 1, j] = 0.0
+    dense = dense[:, rng.permutation(n)]
+    return tree, ssu_synth.Table.from_dense(dense, tree.tip_names(), ["S%d" % j for j in range(n)])
+
+
+@pytest.mark.parametrize("n,n_tips", [(40, 300), (150, 900), (700, 2500)])
+def test_whole_number_unweighted_of_duplicated_samples(ssu, monkeypatch, n, n_tips):
+    tree, table = _duplicates(n, n, n_tips, 0.05)
+    for method in ("unweighted_fp64", "unweighted_unnormalized_fp64"):
+        call = lambda: ssu.one_off_matrix(tree, table, method)[0]  # noqa: E731
+        check_fp64(call(), _stripe_mode(monkeypatch, call))
+
+
+def test_duplicated_samples_cost_little_more_than_others(ssu):
+    """600 samples, each with a duplicate, against 600 different ones: less than
+    twice as long (with every tile of a duplicate in the stripe form over ten times)."""
+    best = []
+    for copies in (2, 1):
+        tree, table = _duplicates(12, 600, 6000, 0.03, copies)
+        plan = ssu.Plan(tree, table, "unweighted_fp64")
+        plan.set_timing(True)
+        ms = []
+        for _ in range(5):
+            plan.execute()
+            plan.result()
+            ms.append(sum(plan.stage_ms()))
+        best.append(min(ms))
+        plan.close()
+    assert best[0] < 2 * best[1], best

@@ -646,7 +646,7 @@ struct PlanImpl {
     uint32_t n_words_all = 0;
     double *d_len_cols = nullptr;
     unsigned long long *d_nib = nullptr;  // nibble sums of the dense nodes' words
-    PairKernel<double> k_stripe;          // the stripe form, for the tiles that the whole-number form flags
+    decltype(SharedBits::again) xor_again = nullptr;  // sums the pairs again that the whole-number form marks
     ListRule bits_list_rule(const TableSet &set) const;
     int setup_walk_bits(const TableSet &set, const FlatTree &tree);
     int walk_bits_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles, uint32_t ntiles,
@@ -2304,7 +2304,8 @@ int PlanImpl::setup_lists(const TableSet &set, const FlatTree &tree, const Spars
     sparse_unit = 1.0 / sp.scale;
     if (!n_sparse && !path && !walk_weighted) return setup_sample_lists(set, start_of_obs);
     SSU_CK(alloc(&d_sparse_q, sizeof(unsigned long long) * n));
-    SSU_CK(alloc(&d_list_unit, sizeof(double)));
+    SSU_CK(alloc(&d_list_unit, 2 * sizeof(double)));
+    SSU_CK(cudaMemsetAsync(d_list_unit, 0, 2 * sizeof(double), stream));
     double *d_path = nullptr;
     if (path) SSU_CK(upload(&d_path, path->data(), sizeof(double) * path->size()));
     for (Group &g : groups) {
@@ -2932,18 +2933,15 @@ int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     timer.step("bits_layout");
     uint64_t big_tiles = 0;  // 128 x 64 tiles of the upper triangles
     for (const dev::TableDesc &d : tdesc) big_tiles += static_cast<uint64_t>((d.n + 127) / 128) * ((d.n + 127) / 128 + 1);
-    const SharedBitsPair pair =
-        shared_bits_pair(spec.method == Method::unweighted, big_tiles < static_cast<uint64_t>(n_sms));
-    kd = pair.shared;
-    k_stripe = pair.stripe;
-    for (PairKernel<double> *k : {&kd, &k_stripe}) {
-        int bps = 0;
-        if (k->configure(k->smem) != cudaSuccess || k->occupancy(&bps, k->threads, k->smem) != cudaSuccess || bps < 1) {
-            last_error = "pair kernel does not fit on the device";
-            return kOutputError;
-        }
-        k->blocks_per_sm = bps;
+    const SharedBits form = shared_bits(spec.method == Method::unweighted, big_tiles < static_cast<uint64_t>(n_sms));
+    kd = form.pair;
+    xor_again = form.again;
+    int bps = 0;
+    if (kd.configure(kd.smem) != cudaSuccess || kd.occupancy(&bps, kd.threads, kd.smem) != cudaSuccess || bps < 1) {
+        last_error = "pair kernel does not fit on the device";
+        return kOutputError;
     }
+    kd.blocks_per_sm = bps;
     const PairKernel<double> &k = kd;
     uint32_t max_tiles = 1;
     for (Group &g : groups) {
@@ -2958,21 +2956,17 @@ int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
     }
     if (partial_bytes) SSU_CK(alloc(&d_partial, partial_bytes));
     SSU_CK(alloc(&d_flags, sizeof(int) * max_tiles));
+    const size_t marks = sizeof(uint32_t) * (static_cast<size_t>(k.BM) * k.BN / 32) * max_tiles;
+    SSU_CK(alloc(&d_close, marks));
+    SSU_CK(cudaMemsetAsync(d_close, 0, marks, stream));  // (a pass leaves them so)
     SSU_CK(upload(&d_parent_col, parent.data(), sizeof(int32_t) * n_cols));
     SSU_CK(upload(&d_len_cols, len.data(), sizeof(double) * n_cols));
     if (const int rc = setup_lists(set, tree, sp, d_len_cols, n_cols, first, &path, path_starts(tree, col)))
         return rc;
     timer.step("bits_lists");
-    lut_stride = 0;
     SSU_CK(alloc(&d_nib, sizeof(unsigned long long) * dev::NIB_TABLE * std::max(n_words, 1u)));
     if (n_words) dev::build_nibbles_kernel<<<n_words, dev::NIB_TABLE, 0, stream>>>(d_sparse_q, n_words, d_nib);
     SSU_CK(alloc(&d_P, sizeof(unsigned long long) * ld * std::max(n_words_all, 1u)));
-    SSU_CK(alloc(&d_lut, sizeof(double) * 2048 * std::max(n_words_all, 1u)));
-    if (n_words_all) {
-        dev::build_lut_kernel<double><<<dim3(n_words_all * 8, 1), 256, 0, stream>>>(d_len_cols, n_cols,
-                                                                                   static_cast<double *>(d_lut), 0, 0);
-        SSU_CK(cudaGetLastError());
-    }
     SSU_CK(alloc(&d_full, sizeof(double) * std::max<uint64_t>(full_elems, 1)));
     d_shared = static_cast<unsigned long long *>(d_full);  // a pair's sum is read before its distance is written
     SSU_CK(cudaFuncSetAttribute(dev::presence_words_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2983,8 +2977,8 @@ int PlanImpl::setup_walk_bits(const TableSet &set, const FlatTree &tree) {
 }
 
 // One group: the walk (presence words, lists), the sparse nodes' shared sums,
-// the presence-word kernel over the dense words, then over every word on the
-// tiles it flagged.
+// the presence-word kernel over the dense words, then the pairs it marked over
+// every word.
 int PlanImpl::walk_bits_stage(cudaStream_t s, const Group &g, const dev::OutSpec &out, const uint4 *tiles,
                               uint32_t ntiles, uint32_t splits, uint32_t rows, bool first, bool last) {
     if (const int rc = reset_lists(s, g)) return rc;
@@ -3021,6 +3015,7 @@ int PlanImpl::walk_bits_stage(cudaStream_t s, const Group &g, const dev::OutSpec
         a.rs = la.rs;
         a.unit = d_list_unit;
         a.flags_out = d_flags;
+        a.close = d_close;
         if (n_sparse) {
             a.shared.S = d_shared;
             if (const int rc = shared_sums(s, g, a.shared, 0, static_cast<uint32_t>(g.ld))) return rc;
@@ -3034,13 +3029,8 @@ int PlanImpl::walk_bits_stage(cudaStream_t s, const Group &g, const dev::OutSpec
             k.finalize(a, s);
             launches++;
         }
-        a.tile_flags = d_flags;
-        a.lut = static_cast<const double *>(d_lut);
         a.E = n_words_all;
-        a.n_splits = 1;
-        a.rows_per_split = n_words_all;
-        a.partial = nullptr;
-        k_stripe.launch(a, static_cast<uint32_t>(std::min<uint64_t>(ntiles, slots)), k_stripe.smem, s);
+        xor_again(a, d_len_cols, static_cast<uint32_t>(std::min<uint64_t>((static_cast<uint64_t>(ntiles) * k.BM + 7) / 8, 4ull * n_sms)), s);
         launches++;
         SSU_CK(cudaGetLastError());
     }

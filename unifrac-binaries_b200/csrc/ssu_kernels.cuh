@@ -406,8 +406,9 @@ struct PairArgs {
     SharedOut shared;              // S == nullptr: none
     const unsigned long long *rs;  // per column: fixed-point length of its nodes
     const unsigned long long *nib; // [words][16][16] sums of fixed-point lengths by nibble
-    const double *unit;            // value of one fixed-point unit
-    int *flags_out;                // tiles to recompute in the stripe form
+    const double *unit;            // value of one fixed-point unit; whether a length has none
+    int *flags_out;                // tiles with a pair to sum again
+    uint32_t *close;               // per tile a bit for each pair, row-major (zero before and after a pass)
 };
 
 // ---- per-term operators (one (k, l) pair, one embedded node) -------------
@@ -812,7 +813,6 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), 1) pair_bits_kernel(con
     const uint32_t n_work = a.n_tiles * a.n_splits;
     for (uint32_t wi = blockIdx.x; wi < n_work; wi += gridDim.x) {
         const uint32_t split = wi / a.n_tiles, ti = wi - split * a.n_tiles;
-        if (a.tile_flags && !a.tile_flags[ti]) continue;  // uniform over the CTA
         const uint4 tile = a.tiles[ti];
         const uint32_t k0 = tile.x * BM, l0 = tile.y * BN;
         const uint32_t w_begin = split * a.rows_per_split;
@@ -949,14 +949,18 @@ static __global__ void build_nibbles_kernel(const unsigned long long *__restrict
     nib[static_cast<uint64_t>(w) * NIB_TABLE + threadIdx.x] = s;
 }
 
-// Where a pair's distance is below this share of its samples' own lengths,
-// the half unit that each length was rounded by could show: its tile is
-// flagged and recomputed in the stripe form over every node.
-constexpr double kSharedTau = 0.02;
-// So it could where the two samples' lengths are this few units, which the
-// table's largest sample sets: 2^14 of what that one has at most (a clade of
-// branches far below the others').  A pair of m nodes is off by about
-// sqrt(m / 12) units: 1e-14 at 100 nodes.
+// A length's q is the same in every sample, so xor is the exact sum of the q of
+// the nodes that one of the two has, however small beside what they share: only
+// the half unit by which each of those was rounded can show.  Where xor is this
+// few units (m nodes: off by about sqrt(m / 12) of them, 6e-16 at 20 nodes), or 0
+// though some node's length is below half a unit, the pair is marked and summed again
+// by xor_pairs_kernel.  (1,500 samples, each with a duplicate, on 8,000 tips:
+// 389 us; with the stripe form over every tile with a pair below 0.02
+// of its lengths 4,825 us, in the stripe form alone 2,488 us.)
+constexpr unsigned long long kXorLeast = 1ull << 51;
+// Weighted and generalized: one-sided sums of this few units (ssu_rows.cuh,
+// ssu_gen.cuh).  The unit follows the table's largest sample; a pair of m
+// nodes is off by about sqrt(m / 6) units.
 constexpr double kSharedLeast = 0x1p48;
 
 template <bool NORMALIZED, int BM, int BN, int TM, int TN>
@@ -967,14 +971,15 @@ __device__ __forceinline__ void shared_bits_epilogue(const PairArgs<double> &a, 
     const uint32_t k0 = tile.x * BM - td.base, l0 = tile.y * BN - td.base;
     OutSpec o = a.out;
     if (o.mode == 0) o.ptr = static_cast<double *>(o.ptr) + td.out_off;
-    const double unit = *a.unit;
+    const double unit = a.unit[0];
+    const bool lost = a.unit[1] != 0.0;  // a length of no units
     unsigned long long rl[TN];
 #pragma unroll
     for (int j = 0; j < TN; j++) {
         const uint32_t l = l0 + tile_row<BN, TN>(tx, j);
         rl[j] = l < td.n ? a.rs[td.base + l] : 0ull;
     }
-    bool close = false;
+    bool any = false;
 #pragma unroll
     for (int i = 0; i < TM; i++) {
         const uint32_t k = k0 + tile_row<BM, TM>(ty, i);
@@ -986,12 +991,17 @@ __device__ __forceinline__ void shared_bits_epilogue(const PairArgs<double> &a, 
             const uint32_t l = l0 + tile_row<BN, TN>(tx, j);
             if (!(k < l && l < td.n)) continue;
             const unsigned long long own = rk + rl[j], sh = acc[i][j] + (row ? row[l] : 0ull);
-            const double x = static_cast<double>(own - 2 * sh);
-            close = close || x < kSharedTau * static_cast<double>(own) || static_cast<double>(own) < kSharedLeast;
+            const unsigned long long xor_q = own - 2 * sh;
+            const double x = static_cast<double>(xor_q);
+            if (xor_q < kXorLeast && (xor_q || lost)) {
+                const uint32_t e = static_cast<uint32_t>(tile_row<BM, TM>(ty, i) * BN + tile_row<BN, TN>(tx, j));
+                atomicOr(a.close + static_cast<uint64_t>(ti) * (BM * BN / 32) + e / 32, 1u << (e & 31));
+                any = true;
+            }
             emit_pair<double>(o, td.n, k, l, NORMALIZED ? x / static_cast<double>(own - sh) : x * unit);
         }
     }
-    if (close) atomicOr(a.flags_out + ti, 1);
+    if (any) atomicOr(a.flags_out + ti, 1);
 }
 
 template <bool NORMALIZED, int BM, int BN, int TM, int TN, int KW>
@@ -1097,6 +1107,46 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) shared_bits_finalize_ke
                     a.partial)[(static_cast<uint64_t>(s) * a.n_tiles + blockIdx.x) * BM * BN + (i * TN + j) * NT + tid];
         }
     shared_bits_epilogue<NORMALIZED, BM, BN, TM, TN>(a, blockIdx.x, tid % (BN / TN), tid / (BN / TN), acc);
+}
+
+// The marked pairs again, a warp each: the lengths of the nodes that one and that
+// either has, from the two samples' presence words (len: per node column), in fp64.
+// A warp looks after rows of tiles in turn, and clears their marks.
+template <bool NORMALIZED, int BM, int BN>
+__global__ void __launch_bounds__(256) xor_pairs_kernel(const PairArgs<double> a, const double *__restrict__ len) {
+    constexpr uint32_t WPR = BN / 32;
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * 8;
+    const uint64_t n_rows = static_cast<uint64_t>(a.n_tiles) * BM;
+    for (uint64_t u = blockIdx.x * 8 + threadIdx.x / 32; u < n_rows; u += warps) {
+        const uint32_t ti = static_cast<uint32_t>(u / BM), row = static_cast<uint32_t>(u % BM);
+        if (!a.flags_out[ti]) continue;  // uniform over the warp, as all that follows
+        uint32_t *marks = a.close + static_cast<uint64_t>(ti) * (BM * WPR) + row * WPR;
+        const uint4 tile = a.tiles[ti];
+        const TableDesc td = a.tables[tile.z];
+        OutSpec o = a.out;
+        if (o.mode == 0) o.ptr = static_cast<double *>(o.ptr) + td.out_off;
+        const uint32_t kc = tile.x * BM + row;
+        for (uint32_t w = 0; w < WPR; w++) {
+            for (uint32_t m = marks[w]; m; m &= m - 1) {
+                const uint32_t lc = tile.y * BN + w * 32 + __ffs(m) - 1;
+                double x = 0.0, both = 0.0;
+                for (uint32_t i = lane; i < a.E; i += 32) {
+                    const unsigned long long pk = a.P[i * a.ld + kc], pl = a.P[i * a.ld + lc];
+                    for (unsigned long long b = pk ^ pl; b; b &= b - 1) x += len[i * 64 + __ffsll(b) - 1];
+                    if (NORMALIZED)
+                        for (unsigned long long b = pk & pl; b; b &= b - 1) both += len[i * 64 + __ffsll(b) - 1];
+                }
+#pragma unroll
+                for (int s = 16; s > 0; s >>= 1) {
+                    x += __shfl_xor_sync(0xffffffffu, x, s);
+                    both += __shfl_xor_sync(0xffffffffu, both, s);
+                }
+                if (lane == 0) emit_pair<double>(o, td.n, kc - td.base, lc - td.base, NORMALIZED ? x / (x + both) : x);
+            }
+            __syncwarp();
+            if (lane == 0) marks[w] = 0u;
+        }
+    }
 }
 
 }  // namespace dev

@@ -92,7 +92,8 @@ static __global__ void __launch_bounds__(256)
     if (lane == 0) atomicMax(top, static_cast<unsigned long long>(__double_as_longlong(s)));
 }
 
-// q = round(L 2^s), unit = 2^-s.  The scale is `least`, at which the sum of
+// q = round(L 2^s), unit = 2^-s (and 1 behind it, zero before the launch, where a
+// positive length has no units).  The scale is `least`, at which the sum of
 // every sparse length stays below 2^62 units, or (top != nullptr: every column
 // is summed as q) the finest at which no sample's sum reaches 2^63: it is at
 // most *top, and at most `all`, the sum of every length.  (`least` counts the
@@ -108,8 +109,11 @@ static __global__ void fixed_lengths_kernel(const double *__restrict__ len, uint
         scale = m > 0.0 ? ldexp(1.0, min(63 - x, 1000)) : 1.0;
     }
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *unit = 1.0 / scale;
-    if (i < n) q[i] = static_cast<unsigned long long>(__double2ll_rn(len[i] * scale));
+    if (i == 0) unit[0] = 1.0 / scale;
+    if (i < n) {
+        q[i] = static_cast<unsigned long long>(__double2ll_rn(len[i] * scale));
+        if (len[i] > 0.0 && q[i] == 0) unit[1] = 1.0;
+    }
 }
 
 // Walks up from a sample's tips: marks every node on their paths in the

@@ -107,13 +107,13 @@ PairKernel<double> shared_bits_kernel(const char *name, const char *shape) {
     };
     return k;
 }
-// The whole-number form and the stripe form in the same tile shape (the tiles
-// that the first flags are recomputed by the second): 128 x 64, or 32 x 32 where
-// those would not fill the SMs.
-struct SharedBitsPair {
-    PairKernel<double> shared, stripe;
+// The whole-number form in 128 x 64 tiles, or 32 x 32 where those would not fill
+// the SMs, and the kernel that sums its marked pairs again.
+struct SharedBits {
+    PairKernel<double> pair;
+    void (*again)(const dev::PairArgs<double> &a, const double *len, uint32_t ctas, cudaStream_t s);
 };
-SharedBitsPair shared_bits_pair(bool normalized, bool small);
+SharedBits shared_bits(bool normalized, bool small);
 
 // alpha kind: 1 -> sqrt, 2 -> identity, 3 -> constant 1, 0 -> pow
 inline int alpha_kind(double alpha) {

@@ -14,19 +14,20 @@ std::vector<PairKernel<T>> bits_candidates(bool normalized) {
             bits_kernel<T, false, 64, 64, 4, 4, KW>("pair_bits<unweighted_unnormalized>", "64x64/4x4")};
 }
 
-template <bool NORM>
-static SharedBitsPair shared_bits_of(const char *name, const char *stripe, bool small) {
-    if (small)
-        return {shared_bits_kernel<NORM, 32, 32, 2, 2, 4>(name, "32x32/2x2"),
-                bits_kernel<double, NORM, 32, 32, 2, 2, 2>(stripe, "32x32/2x2")};
-    return {shared_bits_kernel<NORM, 128, 64, 8, 4, 4>(name, "128x64/8x4"),
-            bits_kernel<double, NORM, 128, 64, 8, 4, 2>(stripe, "128x64/8x4")};
+template <bool NORM, int BM, int BN>
+static void xor_pairs(const dev::PairArgs<double> &a, const double *len, uint32_t ctas, cudaStream_t s) {
+    dev::xor_pairs_kernel<NORM, BM, BN><<<ctas, 256, 0, s>>>(a, len);
 }
 
-SharedBitsPair shared_bits_pair(bool normalized, bool small) {
-    return normalized ? shared_bits_of<true>("pair_shared_bits<unweighted>", "pair_bits<unweighted>", small)
-                      : shared_bits_of<false>("pair_shared_bits<unweighted_unnormalized>",
-                                              "pair_bits<unweighted_unnormalized>", small);
+template <bool NORM>
+static SharedBits shared_bits_of(const char *name, bool small) {
+    if (small) return {shared_bits_kernel<NORM, 32, 32, 2, 2, 4>(name, "32x32/2x2"), xor_pairs<NORM, 32, 32>};
+    return {shared_bits_kernel<NORM, 128, 64, 8, 4, 4>(name, "128x64/8x4"), xor_pairs<NORM, 128, 64>};
+}
+
+SharedBits shared_bits(bool normalized, bool small) {
+    return normalized ? shared_bits_of<true>("pair_shared_bits<unweighted>", small)
+                      : shared_bits_of<false>("pair_shared_bits<unweighted_unnormalized>", small);
 }
 
 template std::vector<PairKernel<double>> bits_candidates<double>(bool);
