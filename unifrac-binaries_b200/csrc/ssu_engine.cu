@@ -2786,8 +2786,10 @@ int PlanImpl::walk_weighted_stage(cudaStream_t s, const Group &g, const dev::Out
         // near duplicates where the embedding's is (2-norm against long double, counts
         // with 0.1 to 3% noise: 0.5 to 1.3 times; at 0.02 1.0 to 1.3, at 0.002 0.6 to
         // 1.5); 700 of them on 5,000 tips take 0.52 ms (0.60 at 0.02, 0.35 at
-        // 0.002).  Rows in single precision want the wider bound.
-        h.tau = spec.fp64 ? 0.005 : 0.02;
+        // 0.002).  Single precision: 0.25 to 0.4 times the embedding's
+        // error (at 0.02 0.2 to 0.25), and 2,048 near duplicates on 20,000 tips 0.75 ms
+        // (1.99 at 0.02, 1.28 in the embedding's form).
+        h.tau = 0.005;
         h.tile_flags = d_flags;
         h.close = d_close;
         h.partial = h.n_splits > 1 ? d_hpartial : nullptr;
