@@ -1751,7 +1751,6 @@ int PlanImpl::tune_band() {
     return build_units(best_band);
 }
 
-// Row of every row's parent, or -1 under the root.
 // Starting column of each tree observation: its tip's, or the tip's parent's
 // when tips are bypassed; -1 where neither is embedded.
 std::vector<int32_t> path_starts(const FlatTree &tree, const std::vector<int32_t> &col_of_row) {
@@ -2637,7 +2636,6 @@ int PlanImpl::setup_walk_weighted(const TableSet &set, const FlatTree &tree) {
     walk.n_words = n_cols / 32;
     walk.sparse0 = lay.sparse0;
     walk.dense0 = lay.dense0;
-    walk.n_dense = n_dense_rows;
     walk.scale = scale;
     walk.gen = walk_gen ? 1 : 0;
     walk.alpha = spec.alpha;

@@ -6,7 +6,8 @@
 // and shared_kl only needs, for sample k, the lists of the samples of k's own
 // nodes: m^2 / 2 additions for a node that m samples have, against n^2 / 2
 // terms in a dense form.  The lengths are 64-bit fixed point,
-// q = round(L 2^s) with sum_S L 2^s < 2^62, and every sum of them is exact,
+// q = round(L 2^s) with sum_S L 2^s < 2^62 (fp64 results, where every node's length
+// is one: with every sample's sum below 2^63), and every sum of them is exact,
 // so the differences above are exact sums of the q: no cancellation (two
 // samples with the same nodes differ by exactly 0), and no dependence on the
 // order of the additions.
@@ -16,15 +17,15 @@
 //   sum_{n in S} L |u(k) - u(l)| 2^s = rs_k + rs_l - 2 sum min(q_n(k), q_n(l)),
 // rs_k = sum q_n(k): the same sums with min(q(k), q(l)) in place of q, exact in
 // the same way (rounding keeps the order, so the smaller q is the smaller
-// value's).  A sample's rs never exceeds its total times the longest path from
-// the root to a tip, which sets the scale.
+// value's).  A sample's rs never exceeds its total times the largest sum of sparse
+// lengths on a path from the root to a tip, which sets the scale.
 //
 // Lists (built by the walk over each sample's tips, per execute):
 //   node side:   per (table, node) the table's samples that have it, 16 or 32
 //                bits each, at a 16-byte offset laid out once from the tips'
 //                entry counts (an upper bound of the length); a table's
-//                samples are walked in up to LIST_PARTS launches of
-//                consecutive samples, so a list is in order from part to
+//                samples are walked in up to LIST_PARTS launches (twice as
+//                many while a part's columns do not fit a block) of consecutive samples, so a list is in order from part to
 //                part (in any order within one), and where each part starts
 //                is kept: a sample reads its own part and the later ones;
 //   sample side: per sample its sparse nodes, in node order, in one array.
@@ -40,7 +41,7 @@ namespace ssu {
 namespace dev {
 
 constexpr uint32_t LIST_ALIGN = 8;  // entries; node lists start on a multiple (16 bytes of 16-bit entries)
-constexpr uint32_t LIST_PARTS = 8;  // launches of the walk, at most
+constexpr uint32_t LIST_PARTS = 8;  // launches of the walk, unless a part's columns do not fit a block then
 
 // Lists of one group of tables.  Node e of table t (from the group's first)
 // is slot t * n_nodes + e.
@@ -487,7 +488,7 @@ struct WalkArgs {
     const double *totals;        // per column j
     int normalize;
     uint32_t n_words;            // 32-bit words of the bitmap
-    uint32_t sparse0, dense0, n_dense;  // section starts
+    uint32_t sparse0, dense0;    // section starts
     double scale;                // 2^s
     int gen;                     // generalized: q = round(L u^alpha 2^s), rows of u, W = sum L u^alpha
     double alpha;
