@@ -530,8 +530,9 @@ def run_presence(args):
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "u8 operands (presence times 8-bit digits of 23-bit fixed-point lengths, q = 256 u v + s t), "
-                     "exact s32 accumulate per chunk, f64 across chunks and ratios",
+            "dtype": "nodes that few samples have: 64-bit whole-number sums; the others: u8 operands (presence times "
+                     "8-bit digits of 23-bit fixed-point lengths, q = 256 u v + s t), exact s32 accumulate per chunk, "
+                     "f64 across chunks and ratios",
             "data": "synthetic (seeded generator presence_100k_tips_25k_samples)",
             "config": {"workload": PRESENCE_WORKLOAD, "method": method, "pair_kernel": "unweighted_tc_kernel",
                        "n_samples": n, "embedded_branches": gp_units_e(units, n), "per_gpu_units": units,

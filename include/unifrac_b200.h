@@ -54,7 +54,7 @@ typedef struct mat {
     unsigned int n_samples;
     unsigned int cf_size;
     bool is_upper_triangle;
-    double *condensed_form;
+    double *condensed_form; /* singles, widened, for an fp32 method */
     char **sample_ids;
 } mat_t;
 
@@ -87,7 +87,7 @@ typedef struct results_vec {
 typedef struct partial_mat {
     uint32_t n_samples;
     char **sample_ids;
-    double **stripes;
+    double **stripes; /* singles, widened, for an fp32 method */
     uint32_t stripe_start;
     uint32_t stripe_stop;
     uint32_t stripe_total;
