@@ -1191,3 +1191,16 @@ def test_duplicated_samples_cost_little_more_than_others(ssu):
         best.append(min(ms))
         plan.close()
     assert best[0] < 2 * best[1], best
+
+
+def test_near_duplicates_of_uneven_depth(ssu, monkeypatch):
+    """Raw counts, near duplicates whose depths span a factor of 10,000: the shallow
+    pairs are few units of the deepest sample's fixed point, and meet 1e-12 of the dense form."""
+    for seed in range(6):
+        tree, table = _all_near(200 + seed, 14, 3000, 0.1)
+        depth = np.repeat(10.0 ** np.random.default_rng(seed).uniform(0, 4, 7), 2)
+        dense = table.dense() * depth
+        table = ssu_synth.Table.from_dense(dense, table.obs_ids, table.sample_ids)
+        for method in ("weighted_unnormalized_fp64", "weighted_normalized_fp64"):
+            call = lambda: ssu.one_off_matrix(tree, table, method, normalize=False)[0]  # noqa: E731
+            check_fp64(call(), _dense_mode(monkeypatch, call))

@@ -960,8 +960,9 @@ static __global__ void build_nibbles_kernel(const unsigned long long *__restrict
 constexpr unsigned long long kXorLeast = 1ull << 51;
 // Weighted and generalized: one-sided sums of this few units (ssu_rows.cuh,
 // ssu_gen.cuh).  The unit follows the table's largest sample; a pair of m
-// nodes is off by about sqrt(m / 6) units.
-constexpr double kSharedLeast = 0x1p48;
+// nodes is off by about sqrt(m / 6) units, which at 600 nodes and a distance of
+// 0.005 of these sums is 1e-12 of the distance.
+constexpr double kSharedLeast = 0x1p51;
 
 template <bool NORMALIZED, int BM, int BN, int TM, int TN>
 __device__ __forceinline__ void shared_bits_epilogue(const PairArgs<double> &a, uint32_t ti, int tx, int ty,
